@@ -5,16 +5,18 @@
 // expanded[l][block] (GenericPreExpanded, ntt/domain_context.rs:99-159); the forward butterfly is
 // u += v*t; v += u.  Field arithmetic is exact, so any evaluation order gives identical bits.
 //
-// B200 mapping: a pass fuses up to 8 consecutive layers.  One CTA owns a tile of 2^(k+c) elements
+// B200 mapping: a pass fuses up to 13 consecutive layers.  One CTA owns a tile of 2^(k+c) elements
 // (k butterfly bits plus c contiguous low index bits for coalescing) resident in shared memory
-// together with the 2^k - 1 twiddles the tile needs, so each pass reads and writes HBM once with
-// 128-bit accesses.  Reed-Solomon encode (reed_solomon.rs:128-201) fuses the message bit reversal
+// together with the twiddles the tile needs, so each pass reads and writes HBM once with 128-bit
+// accesses.  Transforms of 2^11 elements and more multiply on the tensor cores
+// (ntt_tc_pass_kernel), smaller ones on the integer pipes (ntt_pass_kernel, up to 8 layers).  Reed-Solomon encode (reed_solomon.rs:128-201) fuses the message bit reversal
 // and the 2^R-fold replication into the first pass's load: for the first pass the butterfly bits
 // are exactly the message's low index bits after reversal, so the gather stays coalesced.
 #include <algorithm>
 #include <vector>
 
 #include "gf128.cuh"
+#include "gf_tc.cuh"
 #include "internal.h"
 
 using namespace bgpu;
@@ -123,6 +125,354 @@ __global__ void __launch_bounds__(kNttThreads)
   }
 }
 
+// ---- the tensor-core pass
+//
+// The same pass on a tile of 2^10 to 2^13 elements (up to 128 KiB of shared memory), one CTA of
+// four 128-thread groups per SM, persistent over the tiles.  A layer's butterflies are taken 128 at a time (an M-tile),
+// v t by gf_tc.cuh; a group has a contiguous share of the layer's M-tiles, and prepares the next
+// one while the tensor cores work on this:
+//
+// * butterfly bit h >= 7: an M-tile has one twiddle.  Its matrix is built when it changes, under
+//   the products of the M-tile before.
+// * h = 6, 5: two or four twiddles.  They differ by the layer's twiddles of blocks 1 and 2
+//   (twiddle(block) is linear in the block's bits), whose matrices are built once per layer; the
+//   M-tile's own matrix is the one of its first twiddle, and each row bit from h up is an operand
+//   slot.  Measured per layer of a 2^13 tile: 25 and 28 k cycles, against 34 k with the integer
+//   multiply and 14 k with one twiddle; with four and five slots (h = 4, 3) 31 and 34 k.
+// * h < 5: the integer multiply.
+//
+// What bounds it (five and four layers of a 2^13-element tile, ncu): the logic pipe 63% and the
+// tensor pipe 40% busy with 16 warps an SM, DRAM 12%.  Per 128 products and one layer 450 cycles,
+// of which a lone stream of collections and operand writes takes 235 (tensor-memory reads do not
+// overlap the logic that follows them); the rest is the hand-over between a group's warps (four of
+// them must have read the sums before the next products start, and four groups are all that 512
+// TMEM columns hold with two operand slots each), a fifth of it the drain at the end of a layer.
+// Measured against it and left: three groups with 128 columns of sums and e4m3 / e5m2 operands
+// (690 cycles per 128 products and layer), a separate issuing warp that polls the groups (750).
+constexpr uint32_t kTcGroups = 4;
+constexpr uint32_t kTcThreads = kTcGroups * tc::kGroupThreads;
+constexpr uint32_t kTcTileBits = 13;
+constexpr uint32_t kTcMinTileBits = 10;
+constexpr uint32_t kTcOneBit = 7;     // an M-tile has one twiddle from this butterfly bit up
+constexpr uint32_t kTcLowestBit = 5;  // and takes slots down to this one
+constexpr uint32_t kTcLowLayers = kTcOneBit - kTcLowestBit;
+constexpr uint32_t kTcTmemCols = 512;
+constexpr uint32_t kTcMaxMTiles = 1u << (kTcTileBits - 8);
+constexpr uint32_t kTcLowTwiddles = kTcMaxMTiles + kTcLowLayers;  // of one layer with h < 7
+constexpr uint32_t kTcTwiddles = 2 * kTcMaxMTiles + kTcLowLayers * kTcLowTwiddles;
+constexpr uint32_t kTcMatrices = 2 * kTcGroups;
+
+struct NttTcShared {
+  uint4 tile[1u << kTcTileBits];
+  uint8_t matrices[kTcMatrices][tc::kMatrixBytes];
+  tc::MatrixRows rows[2][kTcLowTwiddles];  // of this layer's and the next one's twiddles
+  uint4 twiddles[kTcTwiddles];
+  uint8_t ones[tc::kOnesBytes];
+  uint64_t done[kTcGroups];
+  uint32_t tmem;
+};
+
+// Set when a wait for the tensor cores ran out (a tile of that launch is then left unwritten).
+__device__ uint32_t g_ntt_tc_stalled;
+
+__device__ __forceinline__ void cp_async16(uint4* smem_dst, const uint4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_addr(smem_dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// One layer of a tile in shared memory on the tensor cores (SLOTS: h < 7); emit(e, x) takes the
+// results.  Returns false when a wait ran out.
+template <bool INVERSE, bool SLOTS, class Emit>
+__device__ __forceinline__ bool ntt_tc_layer(NttTcShared& sh, const tc::MatrixRows* rows,
+                                             uint32_t h, uint32_t n_mtiles, uint32_t group,
+                                             uint32_t tmem, uint32_t& phase, const Emit& emit) {
+  const uint32_t gt = threadIdx.x % tc::kGroupThreads;
+  const uint32_t gw = tc::uniform(gt / 32);
+  const uint32_t lanes = (gw * 32) << 16;
+  const uint32_t row_bits = SLOTS ? kTcOneBit - h : 0;
+  // TMEM columns of a group: its sums, then two operand slots in turn, or the M-tile's slots
+  constexpr uint32_t cols = tc::kSumCols + tc::kOperandCols * (1 + kTcLowLayers);
+  static_assert(kTcGroups * cols + tc::kConstCols <= kTcTmemCols, "TMEM columns");
+  const uint32_t sums = tmem + group * cols;
+  const uint32_t slot0 = sums + tc::kSumCols;
+  const uint32_t consts = tmem + kTcTmemCols - tc::kConstCols;
+  const uint32_t ones = tc::uniform(tc::smem_addr(sh.ones));
+  const uint32_t matrices = tc::uniform(tc::smem_addr(sh.matrices));
+  uint32_t buf = SLOTS ? group : 2 * group;
+  bool ok = true;
+
+  if (SLOTS) {  // the matrices of the layer's twiddles of blocks 1, 2, 4, ..
+    if (group < row_bits) {
+      tc::matrix_build(sh.matrices[kTcGroups + group], rows[n_mtiles + group], gt);
+      tc::fence_smem_to_tensor();
+    }
+    __syncthreads();
+  }
+  const uint32_t i0 = n_mtiles * group / kTcGroups, i1 = n_mtiles * (group + 1) / kTcGroups;
+
+  const uint32_t hs = SLOTS ? 0 : h - kTcOneBit;  // M-tile i has twiddle i >> hs
+  auto first = [&](uint32_t i) {  // the tile index of this thread's u
+    if (SLOTS) {
+      const uint32_t q = i * tc::kGroupThreads + gt;
+      return ((q >> h) << (h + 1)) | (q & ((1u << h) - 1));
+    }
+    return ((i >> hs) << (h + 1)) + ((i & ((1u << hs) - 1)) * tc::kGroupThreads) + gt;
+  };
+  auto build = [&](uint32_t j) {
+    tc::matrix_build(sh.matrices[buf], rows[j], gt);
+    tc::fence_smem_to_tensor();
+  };
+  uint32_t slot = slot0;
+  auto store_operand = [&](uint4 x) {
+    uint32_t r[16];
+    tc::operand_words(x, r);
+    tc::operand_store(slot + lanes, r);
+    if (SLOTS) {
+      for (uint32_t j = 0; j < row_bits; j++) {
+        const bool on = (gt >> (h + j)) & 1;
+        uint32_t m[16];
+#pragma unroll
+        for (int w = 0; w < 16; w++) m[w] = on ? r[w] : 0u;
+        tc::operand_store(slot0 + tc::kOperandCols * (1 + j) + lanes, m);
+      }
+    }
+    tc::wait_stores();
+  };
+  // operand and matrix written, sums read by the whole group: one warp issues the next products
+  auto start = [&](uint32_t turn, uint32_t part) {
+    tc::fence_before();
+    if (gw != (turn & 3)) {
+      tc::group_arrive(group + 1);
+      return;
+    }
+    tc::group_wait(group + 1);
+    tc::fence_after();
+    if (!SLOTS) {
+      tc::issue_pairs(sums, slot, matrices + buf * tc::kMatrixBytes, consts, ones,
+                      &sh.done[group]);
+      return;
+    }
+    tc::issue_ones(sums, consts, ones);
+    tc::issue_part(sums, slot, matrices + buf * tc::kMatrixBytes, part, consts);
+    for (uint32_t j = 0; j < row_bits; j++)
+      tc::issue_part(sums, slot0 + tc::kOperandCols * (1 + j),
+                     matrices + (kTcGroups + j) * tc::kMatrixBytes, part, consts);
+    tc::commit(&sh.done[group]);
+  };
+  auto finish = [&]() {
+    ok = tc::mbar_wait(&sh.done[group], phase) && ok;
+    phase ^= 1;
+    tc::fence_after();
+  };
+
+  build(i0 >> hs);
+  uint32_t e0 = first(i0);
+  uint4 u = sh.tile[e0], v = sh.tile[e0 | (1u << h)];
+  if (INVERSE) gf_add_into(v, u);
+  store_operand(v);
+  start(i0, 0);
+  for (uint32_t i = i0; i < i1; i++) {
+    const bool next = i + 1 < i1;
+    uint32_t ne0 = e0;
+    uint4 nu = u, nv = v, tv;
+    uint2 part0;
+    if (SLOTS) {
+      finish();
+      part0 = tc::collect_part(sums + lanes);
+      start(i + 1, 1);
+    }
+    if (next) {
+      ne0 = first(i + 1);
+      nu = sh.tile[ne0];
+      nv = sh.tile[ne0 | (1u << h)];
+      if (INVERSE) gf_add_into(nv, nu);
+      if (!SLOTS) {
+        if (((i + 1) >> hs) != (i >> hs)) {
+          buf ^= 1;
+          build((i + 1) >> hs);
+        }
+        slot ^= slot0 ^ (slot0 + tc::kOperandCols);
+        store_operand(nv);
+      }
+    }
+    finish();
+    if (SLOTS) {
+      if (next) {
+        build(i + 1);
+        store_operand(nv);
+      }
+      tv = tc::join_parts(part0, tc::collect_part(sums + lanes));
+    } else {
+      tv = tc::collect_pairs(sums + lanes);
+    }
+    if (next) start(i + 1, 0);
+    gf_add_into(u, tv);
+    if (!INVERSE) gf_add_into(v, u);
+    emit(e0, u);
+    emit(e0 | (1u << h), v);
+    e0 = ne0;
+    u = nu;
+    v = nv;
+  }
+  return ok;
+}
+
+template <bool INVERSE, bool RS>
+__global__ void __launch_bounds__(kTcThreads, 1)
+    ntt_tc_pass_kernel(uint4* __restrict__ data, const uint4* __restrict__ src,
+                       const uint4* __restrict__ tw, NttPass p, uint32_t n_tiles) {
+  extern __shared__ __align__(128) uint8_t tc_smem[];
+  NttTcShared& sh = *reinterpret_cast<NttTcShared*>(tc_smem);
+  const uint32_t k = p.k, c = p.c;
+  const uint32_t tile_elems = 1u << (k + c);
+  const uint32_t s = p.log_d - p.l0 - k;  // lowest butterfly index bit
+  const uint32_t half = tile_elems >> 1;
+  const uint32_t n_mtiles = half / tc::kGroupThreads;
+  const uint32_t n_one = min(k, c + k - kTcOneBit);           // layers with h >= kTcOneBit
+  const uint32_t n_low = min(k - n_one, kTcLowLayers);        // with kTcOneBit > h >= kTcLowestBit
+  const uint32_t group = tc::uniform(threadIdx.x / tc::kGroupThreads);
+
+  // element e of a tile <-> its base | e's butterfly bits << s | its low c bits
+  auto tile_base = [&](uint32_t t) {
+    return ((uint64_t)(t >> (s - c)) << (s + k)) | ((uint64_t)(t & ((1u << (s - c)) - 1)) << c);
+  };
+  auto tile_offset = [&](uint32_t e) { return ((uint64_t)(e >> c) << s) | (e & ((1u << c) - 1)); };
+  auto load_tile = [&](uint32_t t) {
+    const uint64_t base = tile_base(t);
+    for (uint32_t e = threadIdx.x; e < tile_elems; e += kTcThreads) {
+      if (RS) {
+        const uint64_t msg_mask = (p.rs_bits == 64) ? ~0ull : ((1ull << p.rs_bits) - 1);
+        const uint32_t bfly = rev_bits32(e & ((1u << k) - 1), k);
+        const uint32_t inner = e >> k;
+        const uint64_t g = base | ((uint64_t)bfly << s) | inner;
+        cp_async16(sh.tile + ((bfly << c) | inner), src + rev_bits64(g & msg_mask, p.rs_bits));
+      } else {
+        cp_async16(sh.tile + e, data + (base | tile_offset(e)));
+      }
+    }
+  };
+  // its twiddles: layer l0 + m uses blocks (outer_hi << m) + [0, 2^m).  Layers with h >= 7 keep
+  // them all (at 2^m - 1); one below keeps each M-tile's first and those of blocks 1, 2, 4, ..
+  auto load_twiddles = [&](uint32_t t) {
+    const uint64_t outer_hi = (uint64_t)t >> (s - c);
+    for (uint32_t i = threadIdx.x; i + 1 < (1u << n_one); i += kTcThreads) {
+      const uint32_t m = 31 - __clz(i + 1);
+      cp_async16(sh.twiddles + i,
+                 tw + ((1ull << (p.l0 + m)) - 1) + (outer_hi << m) + (i + 1 - (1u << m)));
+    }
+    for (uint32_t x = threadIdx.x; x < n_low * kTcLowTwiddles; x += kTcThreads) {
+      const uint32_t low = x / kTcLowTwiddles, i = x % kTcLowTwiddles, m = n_one + low;
+      const uint4* layer = tw + ((1ull << (p.l0 + m)) - 1);
+      uint4* dst = sh.twiddles + 2 * kTcMaxMTiles + low * kTcLowTwiddles + i;
+      if (i < n_mtiles)
+        cp_async16(dst, layer + (outer_hi << m) + ((uint64_t)i << (low + 1)));
+      else if (i < n_mtiles + low + 1)
+        cp_async16(dst, layer + (1u << (i - n_mtiles)));
+    }
+  };
+  // the matrix rows of layer m's twiddles into the buffer of its parity
+  auto prepare_rows = [&](uint32_t m) {
+    if (m >= n_one + n_low) return;
+    const bool one = m < n_one;
+    const uint4* t = sh.twiddles + (one ? (1u << m) - 1
+                                        : 2 * kTcMaxMTiles + (m - n_one) * kTcLowTwiddles);
+    const uint32_t n = one ? 1u << m : n_mtiles + m - n_one + 1;
+    for (uint32_t x = threadIdx.x; x < n * tc::kRowItems; x += kTcThreads)
+      tc::matrix_rows(sh.rows[m & 1][x / tc::kRowItems], t[x / tc::kRowItems], x % tc::kRowItems);
+  };
+
+  if (threadIdx.x < 32) tc::tmem_alloc(&sh.tmem, kTcTmemCols);
+  if (threadIdx.x == 0) {
+    for (uint32_t g = 0; g < kTcGroups; g++) tc::mbar_init(&sh.done[g], 1);
+    tc::mbar_init_fence();
+  }
+  load_tile(blockIdx.x);
+  load_twiddles(blockIdx.x);
+  cp_async_wait_all();
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tc::uniform(sh.tmem);
+  if (group == 0) {
+    tc::constants_store(tmem + kTcTmemCols - tc::kConstCols + ((threadIdx.x / 32 * 32) << 16),
+                        sh.ones);
+    tc::fence_smem_to_tensor();
+  }
+  prepare_rows(INVERSE ? k - 1 : 0);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+
+  uint32_t phase = 0;
+  bool ok = true;
+  for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+    const uint64_t outer_hi = (uint64_t)t >> (s - c);
+    const uint32_t nt = t + gridDim.x;
+    uint4* out = data + tile_base(t);
+    const uint4* next = data + (nt < n_tiles ? tile_base(nt) : 0);
+    for (uint32_t mm = 0; mm < k; mm++) {
+      const uint32_t m = INVERSE ? (k - 1 - mm) : mm;
+      const uint32_t h = c + k - 1 - m;
+      const bool last = mm + 1 == k;
+      // The last layer's results go to memory at once (unless a wait ran out: then nothing more
+      // is written), and the next tile's elements come into the places that are now free.
+      auto emit = [&](uint32_t e, uint4 x) {
+        if (!last) {
+          sh.tile[e] = x;
+          return;
+        }
+        const uint64_t offset = tile_offset(e);
+        if (ok) out[offset] = x;
+        if (!RS && nt < n_tiles) cp_async16(sh.tile + e, next + offset);
+      };
+      const tc::MatrixRows* rows = sh.rows[m & 1];
+      if (h >= kTcOneBit) {
+        ok = ntt_tc_layer<INVERSE, false>(sh, rows, h, n_mtiles, group, tmem, phase, emit) && ok;
+      } else if (h >= kTcLowestBit) {
+        ok = ntt_tc_layer<INVERSE, true>(sh, rows, h, n_mtiles, group, tmem, phase, emit) && ok;
+      } else {
+        const uint4* lt = tw + ((1ull << (p.l0 + m)) - 1) + (outer_hi << m);
+        for (uint32_t q = threadIdx.x; q < half; q += kTcThreads) {
+          const uint32_t e0 = ((q >> h) << (h + 1)) | (q & ((1u << h) - 1));
+          const uint32_t e1 = e0 | (1u << h);
+          const uint4 twd = __ldg(lt + (q >> h));
+          uint4 u = sh.tile[e0], v = sh.tile[e1];
+          if (!INVERSE) {
+            gf_add_into(u, gf_mul(v, twd));
+            gf_add_into(v, u);
+          } else {
+            gf_add_into(v, u);
+            gf_add_into(u, gf_mul(v, twd));
+          }
+          emit(e0, u);
+          emit(e1, v);
+        }
+      }
+      if (!last) {
+        prepare_rows(INVERSE ? m - 1 : m + 1);
+        __syncthreads();
+      }
+    }
+    if (!ok) atomicOr(&g_ntt_tc_stalled, 1u);
+    if (nt < n_tiles) {
+      __syncthreads();
+      if (RS) load_tile(nt);
+      load_twiddles(nt);
+      cp_async_wait_all();
+      __syncthreads();
+      prepare_rows(INVERSE ? k - 1 : 0);
+      __syncthreads();
+    }
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) tc::tmem_free(tmem, kTcTmemCols);
+}
+
 std::vector<NttPass> plan_passes(uint32_t log_d, uint32_t skip_early, uint32_t skip_late,
                                  bool rs, uint32_t rs_bits) {
   // tiles of 2^tile_bits elements: fewer, larger tiles fuse more work per CTA; more, smaller ones
@@ -150,6 +500,56 @@ std::vector<NttPass> plan_passes(uint32_t log_d, uint32_t skip_early, uint32_t s
     l0 += k;
   }
   return passes;
+}
+
+// The tensor-core passes of a transform: tiles of 2^tile_bits elements.  The last pass takes every
+// layer its tile can hold above the skipped low bits (its layers below bit 7 are the slower ones
+// whatever the split); the others keep at least 2^7 contiguous elements, so that each M-tile of
+// theirs has one twiddle, and are as even as they can be.
+std::vector<NttPass> plan_tc_passes(uint32_t log_d, uint32_t skip_early, uint32_t skip_late,
+                                    uint32_t tile_bits, uint32_t rs_bits) {
+  std::vector<NttPass> passes;
+  const uint32_t n_layers = log_d - skip_late - skip_early;
+  const uint32_t most = tile_bits - kTcOneBit;
+  const uint32_t last = std::min(n_layers, tile_bits - std::min(skip_late, kTcOneBit));
+  const uint32_t rest = n_layers - last;
+  const uint32_t n_rest = (rest + most - 1) / most;
+  uint32_t l0 = skip_early;
+  for (uint32_t i = 0; i <= n_rest; i++) {
+    const uint32_t k = i == n_rest ? last : rest / n_rest + (i < rest % n_rest ? 1 : 0);
+    const uint32_t s = log_d - l0 - k;
+    passes.push_back({log_d, l0, k, std::min(tile_bits - k, s), i == 0 ? rs_bits : 0u});
+    l0 += k;
+  }
+  return passes;
+}
+
+// Tile bits of a transform's tensor-core passes, 0 = the integer passes.  2^(log_d - 7) elements
+// a tile gives 128 CTAs for the 148 SMs; beyond 2^20 the largest tile that fits (fewer passes and
+// fewer matrices per product), below 2^17 the smallest whose four groups all have an M-tile.
+// Measured on B200, Reed-Solomon encode / inverse transform in us, integer passes -> these:
+// 2^26 x 64 columns 17320 -> 7690, 2^24 x 16 4399 -> 2190, 2^20 x 16 265 -> 134 (tiles of 2^12:
+// 157), 2^18 x 16 99 -> 53 (2^12: 72, 2^10: 74), 2^16 x 16 70 -> 37, 2^12 x 16 36 -> 25; inverse
+// 2^22 .. 2^12 at 0.5-0.6 of the time.  At 2^11 the two meet (39 -> 34) and below it the integer
+// passes win (2^10: 24 against 28).
+uint32_t tc_tile_bits(uint32_t log_d, uint32_t skip_early, uint32_t skip_late) {
+  if (log_d < 11 || log_d == skip_early + skip_late) return 0;
+  const uint32_t bits = std::min(std::max(log_d - 7, kTcMinTileBits), kTcTileBits);
+  return log_d - skip_early >= bits ? bits : 0;
+}
+
+template <bool INVERSE, bool RS>
+int launch_tc_pass(const NttPass& p, uint4* data, const uint4* src, const uint4* tw,
+                   cudaStream_t stream) {
+  auto kern = ntt_tc_pass_kernel<INVERSE, RS>;
+  if (int rc = ensure_smem_limit(reinterpret_cast<const void*>(kern), sizeof(NttTcShared))) return rc;
+  const uint64_t n_tiles = 1ull << (p.log_d - p.k - p.c);
+  if (n_tiles > 0x7fffffffull) return set_error(BINIUS_E_ARG, "ntt: buffer too large");
+  kern<<<(unsigned)std::min<uint64_t>(n_tiles, 148), kTcThreads, sizeof(NttTcShared), stream>>>(
+      data, src, tw, p, (uint32_t)n_tiles);
+  BGPU_LAUNCH_CHECK("ntt_tc_pass_kernel");
+  count_launch();
+  return BINIUS_OK;
 }
 
 template <bool INVERSE, bool RS>
@@ -187,10 +587,21 @@ int ntt_transform(const binius_ntt* ntt, void* d_data, uint32_t log_len, uint32_
   BGPU_ARG(skip_early + skip_late <= log_len, "skip_early + skip_late must be <= log_len");
   BGPU_ARG(log_len - skip_late <= ntt->log_domain, "domain context too small for the transform");
   if (int rc = check_device(ntt)) return rc;
-  auto passes = plan_passes(log_len, skip_early, skip_late, false, 0);
   uint4* data = static_cast<uint4*>(d_data);
   const uint4* tw = static_cast<const uint4*>(ntt->d_twiddles);
   cudaStream_t s = as_stream(stream);
+  if (const uint32_t tb = tc_tile_bits(log_len, skip_early, skip_late)) {
+    auto passes = plan_tc_passes(log_len, skip_early, skip_late, tb, 0);
+    if (!inverse) {
+      for (const auto& p : passes)
+        if (int rc = launch_tc_pass<false, false>(p, data, nullptr, tw, s)) return rc;
+    } else {
+      for (auto it = passes.rbegin(); it != passes.rend(); ++it)
+        if (int rc = launch_tc_pass<true, false>(*it, data, nullptr, tw, s)) return rc;
+    }
+    return clear_error();
+  }
+  auto passes = plan_passes(log_len, skip_early, skip_late, false, 0);
   if (!inverse) {
     for (const auto& p : passes)
       if (int rc = launch_pass<false, false>(p, data, nullptr, tw, s)) return rc;
@@ -218,10 +629,19 @@ int rs_encode_batch(const binius_ntt* ntt, const void* d_msg, uint32_t log_dim,
   BGPU_ARG(log_dim + log_inv_rate <= ntt->log_domain,
            "NTT domain smaller than the code's evaluation domain");
   if (int rc = check_device(ntt)) return rc;
-  auto passes = plan_passes(log_out, log_inv_rate, log_batch, true, log_msg);
   uint4* out = static_cast<uint4*>(d_codeword);
   const uint4* msg = static_cast<const uint4*>(d_msg);
   const uint4* tw = static_cast<const uint4*>(ntt->d_twiddles);
+  if (const uint32_t tb = tc_tile_bits(log_out, log_inv_rate, log_batch)) {
+    auto passes = plan_tc_passes(log_out, log_inv_rate, log_batch, tb, log_msg);
+    for (size_t i = 0; i < passes.size(); i++) {
+      int rc = (i == 0) ? launch_tc_pass<false, true>(passes[i], out, msg, tw, stream)
+                        : launch_tc_pass<false, false>(passes[i], out, nullptr, tw, stream);
+      if (rc) return rc;
+    }
+    return clear_error();
+  }
+  auto passes = plan_passes(log_out, log_inv_rate, log_batch, true, log_msg);
   for (size_t i = 0; i < passes.size(); i++) {
     int rc = (i == 0) ? launch_pass<false, true>(passes[i], out, msg, tw, stream)
                       : launch_pass<false, false>(passes[i], out, nullptr, tw, stream);
