@@ -473,26 +473,28 @@ struct AndRoundConst {
 // the round polynomial by RoundEvals2::interpolate_eq (prover/prover/src/protocols/sumcheck/
 // round_evals.rs:80-86) -> the truncated proof (c_1, c_2) (mlecheck::RoundProof::truncate) ->
 // the challenge r -> the next claim c_0 + c_1 r + c_2 r^2.  One warp runs the chain.
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kFsThreads)
     and_round_finish_kernel(TranscriptState* __restrict__ ts, uint8_t* __restrict__ tape,
                             const uint4* __restrict__ ys, const AndRoundConst* __restrict__ rc,
                             uint4* __restrict__ claim, uint4* __restrict__ r_out) {
   pdl_wait();
   pdl_trigger();
-  {
-    DevTr st;
-    st.load(ts);
-    const uint4 y1 = ys[0], yinf = ys[1];
-    const uint4 y0 =
-        gf_mul_warp(gf_add(*claim, gf_mul_warp(y1, rc->alpha)), rc->inv_one_plus_alpha);
-    const uint4 c0 = y0, c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
-    const uint4 msg[2] = {c1, c2};
-    st.message_elems(tape, msg, 2);
-    const uint4 r = st.sample_elem();
-    *r_out = r;
-    *claim = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
-    st.store(ts);
+  __shared__ FsShared fs;
+  FsStep st;
+  if (threadIdx.x < 32) st.begin(fs, ts);
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    fs_help(fs, fs.slow);
+    return;
   }
+  const uint4 y1 = ys[0], yinf = ys[1];
+  const uint4 y0 = gf_mul_warp(gf_add(*claim, gf_mul_warp(y1, rc->alpha)), rc->inv_one_plus_alpha);
+  const uint4 c0 = y0, c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
+  const uint4 msg[2] = {c1, c2};
+  const uint4 r = st.step(fs, ts, tape, msg, 2, fs.slow);
+  *r_out = r;
+  *claim = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
+  st.end(fs, ts);
 }
 
 // The small last rounds of the MLE-check in one CTA (see bivariate_tail_kernel): per round fold
@@ -509,14 +511,16 @@ __global__ void __launch_bounds__(kAndTailThreads)
   pdl_wait();
   pdl_trigger();
   __shared__ uint4 r_sh;
-  DevTr st;
+  __shared__ FsShared fs;
+  FsStep st;
   uint4 cl = gf_zero();
   if (threadIdx.x < 32) {
-    st.load(ts);
+    st.begin(fs, ts);
     cl = *claim;
     r_sh = *r_first;
   }
   __syncthreads();
+  const bool slow = fs.slow;
   for (uint32_t k = 0; k < n_rounds; k++) {
     const uint4 r = r_sh;
     const uint64_t h = len >> 1, q = len >> 2;
@@ -543,16 +547,17 @@ __global__ void __launch_bounds__(kAndTailThreads)
       const uint4 y0 = gf_mul_warp(gf_add(cl, gf_mul_warp(y1, c.alpha)), c.inv_one_plus_alpha);
       const uint4 c0 = y0, c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
       const uint4 msg[2] = {c1, c2};
-      st.message_elems(tape, msg, 2);
-      const uint4 rr = st.sample_elem();
+      const uint4 rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
       chal[k] = rr;
       cl = gf_add(c0, gf_mul_warp(rr, gf_add(c1, gf_mul_warp(c2, rr))));
       r_sh = rr;
+    } else {
+      fs_help(fs, slow && k == 0);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    st.store(ts);
+  if (threadIdx.x < 32 && n_rounds) {
+    st.end(fs, ts);
     *claim = cl;
   }
 }
@@ -776,7 +781,7 @@ int and_reduction_finish(const binius_cs* cs, AndPrep& p, Transcript& t, AndResu
                        fb, fc, eq, size * 2, (const uint4*)(d_chal + k - 1), acc);
       }
       if (e != cudaSuccess) { rc = cuda_error(e, "AND MLE-check round"); break; }
-      e = launch_pdl(and_round_finish_kernel, 1, 32, 0, s, dt.state(), dt.tape(),
+      e = launch_pdl(and_round_finish_kernel, 1, kFsThreads, 0, s, dt.state(), dt.tape(),
                      reinterpret_cast<const uint4*>(acc), (const AndRoundConst*)(d_consts + k),
                      d_claim, d_chal + k);
       if (e != cudaSuccess) { rc = cuda_error(e, "and_round_finish_kernel"); break; }

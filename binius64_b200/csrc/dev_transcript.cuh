@@ -22,40 +22,46 @@
 namespace bgpu {
 
 // The scalar protocol steps run on one warp, where every dependent instruction waits out its full
-// latency.  Measured on a B200, one warp: the multiply below 0.38 us (the 16 partial products
-// combined by shuffle butterflies instead: 0.45 us; nine clmul32 on one thread: 0.63 us); a
-// SHA-256 compression fully unrolled on registers 1.5 us, a compact loop (four- or sixteen-round
-// body, round constants loaded) 2.2 us.  A Fiat-Shamir step of its own launch (two compressions,
-// two multiplies) costs 7.3 us with the unrolled compression against 8.5 us with the loop, so the
-// transcript uses the unrolled one everywhere; the tail loops, whose warp 0 alternates between a
-// step and the round's folds, also keep their folds on the out-of-line multiply (gf_mul_nl) so
-// that the loop's code stays within the instruction cache (measured: the three tails with inlined
-// folds and the unrolled compression took 120 us longer per 2^20 proof than with the compact loop;
-// with out-of-line folds the unrolled compression is ~30 us faster than the loop).
+// latency and every logic instruction takes the warp's 16-lane pipe for two cycles.  Measured on a
+// B200, one warp: the multiply below 0.13 us (a 32x32 carry-less product per lane and eight warp
+// reductions: 0.37 us; one thread: 0.67 us); a SHA-256 compression fully unrolled on registers 1.5
+// us.  The steps of a stretch run as FsStep below (2.4 us for message and challenge) where the
+// transcript is in its usual state, else as DevTr (4.9 us).
 __device__ __forceinline__ uint4 gf_mul_1t(uint4 a, uint4 b) { return gf_mul_nl(a, b); }
 
 // A product on the critical path of a Fiat-Shamir step, computed by a whole warp: every lane
-// passes the same a and b; lane l < 16 forms the 32x32 carry-less product of word l/4 of a and
-// word l%4 of b, each of the eight words of the 256-bit product is the XOR of the partial-product
-// halves that land on it (one warp reduction, __reduce_xor_sync, per word), and every lane returns the
-// reduced product.  One out-of-line copy keeps the code of the launches that call it small.
+// passes the same a and b and gets the product.  Lane l takes bits l, 32 + l, 64 + l and 96 + l of
+// a: their multiples of b lie at whole-word offsets of one another, so they are masks of b's words
+// XORed in place, shifted by l once, reduced, and XORed over the warp (one warp reduction,
+// __reduce_xor_sync, per word).  One out-of-line copy keeps the code of the launches that call it
+// small.
 static __device__ __noinline__ uint4 gf_mul_warp(uint4 a, uint4 b) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t i = (lane >> 2) & 3, j = lane & 3;
-  const uint32_t ai = i == 0 ? a.x : i == 1 ? a.y : i == 2 ? a.z : a.w;
-  const uint32_t bj = j == 0 ? b.x : j == 1 ? b.y : j == 2 ? b.z : b.w;
-  const uint64_t p = lane < 16 ? clmul32(ai, bj) : 0ull;
-  const uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32), k = i + j;
-  uint32_t w[8];
-#pragma unroll
-  for (uint32_t q = 0; q < 8; q++)
-    w[q] = __reduce_xor_sync(0xffffffffu, (k == q ? lo : 0u) ^ (k + 1 == q ? hi : 0u));
-  u256 r;
-  r.p0 = ((uint64_t)w[1] << 32) | w[0];
-  r.p1 = ((uint64_t)w[3] << 32) | w[2];
-  r.p2 = ((uint64_t)w[5] << 32) | w[4];
-  r.p3 = ((uint64_t)w[7] << 32) | w[6];
-  return reduce256(r);
+  const uint32_t l = threadIdx.x & 31;
+  auto mask = [&](uint32_t w) { return (uint32_t)((int32_t)(w << (31 - l)) >> 31); };
+  const uint32_t m0 = mask(a.x), m1 = mask(a.y), m2 = mask(a.z), m3 = mask(a.w);
+  const uint32_t w0 = b.x & m0;
+  const uint32_t w1 = (b.y & m0) ^ (b.x & m1);
+  const uint32_t w2 = (b.z & m0) ^ (b.y & m1) ^ (b.x & m2);
+  const uint32_t w3 = (b.w & m0) ^ (b.z & m1) ^ (b.y & m2) ^ (b.x & m3);
+  const uint32_t w4 = (b.w & m1) ^ (b.z & m2) ^ (b.y & m3);
+  const uint32_t w5 = (b.w & m2) ^ (b.z & m3);
+  const uint32_t w6 = b.w & m3;
+  const uint32_t h0 = __funnelshift_l(w3, w4, l), h1 = __funnelshift_l(w4, w5, l);
+  const uint32_t h2 = __funnelshift_l(w5, w6, l), h3 = __funnelshift_l(w6, 0u, l);
+  const uint32_t t = (h3 >> 31) ^ (h3 >> 30) ^ (h3 >> 25);  // what the fold pushes past x^127
+  auto fold = [](uint32_t lo, uint32_t hi) {  // word of H (1 + x + x^2 + x^7)
+    return hi ^ __funnelshift_l(lo, hi, 1) ^ __funnelshift_l(lo, hi, 2) ^ __funnelshift_l(lo, hi, 7);
+  };
+  uint4 o;
+  o.x = (w0 << l) ^ fold(0u, h0) ^ t ^ (t << 1) ^ (t << 2) ^ (t << 7);
+  o.y = __funnelshift_l(w0, w1, l) ^ fold(h0, h1);
+  o.z = __funnelshift_l(w1, w2, l) ^ fold(h1, h2);
+  o.w = __funnelshift_l(w2, w3, l) ^ fold(h2, h3);
+  o.x = __reduce_xor_sync(0xffffffffu, o.x);
+  o.y = __reduce_xor_sync(0xffffffffu, o.y);
+  o.z = __reduce_xor_sync(0xffffffffu, o.z);
+  o.w = __reduce_xor_sync(0xffffffffu, o.w);
+  return o;
 }
 
 // One compression of blk into st, both held in local memory by the caller: copied to registers,
@@ -268,6 +274,224 @@ struct DevTr {
   }
 };
 
+
+// A round's Fiat-Shamir step, message() of n elements then sample(), by three warps of a block.
+//
+// Between the rounds of a stretch the transcript is nearly always in one state: it has just been
+// sampled, so the SHA-256 stream holds the 32 bytes of the last digest and nothing else.  From
+// there a step absorbs those, 8 bytes for the return to observing and the message, and digests
+// the padded stream: two blocks, whose words are all known before the first compression.  Warp 0
+// lays the words out (one per lane) and runs the 64 + 64 rounds; warps 1 and 2, on other
+// schedulers, expand the two message schedules meanwhile and hand them over through shared memory
+// with the round constants added.  A compression on one warp is bound by that warp's logic pipe
+// (1376 instructions of two cycles); without the schedules 900 are left.  Measured, one step:
+// 2.4 us against 4.9 us with DevTr; a 2^12-word proof 2.55 -> 2.20 ms, one of 2^18 words and 256
+// multiplications 5.30 -> 4.46 ms, one of 2^20 words 3.04 -> 2.78 ms (with the multiply above).
+// From any other state (a stretch that begins before the host has sampled; none of the protocol's
+// does) the first step runs as DevTr.
+constexpr uint32_t kFsThreads = 96;  // warps 0, 1 and 2 take part
+struct __align__(16) FsShared {
+  uint32_t words[32];   // the stream's two padded blocks; between steps the digest in 0..7
+  uint32_t kw[2][64];   // their schedules plus round constants
+  uint32_t slow;        // not in the usual state (set by FsStep::begin)
+};
+
+// Named barriers of a step; 0 is __syncthreads.
+constexpr uint32_t kFsWords = 8, kFsSecond = 12;  // 9, 10, 11: 16 schedule words each
+__device__ __forceinline__ void fs_wait(uint32_t id, uint32_t threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void fs_arrive(uint32_t id, uint32_t threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// 64 rounds on s from schedule words with their constants added, 16 at a time; with `chunked`
+// the words past the first 16 are waited for as they come.
+__device__ __forceinline__ void fs_rounds(uint32_t (&s)[8], const uint32_t* kw, bool chunked) {
+  uint32_t a = s[0], b = s[1], c = s[2], d = s[3], e = s[4], f = s[5], g = s[6], h = s[7];
+#pragma unroll 1
+  for (uint32_t it = 0; it < 4; it++) {
+    if (chunked && it) fs_wait(kFsWords + it, 64);
+    uint4 k4[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) k4[i] = reinterpret_cast<const uint4*>(kw + 16 * it)[i];
+    const uint32_t* k = reinterpret_cast<const uint32_t*>(k4);
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+      const uint32_t S1 = rotr32(e, 6) ^ rotr32(e, 11) ^ rotr32(e, 25);
+      const uint32_t ch = (e & f) ^ (~e & g);
+      const uint32_t S0 = rotr32(a, 2) ^ rotr32(a, 13) ^ rotr32(a, 22);
+      const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
+      const uint32_t y = ch + (h + k[t]);
+      const uint32_t ne = (d + y) + S1, na = (y + S1) + (S0 + mj);
+      h = g;
+      g = f;
+      f = e;
+      e = ne;
+      d = c;
+      c = b;
+      b = a;
+      a = na;
+    }
+  }
+  s[0] += a;
+  s[1] += b;
+  s[2] += c;
+  s[3] += d;
+  s[4] += e;
+  s[5] += f;
+  s[6] += g;
+  s[7] += h;
+}
+
+// Warp 1 (block = 0) and warp 2 (block = 1) of a step.
+static __device__ __noinline__ void fs_schedule(FsShared& sh, uint32_t block) {
+  fs_wait(kFsWords, kFsThreads);
+  uint32_t w[16];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint4 v = reinterpret_cast<const uint4*>(sh.words + 16 * block)[i];
+    w[4 * i] = v.x;
+    w[4 * i + 1] = v.y;
+    w[4 * i + 2] = v.z;
+    w[4 * i + 3] = v.w;
+  }
+#pragma unroll 1
+  for (uint32_t it = 1; it < 4; it++) {
+    uint32_t o[16];
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+      const uint32_t w15 = w[(t + 1) & 15], w2 = w[(t + 14) & 15];
+      const uint32_t s0 = rotr32(w15, 7) ^ rotr32(w15, 18) ^ (w15 >> 3);
+      const uint32_t s1 = rotr32(w2, 17) ^ rotr32(w2, 19) ^ (w2 >> 10);
+      w[t] = w[t] + s0 + w[(t + 9) & 15] + s1;
+      o[t] = w[t] + kSha256K[16 * it + t];
+    }
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        reinterpret_cast<uint4*>(sh.kw[block] + 16 * it)[i] =
+            make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+    }
+    if (block == 0) fs_arrive(kFsWords + it, 64);
+  }
+  if (block) fs_arrive(kFsSecond, 64);
+}
+
+// Warp 0's side: every lane holds the same values.
+struct FsStep {
+  uint32_t k16;  // round constant lane mod 16
+  uint32_t index, tape_len, tape_cap, error;
+
+  // Before a barrier of the block, after which every warp reads sh.slow.
+  __device__ __forceinline__ void begin(FsShared& sh, const TranscriptState* g) {
+    const uint32_t lane = threadIdx.x & 31;
+    k16 = kSha256K[lane & 15];
+    index = g->index;
+    tape_len = g->tape_len;
+    tape_cap = g->tape_cap;
+    error = g->error;
+    if (lane < 8) sh.words[lane] = g->w[lane];
+    if (lane == 0)
+      sh.slow = !(g->block_len == 32 && g->total == 32 && g->sampling && (tape_len & 3u) == 0);
+  }
+
+  // The step from a state that is not the usual one: the transcript as begin() found it.
+  __device__ __noinline__ uint4 step_slow(FsShared& sh, const TranscriptState* g, uint8_t* tape,
+                                          const uint4* msg, uint32_t n) {
+    DevTr st;
+    st.load(g);
+    st.message_elems(tape, msg, n);
+    const uint4 r = st.sample_elem();
+    if ((threadIdx.x & 31) == 0)
+      for (int i = 0; i < 8; i++) sh.words[i] = st.w[i];
+    index = st.index;
+    tape_len = st.tape_len;
+    error = st.error;
+    __syncwarp();
+    return r;
+  }
+
+  // n <= 4 elements.  `slow` (the block's first step, when sh.slow was set): fs_help does nothing.
+  __device__ __forceinline__ uint4 step(FsShared& sh, const TranscriptState* g, uint8_t* tape,
+                                        const uint4* msg, uint32_t n, bool slow) {
+    if (slow) return step_slow(sh, g, tape, msg, n);
+    const uint32_t lane = threadIdx.x & 31;
+    if (lane == 0) {
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        if ((uint32_t)e >= n) break;
+        uint2* w = reinterpret_cast<uint2*>(sh.words + 10 + 4 * e);
+        w[0] = make_uint2(bswap32(msg[e].x), bswap32(msg[e].y));
+        w[1] = make_uint2(bswap32(msg[e].z), bswap32(msg[e].w));
+      }
+    }
+    __syncwarp();
+    const uint32_t end = 10 + 4 * n;
+    uint32_t x = sh.words[lane];
+    if (lane == 8) x = bswap32(index);
+    if (lane == 9) x = 0;
+    if (tape_len + 16 * n > tape_cap) {
+      error = 1;
+    } else {
+      if (lane >= 10 && lane < end) {
+        const uint32_t at = tape_len + 4 * (lane - 10);
+        if ((tape_len & 3u) == 0) {
+          *reinterpret_cast<uint32_t*>(tape + at) = bswap32(x);
+        } else {
+          for (int i = 0; i < 4; i++) tape[at + i] = (uint8_t)(x >> (24 - 8 * i));
+        }
+      }
+      tape_len += 16 * n;
+    }
+    if (lane == end) x = 0x80000000u;
+    if (lane > end) x = lane == 31 ? 32 * end : 0u;
+    sh.words[lane] = x;
+    sh.kw[lane >> 4][lane & 15] = x + k16;
+    fs_wait(kFsWords, kFsThreads);
+    uint32_t s[8];
+    sha256_init(s);
+    fs_rounds(s, sh.kw[0], true);
+    fs_wait(kFsSecond, 64);
+    fs_rounds(s, sh.kw[1], false);
+    if (lane == 0) {
+      reinterpret_cast<uint4*>(sh.words)[0] = make_uint4(s[0], s[1], s[2], s[3]);
+      reinterpret_cast<uint4*>(sh.words)[1] = make_uint4(s[4], s[5], s[6], s[7]);
+    }
+    __syncwarp();
+    index = 16;
+    return make_uint4(bswap32(s[0]), bswap32(s[1]), bswap32(s[2]), bswap32(s[3]));
+  }
+
+  // After at least one step.
+  __device__ __forceinline__ void end(const FsShared& sh, TranscriptState* g) const {
+    const uint32_t lane = threadIdx.x & 31;
+    if (lane < 8) {
+      uint32_t iv[8];
+      sha256_init(iv);
+      uint32_t v = iv[0];
+#pragma unroll
+      for (int i = 1; i < 8; i++) v = lane == (uint32_t)i ? iv[i] : v;
+      g->h[lane] = v;
+      g->w[lane] = sh.words[lane];
+      g->buf[lane] = bswap32(sh.words[lane]);
+    }
+    if (lane == 0) {
+      g->block_len = 32;
+      g->total = 32;
+      g->sampling = 1;
+      g->index = index;
+      g->tape_len = tape_len;
+      g->error = error;
+    }
+  }
+};
+
+// The other warps of the block during a step.
+__device__ __forceinline__ void fs_help(FsShared& sh, bool slow) {
+  const uint32_t warp = threadIdx.x / 32;
+  if (!slow && (warp == 1 || warp == 2)) fs_schedule(sh, warp - 1);
+}
 
 // Host side of one device stretch.  begin() hands the host transcript's state to the device;
 // kernels advance state() and write to tape(); read() queues the copy-back of the state and of

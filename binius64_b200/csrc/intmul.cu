@@ -374,6 +374,9 @@ __global__ void __launch_bounds__(kImFinishThreads)
   pdl_trigger();
   __shared__ uint4 s_prime[kImMaxClaims][3];
   __shared__ uint4 s_r;
+  __shared__ FsShared fs;
+  FsStep st;
+  if (threadIdx.x < 32) st.begin(fs, ts);
   uint4 acc[4] = {gf_zero(), gf_zero(), gf_zero(), gf_zero()};
   for (uint32_t i = threadIdx.x; i < n_claims; i += blockDim.x) {
     const ImClaim c = claims[i];
@@ -401,16 +404,14 @@ __global__ void __launch_bounds__(kImFinishThreads)
   }
   block_xor_sum<4>(acc);
   if (threadIdx.x < 32) {
-    DevTr st;
-    st.load(ts);
-    st.message_elems(tape, acc, msg_coeffs);
-    const uint4 r = st.sample_elem();
-    __syncwarp();
+    const uint4 r = st.step(fs, ts, tape, acc, msg_coeffs, fs.slow);
     if (threadIdx.x == 0) {
       *r_out = r;
-      st.store(ts);
       s_r = r;
     }
+    st.end(fs, ts);
+  } else {
+    fs_help(fs, fs.slow);
   }
   __syncthreads();
   const uint4 r = s_r;
@@ -446,7 +447,8 @@ __global__ void __launch_bounds__(kImTailThreads)
   pdl_wait();
   pdl_trigger();
   __shared__ uint4 r_sh;
-  DevTr st;
+  __shared__ FsShared fs;
+  FsStep st;
   uint4 G = gf_zero(), pf = gf_zero();
   {
     uint4 v[1] = {gf_zero()};
@@ -456,11 +458,12 @@ __global__ void __launch_bounds__(kImTailThreads)
     if (threadIdx.x < 32) {
       G = v[0];
       pf = prefix[0];
-      st.load(ts);
+      st.begin(fs, ts);
       if (t0 > 0) r_sh = chal[t0 - 1];
     }
     __syncthreads();
   }
+  const bool slow = fs.slow;
   for (uint32_t t = t0; t < n; t++) {
     const bool fold = t > 0;
     const uint4 r = r_sh;
@@ -498,18 +501,19 @@ __global__ void __launch_bounds__(kImTailThreads)
       const uint4 m[3] = {gf_mul_warp(pf, gf_mul_warp(oma, T0)),
                           gf_mul_warp(pf, gf_add(gf_mul_warp(oma, T1), T0)),
                           gf_mul_warp(pf, gf_add(gf_mul_warp(oma, T2), T1))};
-      st.message_elems(tape, m, 3);
-      const uint4 rr = st.sample_elem();
+      const uint4 rr = st.step(fs, ts, tape, m, 3, slow && t == t0);
       chal[t] = rr;
       G = gf_add(T0, gf_mul_warp(rr, gf_add(T1, gf_mul_warp(rr, T2))));
       uint4 f = gf_add(rr, al.alpha);
       f.x ^= 1u;
       pf = gf_mul_warp(pf, f);
       r_sh = rr;
+    } else {
+      fs_help(fs, slow && t == t0);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) st.store(ts);
+  if (threadIdx.x < 32 && t0 < n) st.end(fs, ts);
 }
 
 // The small last rounds of the leaf batch (IntMulDevice phase 5) in one CTA, from round t0 on,
@@ -532,7 +536,8 @@ __global__ void __launch_bounds__(kImTailThreads)
   pdl_trigger();
   constexpr uint32_t kClaims0 = kLeafPairs + 1, kClaims = kClaims0 + kLeafCols;
   __shared__ uint4 r_sh;
-  DevTr st;
+  __shared__ FsShared fs;
+  FsStep st;
   uint4 G[2] = {gf_zero(), gf_zero()}, pf[2] = {gf_zero(), gf_zero()};
   {
     uint4 v[2] = {gf_zero(), gf_zero()};
@@ -544,11 +549,12 @@ __global__ void __launch_bounds__(kImTailThreads)
       G[1] = v[1];
       pf[0] = prefix[0];
       pf[1] = prefix[1];
-      st.load(ts);
+      st.begin(fs, ts);
       if (t0 > 0) r_sh = chal[t0 - 1];
     }
     __syncthreads();
   }
+  const bool slow = fs.slow;
   auto fold2 = [](uint4* col, uint64_t i, uint64_t L, uint64_t h, uint4 r, bool fold,
                   uint4& x0, uint4& x1) {
     x0 = col[i];
@@ -601,8 +607,7 @@ __global__ void __launch_bounds__(kImTailThreads)
         gf_add_into(m3[1], gf_mul_warp(pf[g], gf_add(gf_mul_warp(oma, T[g][1]), T[g][0])));
         gf_add_into(m3[2], gf_mul_warp(pf[g], gf_add(gf_mul_warp(oma, T[g][2]), T[g][1])));
       }
-      st.message_elems(tape, m3, 3);
-      const uint4 rr = st.sample_elem();
+      const uint4 rr = st.step(fs, ts, tape, m3, 3, slow && t == t0);
       chal[t] = rr;
       for (int g = 0; g < 2; g++) {
         G[g] = gf_add(T[g][0], gf_mul_warp(rr, gf_add(T[g][1], gf_mul_warp(rr, T[g][2]))));
@@ -611,10 +616,12 @@ __global__ void __launch_bounds__(kImTailThreads)
         pf[g] = gf_mul_warp(pf[g], f);
       }
       r_sh = rr;
+    } else {
+      fs_help(fs, slow && t == t0);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) st.store(ts);
+  if (threadIdx.x < 32 && t0 < n) st.end(fs, ts);
 }
 
 // ---------------------------------------------------------------- host side

@@ -372,16 +372,22 @@ struct ShiftRoundConst {
 // times the in/out check's Gruen-scaled (d_0, d_1) (MleToSumCheckDecorator + batch_prove); then r
 // is sampled and the three running values advance.  When init_lohi is set (the first round) the
 // in/out claim is first set to lo + (hi - lo) z0 from it.  One warp runs the step.
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kFsThreads)
     shift_round_finish_kernel(TranscriptState* __restrict__ ts, uint8_t* __restrict__ tape,
                               const uint4* __restrict__ ys, const ShiftRoundConst* __restrict__ rc,
                               const uint4* __restrict__ init_lohi, uint4 z0, uint4 beta,
                               uint4* __restrict__ st3, uint4* __restrict__ r_out) {
   pdl_wait();
   pdl_trigger();
+  __shared__ FsShared fs;
+  FsStep st;
+  if (threadIdx.x < 32) st.begin(fs, ts);
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    fs_help(fs, fs.slow);
+    return;
+  }
   {
-    DevTr st;
-    st.load(ts);
     const ShiftRoundConst c = *rc;
     uint4 inout = st3[1];
     if (init_lohi)
@@ -403,15 +409,14 @@ __global__ void __launch_bounds__(32)
     const uint4 d0 = gf_mul_warp(gf_mul_warp(q0, one_a), eqp);
     const uint4 d1 = gf_mul_warp(gf_add(gf_mul_warp(q1, one_a), q0), eqp);
     const uint4 msg[2] = {gf_add(s0, gf_mul_warp(beta, d0)), gf_add(s1, gf_mul_warp(beta, d1))};
-    st.message_elems(tape, msg, 2);
-    const uint4 r = st.sample_elem();
+    const uint4 r = st.step(fs, ts, tape, msg, 2, fs.slow);
     *r_out = r;
     st3[0] = gf_add(s0, gf_mul_warp(r, gf_add(s1, gf_mul_warp(s2, r))));
     st3[1] = gf_add(q0, gf_mul_warp(q1, r));
     uint4 f = gf_add(r, c.alpha_dec);
     f.x ^= 1u;
     st3[2] = gf_mul_warp(eqp, f);
-    st.store(ts);
+    st.end(fs, ts);
   }
 }
 
@@ -432,16 +437,18 @@ __global__ void __launch_bounds__(kShiftTailThreads)
   pdl_wait();
   pdl_trigger();
   __shared__ uint4 r_sh;
-  DevTr st;
+  __shared__ FsShared fs;
+  FsStep st;
   uint4 sum = gf_zero(), inout = gf_zero(), eqp = gf_zero();
   if (threadIdx.x < 32) {
-    st.load(ts);
+    st.begin(fs, ts);
     sum = run[0];
     inout = run[1];
     eqp = run[2];
     r_sh = *r_first;
   }
   __syncthreads();
+  const bool slow = fs.slow;
   for (uint32_t k = 0, n_rem = n_rem0; n_rem > 0; k++, n_rem--) {
     const uint4 r = r_sh;
     const uint64_t h = 1ull << n_rem, half = h >> 1;
@@ -486,8 +493,7 @@ __global__ void __launch_bounds__(kShiftTailThreads)
       const uint4 d0 = gf_mul_warp(gf_mul_warp(q0, one_a), eqp);
       const uint4 d1 = gf_mul_warp(gf_add(gf_mul_warp(q1, one_a), q0), eqp);
       const uint4 msg[2] = {gf_add(s0, gf_mul_warp(beta, d0)), gf_add(s1, gf_mul_warp(beta, d1))};
-      st.message_elems(tape, msg, 2);
-      const uint4 rr = st.sample_elem();
+      const uint4 rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
       chal[k] = rr;
       sum = gf_add(s0, gf_mul_warp(rr, gf_add(s1, gf_mul_warp(s2, rr))));
       inout = gf_add(q0, gf_mul_warp(q1, rr));
@@ -495,11 +501,13 @@ __global__ void __launch_bounds__(kShiftTailThreads)
       f.x ^= 1u;
       eqp = gf_mul_warp(eqp, f);
       r_sh = rr;
+    } else {
+      fs_help(fs, slow && k == 0);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    st.store(ts);
+  if (threadIdx.x < 32 && n_rem0) {
+    st.end(fs, ts);
     run[0] = sum;
     run[1] = inout;
     run[2] = eqp;
@@ -800,7 +808,7 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
       SHIFT_TRY(dot2(half, half, half, ys + 2));
     }
     if (n_rem <= p) gn--;
-    BGPU_CUDA(launch_pdl(shift_round_finish_kernel, 1, 32, 0, s, dt.state(), dt.tape(),
+    BGPU_CUDA(launch_pdl(shift_round_finish_kernel, 1, kFsThreads, 0, s, dt.state(), dt.tape(),
                          (const uint4*)ys, (const ShiftRoundConst*)(rconst + k),
                          n_rem == log_words ? (const uint4*)init_lohi : (const uint4*)nullptr, z0,
                          u4(beta), run, chal + 12 + k));

@@ -254,31 +254,35 @@ __global__ void __launch_bounds__(kThreads)
 // message is (c_0, c_1), then optionally a 32-byte commitment (a Merkle root the device just
 // built), then the challenge r is sampled and the claim becomes c_0 + c_1 r + c_2 r^2.  The claim
 // is read from claim_init when that is set (the first round).  One warp runs the step.
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kFsThreads)
     bivariate_round_finish_kernel(TranscriptState* __restrict__ ts, uint8_t* __restrict__ tape,
                                   const uint4* __restrict__ ys, const uint4* __restrict__ claim_init,
                                   uint4* __restrict__ claim, const uint8_t* __restrict__ commitment,
                                   uint4* __restrict__ r_out) {
   pdl_wait();
   pdl_trigger();
-  {
-    DevTr st;
-    st.load(ts);
-    const uint4 y1 = ys[0], yinf = ys[1];
-    const uint4 c0 = gf_add(claim_init ? *claim_init : *claim, y1), c2 = yinf;
-    const uint4 c1 = gf_add(gf_add(y1, c0), c2);
-    const uint4 msg[2] = {c0, c1};
-    st.message_elems(tape, msg, 2);
-    if (commitment) {
-      uint32_t root[8];
-      for (int i = 0; i < 8; i++) root[i] = reinterpret_cast<const uint32_t*>(commitment)[i];
-      st.message_words(tape, root, 8);
-    }
-    const uint4 r = st.sample_elem();
-    *r_out = r;
-    *claim = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
-    st.store(ts);
+  __shared__ FsShared fs;
+  FsStep st;
+  if (threadIdx.x < 32) st.begin(fs, ts);
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    fs_help(fs, fs.slow);
+    return;
   }
+  const uint4 y1 = ys[0], yinf = ys[1];
+  const uint4 c0 = gf_add(claim_init ? *claim_init : *claim, y1), c2 = yinf;
+  const uint4 c1 = gf_add(gf_add(y1, c0), c2);
+  uint4 msg[4] = {c0, c1, gf_zero(), gf_zero()};
+  if (commitment) {
+    uint32_t root[8];
+    for (int i = 0; i < 8; i++) root[i] = reinterpret_cast<const uint32_t*>(commitment)[i];
+    msg[2] = make_uint4(root[0], root[1], root[2], root[3]);
+    msg[3] = make_uint4(root[4], root[5], root[6], root[7]);
+  }
+  const uint4 r = st.step(fs, ts, tape, msg, commitment ? 4 : 2, fs.slow);
+  *r_out = r;
+  *claim = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
+  st.end(fs, ts);
 }
 
 // The small last rounds of a plain bivariate product sumcheck in one CTA: per round, fold (a, b)
@@ -295,14 +299,16 @@ __global__ void __launch_bounds__(kTailThreads)
   pdl_wait();
   pdl_trigger();
   __shared__ uint4 r_sh;
-  DevTr st;
+  __shared__ FsShared fs;
+  FsStep st;
   uint4 cl = gf_zero();
   if (threadIdx.x < 32) {
-    st.load(ts);
+    st.begin(fs, ts);
     cl = *claim;
     if (r_first) r_sh = *r_first;
   }
   __syncthreads();
+  const bool slow = fs.slow;
   for (uint32_t k = 0; k < n_rounds; k++) {
     if (k > 0 || r_first) {
       const uint4 r = r_sh;
@@ -327,16 +333,17 @@ __global__ void __launch_bounds__(kTailThreads)
       const uint4 y1 = v[0], yinf = v[1];
       const uint4 c0 = gf_add(cl, y1), c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
       const uint4 msg[2] = {c0, c1};
-      st.message_elems(tape, msg, 2);
-      const uint4 r = st.sample_elem();
+      const uint4 r = st.step(fs, ts, tape, msg, 2, slow && k == 0);
       chal[k] = r;
       cl = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
       r_sh = r;
+    } else {
+      fs_help(fs, slow && k == 0);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    st.store(ts);
+  if (threadIdx.x < 32 && n_rounds) {
+    st.end(fs, ts);
     *claim = cl;
   }
 }
@@ -454,7 +461,7 @@ int bivariate_fold_eval_dev(uint4* d_a, uint4* d_b, uint64_t size, const uint4* 
 int bivariate_round_finish(const DeviceTranscript& dt, const uint4* d_ys, const uint4* d_claim_init,
                            uint4* d_claim, const uint8_t* d_commitment, uint4* d_r_out,
                            cudaStream_t s) {
-  cudaError_t e = launch_pdl(bivariate_round_finish_kernel, 1, 32, 0, s, dt.state(), dt.tape(),
+  cudaError_t e = launch_pdl(bivariate_round_finish_kernel, 1, kFsThreads, 0, s, dt.state(), dt.tape(),
                              d_ys, d_claim_init, d_claim, d_commitment, d_r_out);
   if (e != cudaSuccess) return cuda_error(e, "bivariate_round_finish_kernel");
   count_launch();
