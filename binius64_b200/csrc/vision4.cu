@@ -20,10 +20,11 @@
 //    x; the tables are stored as four 32-bit planes so a warp's lookups of one nibble position
 //    fall into 16 consecutive words of shared memory (no bank conflicts).
 // Six maps x 8 KiB of tables + the round constants stay in shared memory for the kernel's life.
-// Trees of up to 2^12 leaves (the FRI fold rounds') run one permutation over four lanes instead,
-// which shortens the chain of dependent permutations they are made of (see the lane kernels).
+// Trees of up to 2^12 leaves (the FRI fold rounds') run one permutation over four warps instead,
+// which shortens the chain of dependent permutations they are made of (see the warp kernels).
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -187,6 +188,55 @@ int device_image(const uint4** out) {
     void* d = nullptr;
     BGPU_CUDA(cudaMalloc(&d, kImageBytes));
     BGPU_CUDA(cudaMemcpy(d, img.data(), kImageBytes, cudaMemcpyHostToDevice));
+    images[dev] = static_cast<const uint4*>(d);
+  }
+  *out = images[dev];
+  return BINIUS_OK;
+}
+
+// The image of the warp kernels: the maps of their inversion chain and the two affine maps after
+// its last squaring, as 16-byte rows [nibble position][nibble value], then the same constants.
+enum : uint32_t {
+  kWarpSq1 = 0, kWarpSq3, kWarpSq6, kWarpSq12, kWarpSq24, kWarpSq48, kWarpLinv, kWarpLfwd, kWarpMaps
+};
+constexpr uint32_t kWarpMapRows = 32 * 16;
+constexpr uint32_t kWarpRcOff = kWarpMaps * kWarpMapRows;
+constexpr uint32_t kWarpC0Off = kWarpRcOff + 17 * 4, kWarpBinv0Off = kWarpC0Off + 1;
+constexpr size_t kWarpImageBytes = 16 * (kWarpBinv0Off + 1);
+
+int device_warp_image(const uint4** out) {
+  static std::mutex mu;
+  static const uint4* images[64] = {};
+  int dev = 0;
+  BGPU_CUDA(cudaGetDevice(&dev));
+  BGPU_ARG(dev >= 0 && dev < 64, "device ordinal out of range");
+  std::lock_guard<std::mutex> g(mu);
+  if (!images[dev]) {
+    const HostParams& p = host_params();
+    std::vector<uint32_t> img(kWarpImageBytes / 4, 0);
+    const uint32_t sq_k[6] = {1, 3, 6, 12, 24, 48};
+    for (uint32_t m = 0; m < kWarpMaps; m++) {
+      hu128 cols[128];
+      for (int i = 0; i < 128; i++) {
+        hu128 x = (hu128)1 << i;
+        for (uint32_t k = 0; k < (m < 6 ? sq_k[m] : 1); k++) x = host_gf_mul(x, x);
+        if (m >= 6) x = apply_cols(p.cols[m == kWarpLinv ? kMapLinv : kMapLfwd], x);
+        cols[i] = x;
+      }
+      for (uint32_t row = 0; row < kWarpMapRows; row++) {
+        hu128 v = 0;
+        for (int b = 0; b < 4; b++)
+          if ((row >> b) & 1) v ^= cols[4 * (row / 16) + b];
+        put_elem(&img[4 * (m * kWarpMapRows + row)], v);
+      }
+    }
+    for (int r = 0; r < 17; r++)
+      for (int i = 0; i < 4; i++) put_elem(&img[4 * (kWarpRcOff + 4 * r + i)], p.rc[r][i]);
+    put_elem(&img[4 * kWarpC0Off], kBFwd[0]);
+    put_elem(&img[4 * kWarpBinv0Off], p.binv0);
+    void* d = nullptr;
+    BGPU_CUDA(cudaMalloc(&d, kWarpImageBytes));
+    BGPU_CUDA(cudaMemcpy(d, img.data(), kWarpImageBytes, cudaMemcpyHostToDevice));
     images[dev] = static_cast<const uint4*>(d);
   }
   *out = images[dev];
@@ -432,137 +482,159 @@ __global__ void __launch_bounds__(kV4Threads, 2)
   }
 }
 
-// ---- small trees: one permutation over four lanes
+// ---- small trees: one permutation over four warps
 //
-// A tree of few leaves cannot fill the GPU, so its time is the chain of dependent permutations
-// (a leaf's sponge, then one per layer) on single threads.  Here four consecutive lanes hold one
-// state, element e = lane & 3 each: every lane inverts its own element (four inversions instead
-// of Montgomery's one, but nothing of the sbox waits for another element) and applies B or B^-1;
-// the MDS combines the four elements by shuffles.  About half the instructions of one thread's
-// permutation sit on the chain.
+// A tree of few leaves cannot fill the GPU, so its time is the chain of dependent permutations: a
+// leaf's sponge (more than a hundred for a leaf of an FRI tree of high arity), then one per layer.
+// Here a group of four warps holds one state, a warp per element
+// with all its lanes holding the same value, so every product (gf_mul_lanes) and every linear map
+// (one nibble per lane, the 32 rows XORed by warp reductions) is spread over a warp.  An inversion
+// a^(2^128 - 2) is the chain b_(i+j) = b_i^(2^j) b_j, b_k = a^(2^k - 1), over k = 1, 2, 3, 6, 12,
+// 24, 48, 96, 120, 126, 127: ten maps and ten products, the last squaring taken into the affine
+// map after it.  The MDS reads the other elements through shared memory, one barrier of the group
+// per half round.
+//
+// A permutation's chain takes 27 us (a product 160 cycles, a map 110; their warp reductions are
+// a third), against 180 us with four lanes per state (the form before).  Measured, that form ->
+// this: 2^6 leaves of 2^7 elements 12.8 -> 2.0 ms, 2^6 of 2^4 2.76 -> 0.47, 2^8 of 2^4 3.13 -> 0.58,
+// 2^10 of 2^4 3.49 -> 1.21, 2^12 of 2^4 3.87 -> 3.45.  A permutation costs ten times the
+// instructions of a one-thread permutation, so from 2^13 leaves (6.54 ms here) the one-thread
+// kernels are at least as fast.
+constexpr uint32_t kWarpMaxLog = 12;
+constexpr uint32_t kGroupLanes = 128;
+constexpr uint32_t kWarpFuse = 2;  // 2^2 leaves (16 warps), or inputs, per CTA
 
-__device__ __forceinline__ uint4 shfl_xor_gf(uint4 v, int m) {
-  return make_uint4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
-                    __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m));
+__device__ __forceinline__ uint4 v4w_map(uint32_t m, uint4 x) {
+  const uint32_t l = threadIdx.x & 31;
+  const uint32_t lo = l & 8 ? x.y : x.x, hi = l & 8 ? x.w : x.z, w = l & 16 ? hi : lo;
+  const uint4 row = v4_img[m * kWarpMapRows + l * 16 + ((w >> (4 * (l & 7))) & 15)];
+  return make_uint4(
+      __reduce_xor_sync(0xffffffffu, row.x), __reduce_xor_sync(0xffffffffu, row.y),
+      __reduce_xor_sync(0xffffffffu, row.z), __reduce_xor_sync(0xffffffffu, row.w));
 }
 
-__device__ __forceinline__ uint4 shfl_gf(uint4 v, int src) {
-  return make_uint4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-                    __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
-}
-
-// The permutation of the state held by this lane's group of four; returns element e.  Every lane
-// of the warp calls it together.
-static __device__ __noinline__ uint4 v4_permute_lane(uint4 x, uint32_t e) {
-  const uint32_t next = (threadIdx.x & 31u & ~3u) | ((e + 1) & 3u);
-  x = gf_add(x, v4_img[kRcOff + e]);
+// The permutation of the group's state; this warp's element e.  `mix` is the group's two sets of
+// four elements in shared memory, `bar` its named barrier.  The whole group calls it.
+static __device__ __noinline__ uint4 v4w_permute(uint4 x, uint32_t e, uint4* mix, uint32_t bar) {
+  x = gf_add(x, v4_img[kWarpRcOff + e]);
 #pragma unroll 1
   for (uint32_t h = 0; h < 16; h++) {
+    // (the product masks its first factor's bits, which are at hand before the map is)
+    const uint4 b3 = gf_mul_lanes(x, v4w_map(kWarpSq1, gf_mul_lanes(x, v4w_map(kWarpSq1, x))));
+    const uint4 b6 = gf_mul_lanes(b3, v4w_map(kWarpSq3, b3));
+    const uint4 b12 = gf_mul_lanes(b6, v4w_map(kWarpSq6, b6));
+    const uint4 b24 = gf_mul_lanes(b12, v4w_map(kWarpSq12, b12));
+    const uint4 b48 = gf_mul_lanes(b24, v4w_map(kWarpSq24, b24));
+    const uint4 b96 = gf_mul_lanes(b48, v4w_map(kWarpSq48, b48));
+    const uint4 b120 = gf_mul_lanes(b24, v4w_map(kWarpSq24, b96));
+    const uint4 b126 = gf_mul_lanes(b6, v4w_map(kWarpSq6, b120));
+    const uint4 b127 = gf_mul_lanes(x, v4w_map(kWarpSq1, b126));
     const bool inverse = (h & 1) == 0;
-    x = gf_add(v4_map(inverse ? kMapLinv : kMapLfwd, v4_inv(x)),
-               v4_img[inverse ? kBinv0Off : kC0Off]);
+    x = gf_add(v4w_map(inverse ? kWarpLinv : kWarpLfwd, b127),
+               v4_img[inverse ? kWarpBinv0Off : kWarpC0Off]);
     // MDS: x_e += (x_0 + x_1 + x_2 + x_3) + 2 (x_e + x_{e+1 mod 4}), all from the old values
-    const uint4 s1 = gf_add(x, shfl_xor_gf(x, 1));
-    const uint4 sum = gf_add(s1, shfl_xor_gf(s1, 2));
-    const uint4 nx = shfl_gf(x, (int)next);
-    x = gf_add(gf_add(x, sum), mul_x(gf_add(x, nx)));
-    x = gf_add(x, v4_img[kRcOff + 4 * (h + 1) + e]);
+    uint4* s = mix + 4 * (h & 1);
+    if ((threadIdx.x & 31) == 0) s[e] = x;
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kGroupLanes) : "memory");
+    const uint4 sum = gf_add(gf_add(s[0], s[1]), gf_add(s[2], s[3]));
+    x = gf_add(gf_add(x, sum), mul_x(gf_add(x, s[(e + 1) & 3])));
+    x = gf_add(x, v4_img[kWarpRcOff + 4 * (h + 1) + e]);
   }
   return x;
 }
 
-// Small CTAs (16 leaves = 2 warps; 16 inputs = 1 warp): the trees are too small to fill the GPU,
-// so spreading them over many SMs leaves each chain a scheduler of its own.
-constexpr uint32_t kLaneLeafFuse = 4;  // 2^4 leaves (64 lanes) per CTA
-constexpr uint32_t kLaneNodeFuse = 4;  // 2^4 inputs per CTA
-// Trees of up to 2^12 leaves take the four-lane kernels.  Measured: 2^14 leaves on them took
-// 9.7 ms against 8.4 ms on the one-thread kernels (four inversions per sbox cost more than the
-// SMs the one-thread kernels leave idle).
-constexpr uint32_t kLaneMaxLog = 12;
+__device__ __forceinline__ void v4w_load_image(const uint4* __restrict__ g) {
+  for (uint32_t i = threadIdx.x; i < kWarpImageBytes / 16; i += blockDim.x) v4_img[i] = g[i];
+  __syncthreads();
+}
+// After the image: per group of the CTA its mix sets, then [2][inputs][2] node elements.
+constexpr size_t kWarpSmem = kWarpImageBytes + 16 * ((8 + 2 * 2) << kWarpFuse);
 
-__global__ void __launch_bounds__(256)
-    vision4_leaves_lanes_kernel(const uint4* __restrict__ img, const uint4* __restrict__ elems,
-                                uint32_t log_batch, uint4* __restrict__ nodes, uint32_t L,
-                                uint32_t fused) {
-  v4_load_image(img);
-  uint4* buf = v4_nodes_buf();
-  const uint32_t e = threadIdx.x & 3, item = threadIdx.x >> 2, n0 = 1u << fused;
-  const bool valid = item < n0;  // lanes past the CTA's leaves compute along for the shuffles
-  const uint64_t leaf = (uint64_t)blockIdx.x * n0 + (valid ? item : 0);
+// MMO compressions of a CTA's n_in nodes (their elements at buf), `fused` layers up; layer `level`
+// is the nodes'.  Group g compresses node g of each layer.
+__device__ __forceinline__ void v4w_layers(uint4* buf, uint32_t n_in, uint32_t fused,
+                                           uint4* __restrict__ nodes, uint32_t L, uint32_t level,
+                                           uint32_t group, uint32_t e, uint4* mix) {
+  for (uint32_t lvl = 1; lvl <= fused; lvl++) {
+    __syncthreads();
+    const uint32_t n = n_in >> lvl;
+    const uint32_t src = ((lvl - 1) & 1) * (2u << kWarpFuse), dst = (lvl & 1) * (2u << kWarpFuse);
+    if (group >= n) continue;
+    const uint4 in = buf[src + 4 * group + e];
+    const uint4 o = gf_add(v4w_permute(in, e, mix, group + 1), in);
+    if (e < 2 && (threadIdx.x & 31) == 0) {
+      buf[dst + 2 * group + e] = o;
+      nodes[2 * (layer_offset(L, level + lvl) + (uint64_t)blockIdx.x * n + group) + e] = o;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kGroupLanes << kWarpFuse)
+    vision4_leaves_warp_kernel(const uint4* __restrict__ img, const uint4* __restrict__ elems,
+                               uint32_t log_batch, uint4* __restrict__ nodes, uint32_t L,
+                               uint32_t fused) {
+  v4w_load_image(img);
+  const uint32_t group = threadIdx.x / kGroupLanes, e = (threadIdx.x / 32) & 3;
+  uint4* mix = v4_img + kWarpImageBytes / 16 + 8 * group;
+  uint4* buf = v4_img + kWarpImageBytes / 16 + (8u << kWarpFuse);
+  const uint64_t leaf = ((uint64_t)blockIdx.x << fused) + group;
   const uint4* ep = elems + (leaf << log_batch);
   uint4 x = gf_zero();
-  if (log_batch == 0) {
+  if (log_batch == 0) {  // 16 bytes: one block with the padding in its second half
     if (e == 0) x = ep[0];
     if (e == 1) x = make_uint4(0x80u, 0u, 0u, 0x01000000u);
-    x = v4_permute_lane(x, e);
+    x = v4w_permute(x, e, mix, group + 1);
   } else {
     const uint32_t blocks = 1u << (log_batch - 1);
+    uint4 next = e < 2 ? ep[e] : gf_zero();
 #pragma unroll 1
     for (uint32_t j = 0; j < blocks; j++) {
-      if (e < 2) x = ep[2 * j + e];
-      x = v4_permute_lane(x, e);
+      if (e < 2) {  // absorb: the block overwrites elements 0 and 1
+        x = next;
+        if (j + 1 < blocks) next = ep[2 * (j + 1) + e];
+      }
+      x = v4w_permute(x, e, mix, group + 1);
     }
     if (e == 0) x = make_uint4(0x80u, 0u, 0u, 0u);
     if (e == 1) x = make_uint4(0u, 0u, 0u, 0x01000000u);
-    x = v4_permute_lane(x, e);
+    x = v4w_permute(x, e, mix, group + 1);
   }
-  if (valid && e < 2) {
+  if (e < 2 && (threadIdx.x & 31) == 0) {
     nodes[2 * leaf + e] = x;
-    buf[2 * item + e] = x;
+    buf[2 * group + e] = x;
   }
-  for (uint32_t lvl = 1; lvl <= fused; lvl++) {
-    __syncthreads();
-    const uint32_t n = n0 >> lvl;
-    const uint32_t src = ((lvl - 1) & 1) * 2 * kV4Threads, dst = (lvl & 1) * 2 * kV4Threads;
-    const bool act = item < n;
-    const uint4 in = act ? buf[src + 4 * item + e] : gf_zero();
-    const uint4 y = v4_permute_lane(in, e);
-    if (act && e < 2) {
-      const uint4 o = gf_add(y, in);
-      buf[dst + 2 * item + e] = o;
-      nodes[2 * (layer_offset(L, lvl) + (uint64_t)blockIdx.x * n + item) + e] = o;
-    }
-  }
+  v4w_layers(buf, 1u << fused, fused, nodes, L, 0, group, e, mix);
 }
 
-__global__ void __launch_bounds__(256)
-    vision4_nodes_lanes_kernel(const uint4* __restrict__ img, uint4* __restrict__ nodes,
-                               uint32_t L, uint32_t in_level, uint32_t fused) {
-  v4_load_image(img);
-  uint4* buf = v4_nodes_buf();
-  const uint32_t e = threadIdx.x & 3, item = threadIdx.x >> 2, n_in = 1u << fused;
-  const uint64_t in_off = layer_offset(L, in_level) + (uint64_t)blockIdx.x * n_in;
-  for (uint32_t lvl = 1; lvl <= fused; lvl++) {
-    const uint32_t n = n_in >> lvl;
-    const uint32_t src = ((lvl - 1) & 1) * 2 * kV4Threads, dst = (lvl & 1) * 2 * kV4Threads;
-    if (lvl > 1) __syncthreads();
-    const bool act = item < n;
-    uint4 in = gf_zero();
-    if (act) in = lvl == 1 ? nodes[2 * in_off + 4 * item + e] : buf[src + 4 * item + e];
-    const uint4 y = v4_permute_lane(in, e);
-    if (act && e < 2) {
-      const uint4 o = gf_add(y, in);
-      buf[dst + 2 * item + e] = o;
-      nodes[2 * (layer_offset(L, in_level + lvl) + (uint64_t)blockIdx.x * n + item) + e] = o;
-    }
-  }
+__global__ void __launch_bounds__(kGroupLanes << kWarpFuse)
+    vision4_nodes_warp_kernel(const uint4* __restrict__ img, uint4* __restrict__ nodes, uint32_t L,
+                              uint32_t in_level, uint32_t fused) {
+  v4w_load_image(img);
+  const uint32_t group = threadIdx.x / kGroupLanes, e = (threadIdx.x / 32) & 3;
+  uint4* mix = v4_img + kWarpImageBytes / 16 + 8 * group;
+  uint4* buf = v4_img + kWarpImageBytes / 16 + (8u << kWarpFuse);
+  const uint64_t in = layer_offset(L, in_level) + ((uint64_t)blockIdx.x << fused);
+  for (uint32_t i = threadIdx.x; i < (2u << fused); i += blockDim.x) buf[i] = nodes[2 * in + i];
+  v4w_layers(buf, 1u << fused, fused, nodes, L, in_level, group, e, mix);
 }
 
-int vision4_commit_lanes(const uint4* img, const uint4* elems, uint32_t L, uint32_t log_batch,
-                         uint4* nodes, cudaStream_t s) {
-  if (int rc = ensure_smem_limit((const void*)vision4_leaves_lanes_kernel, kV4Smem)) return rc;
-  if (int rc = ensure_smem_limit((const void*)vision4_nodes_lanes_kernel, kV4Smem)) return rc;
-  const uint32_t fused = L < kLaneLeafFuse ? L : kLaneLeafFuse;
-  const uint32_t threads = (4u << fused) < 32u ? 32u : (4u << fused);
-  vision4_leaves_lanes_kernel<<<1u << (L - fused), threads, kV4Smem, s>>>(img, elems, log_batch,
-                                                                        nodes, L, fused);
-  BGPU_LAUNCH_CHECK("vision4_leaves_lanes_kernel");
+int vision4_commit_warps(const uint4* elems, uint32_t L, uint32_t log_batch, uint4* nodes,
+                         cudaStream_t s) {
+  const uint4* img = nullptr;
+  if (int rc = device_warp_image(&img)) return rc;
+  if (int rc = ensure_smem_limit((const void*)vision4_leaves_warp_kernel, kWarpSmem)) return rc;
+  if (int rc = ensure_smem_limit((const void*)vision4_nodes_warp_kernel, kWarpSmem)) return rc;
+  // one group per CTA, and so one warp per scheduler, while the leaves are fewer than the SMs
+  const uint32_t fused = std::min(L > 7 ? L - 7 : 0, kWarpFuse);
+  vision4_leaves_warp_kernel<<<1u << (L - fused), kGroupLanes << fused, kWarpSmem, s>>>(
+      img, elems, log_batch, nodes, L, fused);
+  BGPU_LAUNCH_CHECK("vision4_leaves_warp_kernel");
   count_launch();
   for (uint32_t level = fused; level < L;) {
-    const uint32_t f = (L - level) < kLaneNodeFuse ? (L - level) : kLaneNodeFuse;
-    const uint32_t t = (2u << f) < 32u ? 32u : (2u << f);
-    vision4_nodes_lanes_kernel<<<1u << (L - level - f), t, kV4Smem, s>>>(img, nodes, L, level, f);
-    BGPU_LAUNCH_CHECK("vision4_nodes_lanes_kernel");
+    const uint32_t f = std::min(L - level, kWarpFuse);
+    vision4_nodes_warp_kernel<<<1u << (L - level - f), kGroupLanes << (f - 1), kWarpSmem, s>>>(
+        img, nodes, L, level, f);
+    BGPU_LAUNCH_CHECK("vision4_nodes_warp_kernel");
     count_launch();
     level += f;
   }
@@ -583,8 +655,8 @@ int vision4_merkle_commit(const void* d_elems, uint32_t log_leaves, uint32_t log
   if (int rc = ensure_smem_limit((const void*)vision4_nodes_kernel, kV4Smem)) return rc;
   const uint32_t L = log_leaves;
   uint4* nodes = static_cast<uint4*>(d_nodes);
-  if (L <= kLaneMaxLog)
-    return vision4_commit_lanes(img, static_cast<const uint4*>(d_elems), L, log_batch, nodes, s);
+  if (L <= kWarpMaxLog)
+    return vision4_commit_warps(static_cast<const uint4*>(d_elems), L, log_batch, nodes, s);
   // at least 2^8 CTAs: mid-size trees spread over every SM in smaller CTAs
   const uint32_t fused = L - 8 < kV4LeafFuse ? L - 8 : kV4LeafFuse;
   const uint64_t grid = 1ull << (L - fused);
