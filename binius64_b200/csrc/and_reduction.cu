@@ -521,35 +521,52 @@ __global__ void __launch_bounds__(kAndTailThreads)
   }
   __syncthreads();
   const bool slow = fs.slow;
+  // warp 0, beside the folds: the claim after the last challenge, and what of the round's
+  // interpolation y_0 = (claim + alpha y_1) / (1 + alpha) does not wait for the sums
+  uint4 c0 = gf_zero(), c1 = gf_zero(), c2 = gf_zero(), rr = gf_zero();
+  auto next_claim = [&]() {
+    cl = gf_add(c0, gf_mul_warp(rr, gf_add(c1, gf_mul_warp(c2, rr))));
+  };
   for (uint32_t k = 0; k < n_rounds; k++) {
     const uint4 r = r_sh;
-    const uint64_t h = len >> 1, q = len >> 2;
-    for (uint64_t j = threadIdx.x; j < h; j += blockDim.x) {
-      const uint4 a0 = fa[j], b0 = fb[j], c0 = fc[j];
-      fa[j] = gf_add(a0, gf_mul_nl(r, gf_add(fa[h + j], a0)));
-      fb[j] = gf_add(b0, gf_mul_nl(r, gf_add(fb[h + j], b0)));
-      fc[j] = gf_add(c0, gf_mul_nl(r, gf_add(fc[h + j], c0)));
+    const uint32_t h = (uint32_t)(len >> 1), q = h >> 1;
+    uint4 ci = gf_zero(), ai = gf_zero();
+    if (threadIdx.x < 32) {
+      if (k > 0) next_claim();
+      const AndRoundConst c = rc[k];
+      ci = gf_mul_warp(cl, c.inv_one_plus_alpha);
+      ai = gf_mul_warp(c.alpha, c.inv_one_plus_alpha);
     }
-    for (uint64_t j = threadIdx.x; j < q; j += blockDim.x) eq[j] = gf_add(eq[j], eq[q + j]);
+    block_jobs(3 * h, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t j = job & (h - 1);
+      uint4* x = job < h ? fa : job < 2 * h ? fb : fc;
+      const uint4 x0 = x[j], y = gf_add(x0, mul(r, gf_add(x[h + j], x0)));
+      if (own) x[j] = y;
+    });
+    for (uint32_t j = threadIdx.x; j < q; j += blockDim.x) eq[j] = gf_add(eq[j], eq[q + j]);
     len = h;
     __syncthreads();
     uint4 v[2] = {gf_zero(), gf_zero()};
-    for (uint64_t j = threadIdx.x; j < q; j += blockDim.x) {
-      const uint4 e = eq[j];
-      const uint4 a0 = fa[j], a1 = fa[q + j], b0 = fb[j], b1 = fb[q + j], c1 = fc[q + j];
-      gf_add_into(v[0], gf_mul_nl(e, gf_add(gf_mul_nl(a1, b1), c1)));
-      gf_add_into(v[1], gf_mul_nl(e, gf_mul_nl(gf_add(a0, a1), gf_add(b0, b1))));
-    }
+    block_jobs(2 * q, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t j = job & (q - 1);
+      uint4 x = fa[q + j], y = fb[q + j], z = fc[q + j];
+      if (job >= q) {
+        gf_add_into(x, fa[j]);
+        gf_add_into(y, fb[j]);
+        z = gf_zero();
+      }
+      const uint4 m = mul(eq[j], gf_add(mul(x, y), z));
+      if (own) gf_add_into(job < q ? v[0] : v[1], m);
+    });
     block_xor_sum<2>(v);
     if (threadIdx.x < 32) {
-      const AndRoundConst c = rc[k];
       const uint4 y1 = v[0], yinf = v[1];
-      const uint4 y0 = gf_mul_warp(gf_add(cl, gf_mul_warp(y1, c.alpha)), c.inv_one_plus_alpha);
-      const uint4 c0 = y0, c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
+      c0 = gf_add(ci, gf_mul_warp(ai, y1));
+      c2 = yinf;
+      c1 = gf_add(gf_add(y1, c0), c2);
       const uint4 msg[2] = {c1, c2};
-      const uint4 rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
+      rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
       chal[k] = rr;
-      cl = gf_add(c0, gf_mul_warp(rr, gf_add(c1, gf_mul_warp(c2, rr))));
       r_sh = rr;
     } else {
       fs_help(fs, slow && k == 0);
@@ -557,6 +574,7 @@ __global__ void __launch_bounds__(kAndTailThreads)
     __syncthreads();
   }
   if (threadIdx.x < 32 && n_rounds) {
+    next_claim();
     st.end(fs, ts);
     *claim = cl;
   }

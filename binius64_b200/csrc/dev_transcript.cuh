@@ -462,6 +462,24 @@ __device__ __forceinline__ void fs_help(FsShared& sh, bool slow) {
   if (!slow && (warp == 1 || warp == 2)) fs_schedule(sh, warp - 1);
 }
 
+// The products of a small sumcheck round in one block: job(j, mul, own) for j < n, on threads
+// (mul a thread's product; own = true) or, when no more than the block's warps, each on a warp of
+// its own whose lanes all run it (mul a warp's product, a fifth of the latency; own on lane 0).
+// Warp 0, which also runs the Fiat-Shamir step and its algebra, comes last.
+template <class Job>
+__device__ __forceinline__ void block_jobs(uint32_t n, const Job& job) {
+  const uint32_t warps = blockDim.x >> 5;
+  if (n <= warps) {
+    const uint32_t j = warps - 1 - (threadIdx.x >> 5);
+    if (j < n)
+      job(j, [](uint4 a, uint4 b) { return gf_mul_warp(a, b); }, (threadIdx.x & 31) == 0);
+  } else {
+    const uint32_t first = threadIdx.x >= 32 ? threadIdx.x - 32 : threadIdx.x + blockDim.x - 32;
+    for (uint32_t j = first; j < n; j += blockDim.x)
+      job(j, [](uint4 a, uint4 b) { return gf_mul_nl(a, b); }, true);
+  }
+}
+
 // Host side of one device stretch.  begin() hands the host transcript's state to the device;
 // kernels advance state() and write to tape(); read() queues the copy-back of the state and of
 // the `tape_bytes` the stretch is known to write, and finish() (after the reads were waited on)

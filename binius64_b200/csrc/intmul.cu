@@ -446,6 +446,7 @@ __global__ void __launch_bounds__(kImTailThreads)
                              const uint4* __restrict__ beta_pow, uint4* __restrict__ chal) {
   pdl_wait();
   pdl_trigger();
+  extern __shared__ uint4 w_sh[];  // the items' weights
   __shared__ uint4 r_sh;
   __shared__ FsShared fs;
   FsStep st;
@@ -464,49 +465,67 @@ __global__ void __launch_bounds__(kImTailThreads)
     __syncthreads();
   }
   const bool slow = fs.slow;
+  uint4 T0 = gf_zero(), T1 = gf_zero(), T2 = gf_zero(), rr = gf_zero();
   for (uint32_t t = t0; t < n; t++) {
     const bool fold = t > 0;
     const uint4 r = r_sh;
-    const uint64_t L = 1ull << (n - t), h = L >> 1;
-    const uint4* eq = eq_base + ((1ull << (n - t - 1)) - 1);
-    uint4 v[2] = {gf_zero(), gf_zero()};
-    for (uint64_t it = threadIdx.x; it < (uint64_t)pairs * h; it += blockDim.x) {
-      const uint32_t p = (uint32_t)(it / h);
-      const uint64_t i = it - (uint64_t)p * h;
-      uint4* a = set + 2 * (uint64_t)p * stride;
-      uint4* b = a + stride;
-      uint4 a0 = a[i], a1 = a[h + i], b0 = b[i], b1 = b[h + i];
-      if (fold) {
-        a0 = gf_add(a0, gf_mul_nl(r, gf_add(a[L + i], a0)));
-        a1 = gf_add(a1, gf_mul_nl(r, gf_add(a[L + h + i], a1)));
-        b0 = gf_add(b0, gf_mul_nl(r, gf_add(b[L + i], b0)));
-        b1 = gf_add(b1, gf_mul_nl(r, gf_add(b[L + h + i], b1)));
-        a[i] = a0;
-        a[h + i] = a1;
-        b[i] = b0;
-        b[h + i] = b1;
-      }
-      const uint4 w = gf_mul_nl(eq[i], beta_pow[p]);
-      gf_add_into(v[0], gf_mul_nl(w, gf_mul_nl(a1, b1)));
-      gf_add_into(v[1], gf_mul_nl(w, gf_mul_nl(gf_add(a0, a1), gf_add(b0, b1))));
-    }
-    block_xor_sum<2>(v);
+    const uint32_t log_h = n - t - 1, h = 1u << log_h, L = 2 * h, items = pairs << log_h;
+    const uint4* eq = eq_base + (h - 1);
+    // warp 0, beside the folds: the batch's G and prefix after the last challenge, and what of
+    // the round's algebra does not wait for the sums
+    uint4 gi = gf_zero(), ai = gf_zero(), po = gf_zero();
     if (threadIdx.x < 32) {
+      if (t > t0) {
+        G = gf_add(T0, gf_mul_warp(rr, gf_add(T1, gf_mul_warp(rr, T2))));
+        uint4 f = gf_add(rr, alphas[t - 1].alpha);
+        f.x ^= 1u;
+        pf = gf_mul_warp(pf, f);
+      }
       const ImAlpha al = alphas[t];
-      const uint4 y1 = v[0], yinf = v[1];
-      const uint4 T0 = gf_mul_warp(gf_add(G, gf_mul_warp(al.alpha, y1)), al.inv_one_plus_alpha);
-      const uint4 T1 = gf_add(gf_add(y1, T0), yinf), T2 = yinf;
+      gi = gf_mul_warp(G, al.inv_one_plus_alpha);
+      ai = gf_mul_warp(al.alpha, al.inv_one_plus_alpha);
       uint4 oma = al.alpha;
       oma.x ^= 1u;
-      const uint4 m[3] = {gf_mul_warp(pf, gf_mul_warp(oma, T0)),
-                          gf_mul_warp(pf, gf_add(gf_mul_warp(oma, T1), T0)),
-                          gf_mul_warp(pf, gf_add(gf_mul_warp(oma, T2), T1))};
-      const uint4 rr = st.step(fs, ts, tape, m, 3, slow && t == t0);
+      po = gf_mul_warp(pf, oma);
+    }
+    // item (p, i): its weight, and positions i and h + i of both multilinears folded
+    block_jobs((fold ? 5 : 1) * items, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t kind = job / items, it = job - kind * items;
+      const uint32_t p = it >> log_h, i = it & (h - 1);
+      if (kind == 0) {
+        const uint4 w = mul(eq[i], beta_pow[p]);
+        if (own) w_sh[it] = w;
+        return;
+      }
+      uint4* x = set + (2 * (uint64_t)p + ((kind - 1) >> 1)) * stride + ((kind - 1) & 1) * h + i;
+      const uint4 x0 = x[0], y = gf_add(x0, mul(r, gf_add(x[L], x0)));
+      if (own) x[0] = y;
+    });
+    __syncthreads();
+    uint4 v[2] = {gf_zero(), gf_zero()};
+    block_jobs(2 * items, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t it = job < items ? job : job - items;
+      const uint4* a = set + 2 * (uint64_t)(it >> log_h) * stride + (it & (h - 1));
+      const uint4* b = a + stride;
+      uint4 x = a[h], y = b[h];
+      if (job >= items) {
+        gf_add_into(x, a[0]);
+        gf_add_into(y, b[0]);
+      }
+      const uint4 m = mul(w_sh[it], mul(x, y));
+      if (own) gf_add_into(job < items ? v[0] : v[1], m);
+    });
+    block_xor_sum<2>(v);
+    if (threadIdx.x < 32) {
+      const uint4 y1 = v[0], yinf = v[1];
+      T0 = gf_add(gi, gf_mul_warp(ai, y1));
+      T1 = gf_add(gf_add(y1, T0), yinf);
+      T2 = yinf;
+      const uint4 m[3] = {gf_mul_warp(po, T0),
+                          gf_add(gf_mul_warp(po, T1), gf_mul_warp(pf, T0)),
+                          gf_add(gf_mul_warp(po, T2), gf_mul_warp(pf, T1))};
+      rr = st.step(fs, ts, tape, m, 3, slow && t == t0);
       chal[t] = rr;
-      G = gf_add(T0, gf_mul_warp(rr, gf_add(T1, gf_mul_warp(rr, T2))));
-      uint4 f = gf_add(rr, al.alpha);
-      f.x ^= 1u;
-      pf = gf_mul_warp(pf, f);
       r_sh = rr;
     } else {
       fs_help(fs, slow && t == t0);
@@ -535,6 +554,7 @@ __global__ void __launch_bounds__(kImTailThreads)
   pdl_wait();
   pdl_trigger();
   constexpr uint32_t kClaims0 = kLeafPairs + 1, kClaims = kClaims0 + kLeafCols;
+  extern __shared__ uint4 w_sh[];  // the items' weights
   __shared__ uint4 r_sh;
   __shared__ FsShared fs;
   FsStep st;
@@ -555,66 +575,86 @@ __global__ void __launch_bounds__(kImTailThreads)
     __syncthreads();
   }
   const bool slow = fs.slow;
-  auto fold2 = [](uint4* col, uint64_t i, uint64_t L, uint64_t h, uint4 r, bool fold,
-                  uint4& x0, uint4& x1) {
-    x0 = col[i];
-    x1 = col[h + i];
-    if (fold) {
-      x0 = gf_add(x0, gf_mul_nl(r, gf_add(col[L + i], x0)));
-      x1 = gf_add(x1, gf_mul_nl(r, gf_add(col[L + h + i], x1)));
-      col[i] = x0;
-      col[h + i] = x1;
-    }
-  };
+  uint4 T[2][3] = {}, rr = gf_zero();
   for (uint32_t t = t0; t < n; t++) {
     const bool fold = t > 0;
     const uint4 r = r_sh;
-    const uint64_t L = 1ull << (n - t), h = L >> 1;
-    const uint64_t lvl = (1ull << (n - t - 1)) - 1;
-    uint4 v[3] = {gf_zero(), gf_zero(), gf_zero()};  // Y1_0, Yinf_0, Y1_1
-    for (uint64_t it = threadIdx.x; it < (uint64_t)kClaims * h; it += blockDim.x) {
-      const uint32_t m = (uint32_t)(it / h);
-      const uint64_t i = it - (uint64_t)m * h;
-      if (m < kLeafPairs) {
-        uint4 a0, a1, b0, b1;
-        fold2(leaves + 2 * (uint64_t)m * stride, i, L, h, r, fold, a0, a1);
-        fold2(leaves + (2 * (uint64_t)m + 1) * stride, i, L, h, r, fold, b0, b1);
-        const uint4 w = gf_mul_nl(eq_base[lvl + i], beta_pow[m]);
-        gf_add_into(v[0], gf_mul_nl(w, gf_mul_nl(a1, b1)));
-        gf_add_into(v[1], gf_mul_nl(w, gf_mul_nl(gf_add(a0, a1), gf_add(b0, b1))));
-      } else {
-        const bool g0 = m == kLeafPairs;
-        uint4* col = g0 ? lo0 : bcols + (uint64_t)(m - kClaims0) * stride;
-        uint4 c0, c1;
-        fold2(col, i, L, h, r, fold, c0, c1);
-        const uint4 w = gf_mul_nl(g0 ? eq_base[lvl + i] : eq2_base[lvl + i], beta_pow[m]);
-        gf_add_into(v[g0 ? 0 : 2], gf_mul_nl(w, c1));
+    const uint32_t log_h = n - t - 1, h = 1u << log_h, L = 2 * h;
+    const uint4* eq0 = eq_base + (h - 1);
+    const uint4* eq1 = eq2_base + (h - 1);
+    uint4 gi[2] = {}, ai[2] = {}, po[2] = {};
+    if (threadIdx.x < 32) {  // beside the folds, as in intmul_layer_tail_kernel
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        if (t > t0) {
+          G[g] = gf_add(T[g][0], gf_mul_warp(rr, gf_add(T[g][1], gf_mul_warp(rr, T[g][2]))));
+          uint4 f = gf_add(rr, alphas[2 * (t - 1) + g].alpha);
+          f.x ^= 1u;
+          pf[g] = gf_mul_warp(pf[g], f);
+        }
+        const ImAlpha al = alphas[2 * t + g];
+        gi[g] = gf_mul_warp(G[g], al.inv_one_plus_alpha);
+        ai[g] = gf_mul_warp(al.alpha, al.inv_one_plus_alpha);
+        uint4 oma = al.alpha;
+        oma.x ^= 1u;
+        po[g] = gf_mul_warp(pf[g], oma);
       }
     }
+    // the weight of item (m, i), and positions i and h + i of every column folded
+    constexpr uint32_t kCols = 2 * kLeafPairs + 1 + kLeafCols;
+    const uint32_t items = kClaims << log_h, halves = kCols << log_h;
+    block_jobs(items + (fold ? 2 * halves : 0), [&](uint32_t job, auto mul, bool own) {
+      if (job < items) {
+        const uint32_t m = job >> log_h, i = job & (h - 1);
+        const uint4 w = mul(m < kClaims0 ? eq0[i] : eq1[i], beta_pow[m]);
+        if (own) w_sh[job] = w;
+        return;
+      }
+      const uint32_t f = job - items, up = f >= halves ? 1 : 0, c = (f - up * halves) >> log_h;
+      uint4* x = (c < 2 * kLeafPairs ? leaves + (uint64_t)c * stride
+                  : c == 2 * kLeafPairs ? lo0
+                                        : bcols + (uint64_t)(c - 2 * kLeafPairs - 1) * stride) +
+                 up * h + (f & (h - 1));
+      const uint4 x0 = x[0], y = gf_add(x0, mul(r, gf_add(x[L], x0)));
+      if (own) x[0] = y;
+    });
+    __syncthreads();
+    uint4 v[3] = {gf_zero(), gf_zero(), gf_zero()};  // Y1_0, Yinf_0, Y1_1
+    const uint32_t pair_items = kLeafPairs << log_h;
+    block_jobs(items + pair_items, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t it = job < items ? job : job - items, m = it >> log_h, i = it & (h - 1);
+      uint4 x;
+      if (m < kLeafPairs) {
+        const uint4* a = leaves + 2 * (uint64_t)m * stride + i;
+        const uint4* b = a + stride;
+        x = a[h];
+        uint4 y = b[h];
+        if (job >= items) {
+          gf_add_into(x, a[0]);
+          gf_add_into(y, b[0]);
+        }
+        x = mul(x, y);
+      } else {
+        x = (m == kLeafPairs ? lo0 : bcols + (uint64_t)(m - kClaims0) * stride)[h + i];
+      }
+      const uint4 e = mul(w_sh[it], x);
+      if (own) gf_add_into(job >= items ? v[1] : m < kClaims0 ? v[0] : v[2], e);
+    });
     block_xor_sum<3>(v);
     if (threadIdx.x < 32) {
       uint4 m3[3] = {gf_zero(), gf_zero(), gf_zero()};
-      uint4 T[2][3];
+#pragma unroll
       for (int g = 0; g < 2; g++) {
-        const ImAlpha al = alphas[2 * t + g];
         const uint4 y1 = g == 0 ? v[0] : v[2], yinf = g == 0 ? v[1] : gf_zero();
-        T[g][0] = gf_mul_warp(gf_add(G[g], gf_mul_warp(al.alpha, y1)), al.inv_one_plus_alpha);
+        T[g][0] = gf_add(gi[g], gf_mul_warp(ai[g], y1));
         T[g][1] = gf_add(gf_add(y1, T[g][0]), yinf);
         T[g][2] = yinf;
-        uint4 oma = al.alpha;
-        oma.x ^= 1u;
-        gf_add_into(m3[0], gf_mul_warp(pf[g], gf_mul_warp(oma, T[g][0])));
-        gf_add_into(m3[1], gf_mul_warp(pf[g], gf_add(gf_mul_warp(oma, T[g][1]), T[g][0])));
-        gf_add_into(m3[2], gf_mul_warp(pf[g], gf_add(gf_mul_warp(oma, T[g][2]), T[g][1])));
+        gf_add_into(m3[0], gf_mul_warp(po[g], T[g][0]));
+        gf_add_into(m3[1], gf_add(gf_mul_warp(po[g], T[g][1]), gf_mul_warp(pf[g], T[g][0])));
+        gf_add_into(m3[2], gf_add(gf_mul_warp(po[g], T[g][2]), gf_mul_warp(pf[g], T[g][1])));
       }
-      const uint4 rr = st.step(fs, ts, tape, m3, 3, slow && t == t0);
+      rr = st.step(fs, ts, tape, m3, 3, slow && t == t0);
       chal[t] = rr;
-      for (int g = 0; g < 2; g++) {
-        G[g] = gf_add(T[g][0], gf_mul_warp(rr, gf_add(T[g][1], gf_mul_warp(rr, T[g][2]))));
-        uint4 f = gf_add(rr, alphas[2 * t + g].alpha);
-        f.x ^= 1u;
-        pf[g] = gf_mul_warp(pf[g], f);
-      }
       r_sh = rr;
     } else {
       fs_help(fs, slow && t == t0);
@@ -903,7 +943,8 @@ int IntMulDevice::layer(uint4* set, uint32_t pairs, std::vector<hu128>& point,
       if (int rc = batch_round(b, t)) return rc;
     }
     if (t0 < n) {
-      BGPU_CUDA(launch_pdl(intmul_layer_tail_kernel, 1, kImTailThreads, 0, s_, b.dt.state(),
+      BGPU_CUDA(launch_pdl(intmul_layer_tail_kernel, 1, kImTailThreads,
+                           16 * ((size_t)pairs << (n - t0 - 1)), s_, b.dt.state(),
                            b.dt.tape(), set, pairs, N_, n, t0, (const uint4*)eq_,
                            (const uint4*)b.sums, (const uint4*)b.prefix,
                            (const ImAlpha*)b.alphas, (const uint4*)b.beta, b.chal));
@@ -1180,7 +1221,8 @@ int IntMulDevice::run(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* 
       if (int rc = batch_round(b, t)) return rc;
     }
     if (t0 < n_) {
-      BGPU_CUDA(launch_pdl(intmul_leaf_tail_kernel, 1, kImTailThreads, 0, s_, b.dt.state(),
+      BGPU_CUDA(launch_pdl(intmul_leaf_tail_kernel, 1, kImTailThreads,
+                           16 * ((size_t)(kLeafPairs + 1 + kLeafCols) << (n_ - t0 - 1)), s_, b.dt.state(),
                            b.dt.tape(), leaves, lo0, bcols, N_, n_, t0, (const uint4*)eq_,
                            (const uint4*)eq2_, (const uint4*)b.sums, (const uint4*)b.prefix,
                            (const ImAlpha*)b.alphas, (const uint4*)b.beta, b.chal));

@@ -449,57 +449,90 @@ __global__ void __launch_bounds__(kShiftTailThreads)
   }
   __syncthreads();
   const bool slow = fs.slow;
+  uint4 s0 = gf_zero(), s1 = gf_zero(), s2 = gf_zero(), q0 = gf_zero(), q1 = gf_zero();
+  uint4 rr = gf_zero(), alpha = gf_zero();
+  auto next_state = [&]() {  // warp 0: the running sums after the last challenge
+    sum = gf_add(s0, gf_mul_warp(rr, gf_add(s1, gf_mul_warp(s2, rr))));
+    inout = gf_add(q0, gf_mul_warp(q1, rr));
+    uint4 f = gf_add(rr, alpha);
+    f.x ^= 1u;
+    eqp = gf_mul_warp(eqp, f);
+  };
   for (uint32_t k = 0, n_rem = n_rem0; n_rem > 0; k++, n_rem--) {
     const uint4 r = r_sh;
-    const uint64_t h = 1ull << n_rem, half = h >> 1;
-    for (uint64_t j = threadIdx.x; j < h; j += blockDim.x) {
-      const uint4 w0 = W[j], m0 = M[j];
-      W[j] = gf_add(w0, gf_mul_nl(r, gf_add(W[h + j], w0)));
-      M[j] = gf_add(m0, gf_mul_nl(r, gf_add(M[h + j], m0)));
-    }
+    const uint32_t h = 1u << n_rem, half = h >> 1;
     const bool early = p < n_rem;
+    // warp 0, beside the folds: what of the round's algebra does not wait for the sums
+    uint4 zc = gf_zero(), ii = gf_zero(), zi = gf_zero(), k0 = gf_zero(), k1 = gf_zero();
+    if (threadIdx.x < 32) {
+      if (k > 0) next_state();
+      const ShiftRoundConst c = rc[k];
+      alpha = c.alpha_dec;
+      zc = c.zc;
+      if (!c.early) {
+        ii = gf_mul_warp(inout, c.inv_one_plus_zc);
+        zi = gf_mul_warp(zc, c.inv_one_plus_zc);
+      }
+      uint4 one_a = alpha;
+      one_a.x ^= 1u;
+      k0 = gf_mul_warp(beta, eqp);
+      k1 = gf_mul_warp(one_a, k0);
+    }
+    block_jobs(2 * h, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t j = job & (h - 1);
+      uint4* x = job < h ? W : M;
+      const uint4 x0 = x[j], y = gf_add(x0, mul(r, gf_add(x[h + j], x0)));
+      if (own) x[j] = y;
+    });
     if (k > 0 && n_rem < p)
-      for (uint64_t i = threadIdx.x; i < half; i += blockDim.x)
+      for (uint32_t i = threadIdx.x; i < half; i += blockDim.x)
         eq_pub[i] = gf_add(eq_pub[i], eq_pub[half + i]);
     __syncthreads();
     uint4 v[4] = {gf_zero(), gf_zero(), gf_zero(), gf_zero()};
-    for (uint64_t j = threadIdx.x; j < half; j += blockDim.x) {
-      const uint4 w0 = W[j], w1 = W[half + j], m0 = M[j], m1 = M[half + j];
-      gf_add_into(v[0], gf_mul_nl(w1, m1));
-      gf_add_into(v[1], gf_mul_nl(gf_add(w0, w1), gf_add(m0, m1)));
-    }
-    const uint64_t E = early ? 1ull << (p - 1) : half;
-    for (uint64_t i = threadIdx.x; i < E; i += blockDim.x) {
-      const uint4 e = eq_pub[i];
-      gf_add_into(v[2], gf_mul_nl(W[half + i], e));
-      if (early) gf_add_into(v[3], gf_mul_nl(W[half + E + i], e));
-    }
+    const uint32_t E = early ? 1u << (p - 1) : half;
+    block_jobs(2 * half + (early ? 2 : 1) * E, [&](uint32_t job, auto mul, bool own) {
+      uint4 x, y;
+      uint32_t to;
+      if (job < 2 * half) {
+        const uint32_t j = job & (half - 1);
+        to = job < half ? 0 : 1;
+        x = W[half + j];
+        y = M[half + j];
+        if (to) {
+          gf_add_into(x, W[j]);
+          gf_add_into(y, M[j]);
+        }
+      } else {
+        const uint32_t i = job - 2 * half;
+        to = i < E ? 2 : 3;
+        x = W[half + i];
+        y = eq_pub[i & (E - 1)];
+      }
+      const uint4 m = mul(x, y);
+      if (own) gf_add_into(to == 0 ? v[0] : to == 1 ? v[1] : to == 2 ? v[2] : v[3], m);
+    });
     block_xor_sum<4>(v);
     if (threadIdx.x < 32) {
-      const ShiftRoundConst c = rc[k];
-      const uint4 y1 = v[0], yinf = v[1], lo = v[2], hi = early ? v[3] : v[2];
-      const uint4 s0 = gf_add(sum, y1), s2 = yinf, s1 = gf_add(gf_add(y1, s0), s2);
-      uint4 iy0, iy1;
-      if (c.early) {
-        iy1 = gf_add(lo, gf_mul_warp(gf_add(hi, lo), c.zc));
-        iy0 = inout;
+      const uint4 y1 = v[0], yinf = v[1], lo = v[2];
+      s0 = gf_add(sum, y1);
+      s2 = yinf;
+      s1 = gf_add(gf_add(y1, s0), s2);
+      // early: iy_0 = inout, iy_1 = lo + zc (hi + lo); else iy_1 = lo and
+      // iy_0 = (inout + zc iy_1) / (1 + zc)
+      uint4 iy1 = lo;
+      if (early) {
+        iy1 = gf_add(lo, gf_mul_warp(gf_add(v[3], lo), zc));
+        q0 = inout;
       } else {
-        iy1 = lo;
-        iy0 = gf_mul_warp(gf_add(inout, gf_mul_warp(iy1, c.zc)), c.inv_one_plus_zc);
+        q0 = gf_add(ii, gf_mul_warp(zi, lo));
       }
-      const uint4 q0 = iy0, q1 = gf_add(iy1, iy0);
-      uint4 one_a = c.alpha_dec;
-      one_a.x ^= 1u;
-      const uint4 d0 = gf_mul_warp(gf_mul_warp(q0, one_a), eqp);
-      const uint4 d1 = gf_mul_warp(gf_add(gf_mul_warp(q1, one_a), q0), eqp);
-      const uint4 msg[2] = {gf_add(s0, gf_mul_warp(beta, d0)), gf_add(s1, gf_mul_warp(beta, d1))};
-      const uint4 rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
+      q1 = gf_add(iy1, q0);
+      // beta eqp ((1 + alpha) q_0, (1 + alpha) q_1 + q_0)
+      const uint4 msg[2] = {
+          gf_add(s0, gf_mul_warp(k1, q0)),
+          gf_add(s1, gf_add(gf_mul_warp(k1, q1), gf_mul_warp(k0, q0)))};
+      rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
       chal[k] = rr;
-      sum = gf_add(s0, gf_mul_warp(rr, gf_add(s1, gf_mul_warp(s2, rr))));
-      inout = gf_add(q0, gf_mul_warp(q1, rr));
-      uint4 f = gf_add(rr, c.alpha_dec);
-      f.x ^= 1u;
-      eqp = gf_mul_warp(eqp, f);
       r_sh = rr;
     } else {
       fs_help(fs, slow && k == 0);
@@ -507,6 +540,7 @@ __global__ void __launch_bounds__(kShiftTailThreads)
     __syncthreads();
   }
   if (threadIdx.x < 32 && n_rem0) {
+    next_state();
     st.end(fs, ts);
     run[0] = sum;
     run[1] = inout;

@@ -309,40 +309,53 @@ __global__ void __launch_bounds__(kTailThreads)
   }
   __syncthreads();
   const bool slow = fs.slow;
+  uint4 c0 = gf_zero(), c1 = gf_zero(), c2 = gf_zero(), rr = gf_zero();
+  auto next_claim = [&]() {  // warp 0: the claim after round k - 1's challenge
+    cl = gf_add(c0, gf_mul_warp(rr, gf_add(c1, gf_mul_warp(c2, rr))));
+  };
   for (uint32_t k = 0; k < n_rounds; k++) {
+    if (k > 0 && threadIdx.x < 32) next_claim();
     if (k > 0 || r_first) {
       const uint4 r = r_sh;
-      const uint64_t h = len >> 1;
-      for (uint64_t j = threadIdx.x; j < h; j += blockDim.x) {
-        const uint4 a0 = a[j], b0 = b[j];
-        a[j] = gf_add(a0, gf_mul_nl(r, gf_add(a[h + j], a0)));
-        b[j] = gf_add(b0, gf_mul_nl(r, gf_add(b[h + j], b0)));
-      }
+      const uint32_t h = (uint32_t)(len >> 1);
+      block_jobs(2 * h, [&](uint32_t job, auto mul, bool own) {
+        const uint32_t j = job & (h - 1);
+        uint4* x = job < h ? a : b;
+        const uint4 x0 = x[j], y = gf_add(x0, mul(r, gf_add(x[h + j], x0)));
+        if (own) x[j] = y;
+      });
       len = h;
       __syncthreads();
     }
-    const uint64_t h = len >> 1;
+    const uint32_t h = (uint32_t)(len >> 1);
     uint4 v[2] = {gf_zero(), gf_zero()};
-    for (uint64_t j = threadIdx.x; j < h; j += blockDim.x) {
-      const uint4 a0 = a[j], a1 = a[h + j], b0 = b[j], b1 = b[h + j];
-      gf_add_into(v[0], gf_mul_nl(a1, b1));
-      gf_add_into(v[1], gf_mul_nl(gf_add(a0, a1), gf_add(b0, b1)));
-    }
+    block_jobs(2 * h, [&](uint32_t job, auto mul, bool own) {
+      const uint32_t j = job & (h - 1);
+      uint4 x = a[h + j], y = b[h + j];
+      if (job >= h) {
+        gf_add_into(x, a[j]);
+        gf_add_into(y, b[j]);
+      }
+      const uint4 m = mul(x, y);
+      if (own) gf_add_into(job < h ? v[0] : v[1], m);
+    });
     block_xor_sum<2>(v);
     if (threadIdx.x < 32) {
       const uint4 y1 = v[0], yinf = v[1];
-      const uint4 c0 = gf_add(cl, y1), c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
+      c0 = gf_add(cl, y1);
+      c2 = yinf;
+      c1 = gf_add(gf_add(y1, c0), c2);
       const uint4 msg[2] = {c0, c1};
-      const uint4 r = st.step(fs, ts, tape, msg, 2, slow && k == 0);
-      chal[k] = r;
-      cl = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
-      r_sh = r;
+      rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
+      chal[k] = rr;
+      r_sh = rr;
     } else {
       fs_help(fs, slow && k == 0);
     }
     __syncthreads();
   }
   if (threadIdx.x < 32 && n_rounds) {
+    next_claim();
     st.end(fs, ts);
     *claim = cl;
   }
