@@ -51,6 +51,9 @@ class StagedReads {
   int add(void* dst, const void* src, size_t bytes);
   int add2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width,
             size_t height);
+  // Pinned memory that kernels on the stream write themselves (its device address is the same),
+  // valid from wait() until the thread's next reads; nullptr when the stage has no room.
+  int pinned(size_t bytes, uint8_t** at) { return reserve(bytes, at); }
   int wait();
 
  private:

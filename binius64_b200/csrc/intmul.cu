@@ -117,11 +117,29 @@ __device__ __forceinline__ uint4 fold1(uint4 lo, uint4 hi, uint4 r) {
 // `fold`, both multilinears first shrink from 2L to L by r in place (fold_highest_var_inplace);
 // thread i owns positions i and i + L/2, so the fold and the round need one pass.  Grid: (chunks,
 // pairs).  The fold's r is *r_ptr (a challenge in HBM); r_ptr == nullptr means no fold.  Rounds of
-// at most kSmallRound elements run in biv_round_lanes_kernel.
+// at most kSmallRound elements run in biv_round_lanes_kernel.  With `beta`, a pair's sums are
+// weighted by beta[p] and all pairs add into out[0..8).
+__device__ __forceinline__ void biv_round_out(uint4 (&v)[2], uint32_t p,
+                                              const uint4* __restrict__ beta,
+                                              uint32_t* __restrict__ out) {
+  if (!beta) {
+    block_xor_reduce<2>(v, out + 8 * p);
+    return;
+  }
+  block_xor_sum<2>(v);
+  if (threadIdx.x < 32) {
+    const uint4 b = beta[p], y1 = gf_mul_warp(b, v[0]), yinf = gf_mul_warp(b, v[1]);
+    if (threadIdx.x == 0) {
+      atomic_xor_gf(out, y1);
+      atomic_xor_gf(out + 4, yinf);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kT)
     biv_round_kernel(uint4* __restrict__ set, uint64_t L, uint64_t stride,
                      const uint4* __restrict__ eq, const uint4* __restrict__ r_ptr,
-                     uint32_t* __restrict__ out) {
+                     const uint4* __restrict__ beta, uint32_t* __restrict__ out) {
   pdl_wait();
   pdl_trigger();
   const bool fold = r_ptr != nullptr;
@@ -154,7 +172,7 @@ __global__ void __launch_bounds__(kT)
     xor_into(sinf, clmul128(e, gf_mul(gf_add(a0, a1), gf_add(b0, b1))));
   }
   uint4 v[2] = {reduce256(s1), reduce256(sinf)};
-  block_xor_reduce<2>(v, out + 8 * p);
+  biv_round_out(v, p, beta, out);
 }
 
 // The small rounds of biv_round_kernel (L <= kSmallRound) on four lanes per position i: lane k
@@ -164,7 +182,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     biv_round_lanes_kernel(uint4* __restrict__ set, uint64_t L, uint64_t stride,
                            const uint4* __restrict__ eq, const uint4* __restrict__ r_ptr,
-                           uint32_t* __restrict__ out) {
+                           const uint4* __restrict__ beta, uint32_t* __restrict__ out) {
   pdl_wait();
   pdl_trigger();
   const bool fold = r_ptr != nullptr;
@@ -196,7 +214,7 @@ __global__ void __launch_bounds__(kT)
     if (live && k == 1)
       gf_add_into(v[1], gf_mul_nl(eq[i], gf_mul_nl(gf_add(a0, a1), gf_add(b0, b1))));
   }
-  block_xor_reduce<2>(v, out + 8 * p);
+  biv_round_out(v, p, beta, out);
 }
 
 // Column k of `set` (current length L): out[4k..] += sum eq[i] col_k[L/2 + i], with the same
@@ -424,45 +442,168 @@ __global__ void __launch_bounds__(kImFinishThreads)
   }
 }
 
-// The small last rounds of one GKR layer's batched MLE-check (IntMulDevice::layer: `pairs`
-// bivariate product claims, one eq point, messages of three coefficients) in one CTA, from round
-// t0 on: per round every multilinear of the set folds 2L -> L by the previous challenge (r_first
-// for round t0 when t0 > 0), the products are summed with their eq weights, and warp 0 runs the
-// batch's Fiat-Shamir step with the transcript in its registers.  The step is the one of
-// intmul_round_finish_kernel rewritten for a single group: the message is linear in the round's
-// sums, so with Y1 = sum_p beta^p y_1,p and Yinf = sum_p beta^p y_inf,p (one block sum per
-// round) and the running G = sum_p beta^p sum_p, T0 = (G + alpha Y1) / (1 + alpha),
-// T1 = Y1 + T0 + Yinf, T2 = Yinf, the message is prefix ((1 + alpha) T0, (1 + alpha) T1 + T0,
-// (1 + alpha) T2 + T1), and after r the batch keeps G = T0 + r T1 + r^2 T2 and
-// prefix (1 + r + alpha).  Thread items are (pair, index) with the index fastest; item i of pair
-// p folds positions i and L/2 + i of both multilinears and evaluates that pair of positions.
+// One GKR layer's batched MLE-check (IntMulDevice::layer: `pairs` bivariate product claims, one eq
+// point, messages of three coefficients).  The step is the one of intmul_round_finish_kernel
+// rewritten for a single group: the message is linear in the round's sums, so with
+// Y1 = sum_p beta^p y_1,p and Yinf = sum_p beta^p y_inf,p and the running G = sum_p beta^p sum_p,
+// T0 = (G + alpha Y1) / (1 + alpha), T1 = Y1 + T0 + Yinf, T2 = Yinf, the message is
+// prefix ((1 + alpha) T0, (1 + alpha) T1 + T0, (1 + alpha) T2 + T1), and after r the batch keeps
+// G = T0 + r T1 + r^2 T2 and prefix (1 + r + alpha).
+//
+// A layer is one launch when its first round is small (LayerArgs come by value, the CTA builds the
+// eq tensors, and the results go straight to pinned host memory): the eleven layers of an IntMul
+// follow one another through the host, so what each one costs besides its rounds is round trip
+// and launches.  Measured on B200 with four multiplications: 80 us a layer with two host copies,
+// five launches and four copies back, 45 us so.  Larger layers start with intmul_layer_begin_kernel
+// and run a launch pair per large round.
+constexpr uint32_t kLayerMaxVars = 24, kLayerMaxPairs = 48;
+struct LayerArgs {
+  TranscriptState ts;
+  ImAlpha alphas[kLayerMaxVars];
+  uint4 beta[kLayerMaxPairs];  // powers
+  uint4 G;
+  uint32_t pairs, n;
+};
+// The same in device memory for the launches of a larger layer, with the running prefix and the
+// rounds' sums and challenges.
+struct LayerState {
+  LayerArgs a;
+  uint4 prefix;
+  uint4 y[kLayerMaxVars][2];
+  uint4 chal[kLayerMaxVars];
+};
+// What the host reads back, in pinned memory; then 3 n message elements, then 2 pairs evaluations.
+struct LayerResult {
+  TranscriptState ts;
+  uint4 chal[kLayerMaxVars];
+};
+constexpr size_t kLayerTape = (sizeof(LayerResult) + 15) & ~size_t(15);
+
+// eq tensor levels 0 .. n - 1 of the layer's point (as eq_levels_kernel), and the layer's state.
+__global__ void __launch_bounds__(kT)
+    intmul_layer_begin_kernel(LayerArgs a, LayerState* __restrict__ st, uint4* __restrict__ eq) {
+  const uint64_t total = (1ull << a.n) - 1;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
+       t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t lvl = 63 - __clzll(t + 1);
+    const uint64_t i = t + 1 - (1ull << lvl);
+    // four interleaved partial products, as eq_levels_kernel
+    auto factor = [&](uint32_t j) {
+      const uint4 p = a.alphas[a.n - 1 - j].alpha;
+      return ((i >> j) & 1) ? p : gf_add(p, gf_one());
+    };
+    uint4 a0 = gf_one(), a1 = gf_one(), a2 = gf_one(), a3 = gf_one();
+    uint32_t j = 0;
+    for (; j + 4 <= lvl; j += 4) {
+      a0 = gf_mul_nl(a0, factor(j));
+      a1 = gf_mul_nl(a1, factor(j + 1));
+      a2 = gf_mul_nl(a2, factor(j + 2));
+      a3 = gf_mul_nl(a3, factor(j + 3));
+    }
+    for (; j < lvl; j++) a0 = gf_mul_nl(a0, factor(j));
+    eq[t] = gf_mul_nl(gf_mul_nl(a0, a1), gf_mul_nl(a2, a3));
+  }
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      st->a.ts = a.ts;
+      st->a.G = a.G;
+      st->prefix = gf_one();
+    }
+    if (threadIdx.x < a.pairs) st->a.beta[threadIdx.x] = a.beta[threadIdx.x];
+    if (threadIdx.x < a.n) {
+      st->a.alphas[threadIdx.x] = a.alphas[threadIdx.x];
+      st->y[threadIdx.x][0] = gf_zero();
+      st->y[threadIdx.x][1] = gf_zero();
+    }
+  }
+}
+
+// Round t's Fiat-Shamir step of a larger layer.
+__global__ void __launch_bounds__(kFsThreads)
+    intmul_layer_finish_kernel(LayerState* __restrict__ ls, uint8_t* __restrict__ tape,
+                               uint32_t t) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ FsShared fs;
+  FsStep st;
+  if (threadIdx.x < 32) st.begin(fs, &ls->a.ts);
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    fs_help(fs, fs.slow);
+    return;
+  }
+  const ImAlpha al = ls->a.alphas[t];
+  const uint4 y1 = ls->y[t][0], yinf = ls->y[t][1], pf = ls->prefix;
+  uint4 oma = al.alpha;
+  oma.x ^= 1u;
+  const uint4 po = gf_mul_warp(pf, oma);
+  const uint4 T0 =
+      gf_mul_warp(al.inv_one_plus_alpha, gf_add(ls->a.G, gf_mul_warp(al.alpha, y1)));
+  const uint4 T1 = gf_add(gf_add(y1, T0), yinf), T2 = yinf;
+  const uint4 m[3] = {gf_mul_warp(po, T0), gf_add(gf_mul_warp(po, T1), gf_mul_warp(pf, T0)),
+                      gf_add(gf_mul_warp(po, T2), gf_mul_warp(pf, T1))};
+  const uint4 r = st.step(fs, &ls->a.ts, tape, m, 3, fs.slow);
+  ls->chal[t] = r;
+  ls->a.G = gf_add(T0, gf_mul_warp(r, gf_add(T1, gf_mul_warp(r, T2))));
+  uint4 f = gf_add(r, al.alpha);
+  f.x ^= 1u;
+  ls->prefix = gf_mul_warp(pf, f);
+  st.end(fs, &ls->a.ts);
+}
+
+// The rounds from t0 on (all of them when t0 = 0: then `a` holds the arguments, else `ls`) in one
+// CTA, then the evaluations.  Per round every multilinear of the set folds 2L -> L by the previous
+// challenge and the products are summed with their eq and beta weights, one product a job
+// (block_jobs), and warp 0 runs the step.  Item i of pair p folds positions i and L/2 + i of both
+// multilinears and evaluates that pair of positions.
 constexpr int kImTailThreads = 512;
 __global__ void __launch_bounds__(kImTailThreads)
-    intmul_layer_tail_kernel(TranscriptState* __restrict__ ts, uint8_t* __restrict__ tape,
-                             uint4* __restrict__ set, uint32_t pairs, uint64_t stride,
-                             uint32_t n, uint32_t t0, const uint4* __restrict__ eq_base,
-                             const uint4* __restrict__ sums, const uint4* __restrict__ prefix,
-                             const ImAlpha* __restrict__ alphas,
-                             const uint4* __restrict__ beta_pow, uint4* __restrict__ chal) {
+    intmul_layer_tail_kernel(LayerArgs a, const LayerState* __restrict__ ls,
+                             uint4* __restrict__ set, uint64_t stride, uint32_t t0,
+                             uint4* __restrict__ eq_base, uint8_t* __restrict__ result) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ uint4 w_sh[];  // the items' weights
   __shared__ uint4 r_sh;
+  __shared__ uint4 beta_sh[kLayerMaxPairs];
+  __shared__ ImAlpha alpha_sh[kLayerMaxVars];
+  __shared__ TranscriptState ts_sh;
   __shared__ FsShared fs;
+  const uint32_t pairs = a.pairs, n = a.n;
+  LayerResult* res = reinterpret_cast<LayerResult*>(result);
+  uint8_t* tape = result + kLayerTape;
   FsStep st;
-  uint4 G = gf_zero(), pf = gf_zero();
-  {
-    uint4 v[1] = {gf_zero()};
-    for (uint32_t p = threadIdx.x; p < pairs; p += blockDim.x)
-      gf_add_into(v[0], gf_mul_nl(beta_pow[p], sums[p]));
-    block_xor_sum<1>(v);
-    if (threadIdx.x < 32) {
-      G = v[0];
-      pf = prefix[0];
-      st.begin(fs, ts);
-      if (t0 > 0) r_sh = chal[t0 - 1];
+  uint4 G = gf_zero(), pf = gf_one();
+  if (threadIdx.x < pairs) beta_sh[threadIdx.x] = t0 ? ls->a.beta[threadIdx.x] : a.beta[threadIdx.x];
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + n)
+    alpha_sh[threadIdx.x - 64] = t0 ? ls->a.alphas[threadIdx.x - 64] : a.alphas[threadIdx.x - 64];
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) ts_sh = t0 ? ls->a.ts : a.ts;
+    __syncwarp();
+    st.begin(fs, &ts_sh);
+    G = t0 ? ls->a.G : a.G;
+    if (t0) {
+      pf = ls->prefix;
+      r_sh = ls->chal[t0 - 1];
+      if (threadIdx.x < t0) res->chal[threadIdx.x] = ls->chal[threadIdx.x];
     }
+  }
+  __syncthreads();
+  if (t0 == 0) {  // eq tensor levels 0 .. n - 1, each from the one below
+    if (threadIdx.x == 0) eq_base[0] = gf_one();
     __syncthreads();
+    for (uint32_t m = 0; m + 1 < n; m++) {
+      const uint32_t half = 1u << m;
+      const uint4 p = alpha_sh[n - 1 - m].alpha;
+      block_jobs(half, [&](uint32_t i, auto mul, bool own) {
+        const uint4 x = eq_base[half - 1 + i], hi = mul(x, p);
+        if (own) {
+          eq_base[2 * half - 1 + i] = gf_add(x, hi);
+          eq_base[3 * half - 1 + i] = hi;
+        }
+      });
+      __syncthreads();
+    }
   }
   const bool slow = fs.slow;
   uint4 T0 = gf_zero(), T1 = gf_zero(), T2 = gf_zero(), rr = gf_zero();
@@ -477,11 +618,11 @@ __global__ void __launch_bounds__(kImTailThreads)
     if (threadIdx.x < 32) {
       if (t > t0) {
         G = gf_add(T0, gf_mul_warp(rr, gf_add(T1, gf_mul_warp(rr, T2))));
-        uint4 f = gf_add(rr, alphas[t - 1].alpha);
+        uint4 f = gf_add(rr, alpha_sh[t - 1].alpha);
         f.x ^= 1u;
         pf = gf_mul_warp(pf, f);
       }
-      const ImAlpha al = alphas[t];
+      const ImAlpha al = alpha_sh[t];
       gi = gf_mul_warp(G, al.inv_one_plus_alpha);
       ai = gf_mul_warp(al.alpha, al.inv_one_plus_alpha);
       uint4 oma = al.alpha;
@@ -493,7 +634,7 @@ __global__ void __launch_bounds__(kImTailThreads)
       const uint32_t kind = job / items, it = job - kind * items;
       const uint32_t p = it >> log_h, i = it & (h - 1);
       if (kind == 0) {
-        const uint4 w = mul(eq[i], beta_pow[p]);
+        const uint4 w = mul(eq[i], beta_sh[p]);
         if (own) w_sh[it] = w;
         return;
       }
@@ -505,14 +646,13 @@ __global__ void __launch_bounds__(kImTailThreads)
     uint4 v[2] = {gf_zero(), gf_zero()};
     block_jobs(2 * items, [&](uint32_t job, auto mul, bool own) {
       const uint32_t it = job < items ? job : job - items;
-      const uint4* a = set + 2 * (uint64_t)(it >> log_h) * stride + (it & (h - 1));
-      const uint4* b = a + stride;
-      uint4 x = a[h], y = b[h];
+      const uint4* x = set + 2 * (uint64_t)(it >> log_h) * stride + (it & (h - 1));
+      uint4 c = x[h], d = x[stride + h];
       if (job >= items) {
-        gf_add_into(x, a[0]);
-        gf_add_into(y, b[0]);
+        gf_add_into(c, x[0]);
+        gf_add_into(d, x[stride]);
       }
-      const uint4 m = mul(w_sh[it], mul(x, y));
+      const uint4 m = mul(w_sh[it], mul(c, d));
       if (own) gf_add_into(job < items ? v[0] : v[1], m);
     });
     block_xor_sum<2>(v);
@@ -524,15 +664,23 @@ __global__ void __launch_bounds__(kImTailThreads)
       const uint4 m[3] = {gf_mul_warp(po, T0),
                           gf_add(gf_mul_warp(po, T1), gf_mul_warp(pf, T0)),
                           gf_add(gf_mul_warp(po, T2), gf_mul_warp(pf, T1))};
-      rr = st.step(fs, ts, tape, m, 3, slow && t == t0);
-      chal[t] = rr;
+      rr = st.step(fs, &ts_sh, tape, m, 3, slow && t == t0);
+      if (threadIdx.x == 0) res->chal[t] = rr;
       r_sh = rr;
     } else {
       fs_help(fs, slow && t == t0);
     }
     __syncthreads();
   }
-  if (threadIdx.x < 32 && t0 < n) st.end(fs, ts);
+  if (threadIdx.x < 32) st.end(fs, &res->ts);
+  // the multilinears' evaluations: the last pairs folded by the last challenge
+  uint4* evals = reinterpret_cast<uint4*>(tape + 48 * n);
+  const uint4 r = r_sh;
+  block_jobs(2 * pairs, [&](uint32_t m, auto mul, bool own) {
+    const uint4* x = set + m * stride;
+    const uint4 x0 = x[0], y = gf_add(x0, mul(r, gf_add(x[1], x0)));
+    if (own) evals[m] = y;
+  });
 }
 
 // The small last rounds of the leaf batch (IntMulDevice phase 5) in one CTA, from round t0 on,
@@ -782,13 +930,13 @@ class IntMulDevice {
   // Fused round launches on multilinears of current length L (fold from 2L first by *r_ptr when
   // r_ptr is set).
   int biv_round(uint4* set, uint32_t pairs, uint64_t L, const uint4* eq, const uint4* r_ptr,
-                uint32_t* out) {
+                uint32_t* out, const uint4* beta = nullptr) {
     dim3 grid(blocks_for(L / 2, 148 * 2), pairs);
     if (L <= kSmallRound)
       BGPU_CUDA(launch_pdl(biv_round_lanes_kernel, dim3(blocks_for(2 * L, 148 * 2), pairs), kT, 0,
-                           s_, set, L, N_, eq, r_ptr, out));
+                           s_, set, L, N_, eq, r_ptr, beta, out));
     else
-      BGPU_CUDA(launch_pdl(biv_round_kernel, grid, kT, 0, s_, set, L, N_, eq, r_ptr, out));
+      BGPU_CUDA(launch_pdl(biv_round_kernel, grid, kT, 0, s_, set, L, N_, eq, r_ptr, beta, out));
     return check("biv_round_kernel");
   }
   int lin_round(uint4* set, uint32_t cols, uint64_t L, const uint4* eq, const uint4* r_ptr,
@@ -924,43 +1072,74 @@ int IntMulDevice::layer(uint4* set, uint32_t pairs, std::vector<hu128>& point,
                         std::vector<hu128>& claims) {
   const uint32_t n = (uint32_t)point.size();
   const hu128 beta = sample(t_);
-  std::vector<hu128> evals;
   if (n == 0) {
+    std::vector<hu128> evals;
     if (int rc = read_first(set, 2 * pairs, N_, evals)) return rc;
-  } else {
-    if (int rc = eq_levels({&point}, n - 1, eq_)) return rc;
-    std::vector<ImClaim> cl(pairs);
-    for (uint32_t p = 0; p < pairs; p++) cl[p] = ImClaim{(uint16_t)(2 * p), (uint16_t)(2 * p + 1), 2, 0, 0};
-    DevBatch b;
-    if (int rc = batch_begin(b, cl, {&point}, claims, beta, 2 * pairs)) return rc;
-    // rounds of at most tail_items() (pair, position) items run in one intmul_layer_tail_kernel
-    uint32_t t0 = 0;
-    while (t0 < n && ((uint64_t)pairs << (n - t0 - 1)) > tail_items()) t0++;
-    for (uint32_t t = 0; t < t0; t++) {
-      if (int rc = biv_round(set, pairs, 1ull << (n - t), level(eq_, n - t - 1), batch_r(b, t),
-                             batch_slots(b, t)))
-        return rc;
-      if (int rc = batch_round(b, t)) return rc;
-    }
-    if (t0 < n) {
-      BGPU_CUDA(launch_pdl(intmul_layer_tail_kernel, 1, kImTailThreads,
-                           16 * ((size_t)pairs << (n - t0 - 1)), s_, b.dt.state(),
-                           b.dt.tape(), set, pairs, N_, n, t0, (const uint4*)eq_,
-                           (const uint4*)b.sums, (const uint4*)b.prefix,
-                           (const ImAlpha*)b.alphas, (const uint4*)b.beta, b.chal));
-      if (int rc = check("intmul_layer_tail_kernel")) return rc;
-    }
-    std::vector<hu128> ch, last(4 * pairs);
-    StagedReads rd(s_);
-    if (int rc = batch_read(b, rd, ch)) return rc;
-    if (int rc = copy_pairs(rd, set, 2 * pairs, last.data())) return rc;
-    if (int rc = rd.wait()) return rc;
-    if (int rc = batch_end(b)) return rc;
-    evals = fold_pairs(last, ch[n - 1]);
-    point.assign(ch.rbegin(), ch.rend());
+    write_elems(t_, evals);
+    point.clear();
+    claims = evals;
+    return BINIUS_OK;
   }
+  if (n > kLayerMaxVars || pairs > kLayerMaxPairs || claims.size() != pairs)
+    return set_error(BINIUS_E_ARG, "intmul layer: too many variables or pairs");
+  LayerArgs a;
+  memset(&a, 0, sizeof(a));
+  t_.save(a.ts);
+  a.ts.tape_cap = 48 * n;
+  a.pairs = pairs;
+  a.n = n;
+  std::vector<hu128> inv(n);
+  for (uint32_t t = 0; t < n; t++) inv[t] = 1 ^ point[n - 1 - t];
+  batch_inv(inv);
+  for (uint32_t t = 0; t < n; t++) a.alphas[t] = ImAlpha{u4(point[n - 1 - t]), u4(inv[t])};
+  hu128 bp = 1, G = 0;
+  for (uint32_t p = 0; p < pairs; p++, bp = host_gf_mul(bp, beta)) {
+    a.beta[p] = u4(bp);
+    G ^= host_gf_mul(bp, claims[p]);
+  }
+  a.G = u4(G);
+  StagedReads rd(s_);
+  uint8_t* result = nullptr;
+  if (int rc = rd.pinned(kLayerTape + 48 * n + 32 * pairs, &result)) return rc;
+  if (!result) return set_error(BINIUS_E_ARG, "intmul layer: result larger than the stage");
+  // rounds of at most tail_items() (pair, position) items run in the tail
+  uint32_t t0 = 0;
+  while (t0 < n && ((uint64_t)pairs << (n - t0 - 1)) > tail_items()) t0++;
+  t0 = std::min(t0, n - 1);
+  LayerState* ls = nullptr;
+  if (t0 > 0) {
+    uint4* mem = nullptr;
+    if (int rc = alloc(&mem, (sizeof(LayerState) + 15) / 16)) return rc;
+    ls = reinterpret_cast<LayerState*>(mem);
+    intmul_layer_begin_kernel<<<blocks_for(1ull << n), kT, 0, s_>>>(a, ls, eq_);
+    if (int rc = check("intmul_layer_begin_kernel")) return rc;
+    for (uint32_t t = 0; t < t0; t++) {
+      if (int rc = biv_round(set, pairs, 1ull << (n - t), level(eq_, n - t - 1),
+                             t ? &ls->chal[t - 1] : nullptr,
+                             reinterpret_cast<uint32_t*>(ls->y[t]), ls->a.beta))
+        return rc;
+      BGPU_CUDA(launch_pdl(intmul_layer_finish_kernel, 1, kFsThreads, 0, s_, ls,
+                           result + kLayerTape, t));
+      if (int rc = check("intmul_layer_finish_kernel")) return rc;
+    }
+  }
+  BGPU_CUDA(launch_pdl(intmul_layer_tail_kernel, 1, kImTailThreads,
+                       16 * ((size_t)pairs << (n - t0 - 1)), s_, a, (const LayerState*)ls, set, N_,
+                       t0, eq_, result));
+  if (int rc = check("intmul_layer_tail_kernel")) return rc;
+  if (int rc = rd.wait()) return rc;
+  const LayerResult* res = reinterpret_cast<const LayerResult*>(result);
+  if (res->ts.error || res->ts.tape_len != 48 * n)
+    return set_error(BINIUS_E_CUDA, "device transcript wrote an unexpected number of bytes");
+  // the tail leaves the fields it does not own as they were handed over
+  TranscriptState ts = res->ts;
+  ts.tape_cap = a.ts.tape_cap;
+  t_.load(ts, result + kLayerTape);
+  std::vector<hu128> evals(2 * pairs);
+  memcpy(evals.data(), result + kLayerTape + 48 * n, 32 * pairs);
+  point.resize(n);
+  for (uint32_t t = 0; t < n; t++) point[n - 1 - t] = h128(&res->chal[t]);
   write_elems(t_, evals);
-  if (n == 0) point.clear();
   claims = evals;
   return BINIUS_OK;
 }
