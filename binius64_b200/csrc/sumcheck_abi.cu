@@ -16,12 +16,14 @@
 // (fold_highest_var_inplace, verifier/math/src/multilinear/fold.rs:14-29: a[i] += r (a[i + h] -
 // a[i])); the eq expansion and the sums live in the prover object's own device memory.  Round
 // sums come from the prove path's own evaluation kernels (bivariate_eval, and_mle_eval); each
-// execute reads two field elements back and interpolates on the host.  Calls out of order return
+// execute reads two field elements back and interpolates on the host.  The bivariate product's
+// fold is one launch with the next round's evaluation, which leaves the sums in pinned memory.  Calls out of order return
 // BINIUS_E_ARG with the reference's error names (ExpectedFold / ExpectedExecute,
 // sumcheck/error.rs).
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "gf128.cuh"
@@ -77,6 +79,113 @@ __global__ void __launch_bounds__(kThreads)
   block_xor_reduce<1>(v, out);
 }
 
+// One bivariate round: with `fold`, (a, b) shrink from 2 L to L by r in place; then
+// out = (y_1, y_inf) on the L values, through per-block partial sums that the last block adds up
+// and writes, with the sequence number `seq` after them, to pinned host memory.  Four lanes share a
+// position (as bivariate_fold_eval_lanes_kernel), L <= kRoundMax; the host's reads are what a
+// round costs here, so it is one launch without a clear or a copy.  Twenty rounds from 2^20
+// elements on, host algebra included: 800 us with an evaluation, a clear, a copy and a fold per
+// round and the sums allocated by cudaMalloc, 484 us so.
+constexpr uint64_t kRoundMax = 1ull << 14;
+constexpr uint32_t kRoundBlocks = 128;
+struct RoundResult {
+  uint4 y[2];
+  uint64_t seq, pad[3];
+};
+struct RoundPartials {
+  uint4 y[kRoundBlocks][2];
+  uint32_t done, pad[3];
+};
+__global__ void __launch_bounds__(kThreads)
+    bivariate_host_round_kernel(uint4* __restrict__ a, uint4* __restrict__ b, uint64_t L, bool fold,
+                                uint4 r, RoundPartials* __restrict__ parts,
+                                RoundResult* __restrict__ out, uint64_t seq) {
+  const uint64_t h = L >> 1;
+  const uint32_t k = threadIdx.x & 3;
+  uint4 v[2] = {gf_zero(), gf_zero()};
+  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < 4 * h;
+       base += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t j = (base + (threadIdx.x & 31)) >> 2;
+    const bool live = j < h;
+    uint4 f = gf_zero();
+    if (live) {
+      uint4* col = k < 2 ? a : b;
+      const uint64_t pos = j + ((k & 1) ? h : 0);
+      f = col[pos];
+      if (fold) {
+        f = gf_add(f, gf_mul(r, gf_add(col[L + pos], f)));
+        col[pos] = f;
+      }
+    }
+    const uint4 a0 = shfl_gf(f, 0, 4), a1 = shfl_gf(f, 1, 4), b0 = shfl_gf(f, 2, 4),
+                b1 = shfl_gf(f, 3, 4);
+    const uint4 x = k ? gf_add(a0, a1) : a1, y = k ? gf_add(b0, b1) : b1;
+    if (live && k < 2) gf_add_into(k ? v[1] : v[0], gf_mul(x, y));
+  }
+  block_xor_sum<2>(v);
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    parts->y[blockIdx.x][0] = v[0];
+    parts->y[blockIdx.x][1] = v[1];
+    __threadfence();
+    last = atomicAdd(&parts->done, 1u) + 1 == gridDim.x;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v[0] = v[1] = gf_zero();
+  if (threadIdx.x < gridDim.x) {
+    v[0] = __ldcg(&parts->y[threadIdx.x][0]);
+    v[1] = __ldcg(&parts->y[threadIdx.x][1]);
+  }
+  block_xor_sum<2>(v);
+  if (threadIdx.x == 0) {
+    parts->done = 0;
+    out->y[0] = v[0];
+    out->y[1] = v[1];
+    __threadfence_system();
+    *reinterpret_cast<volatile uint64_t*>(&out->seq) = seq;
+  }
+}
+// The sums of a larger round, from where its kernel added them up.
+__global__ void publish_round_kernel(const uint4* __restrict__ sums, RoundResult* __restrict__ out,
+                                     uint64_t seq) {
+  out->y[0] = sums[0];
+  out->y[1] = sums[1];
+  __threadfence_system();
+  *reinterpret_cast<volatile uint64_t*>(&out->seq) = seq;
+}
+
+// Pinned results for the provers alive: slots of one allocation, given back when a prover is
+// destroyed.  Any thread may take or return one.
+constexpr uint32_t kResultSlots = 1024;
+std::mutex g_slots_mu;
+std::vector<RoundResult*> g_free_slots;
+bool g_slots_made = false;
+int take_slot(RoundResult** out) {
+  std::lock_guard<std::mutex> lock(g_slots_mu);
+  *out = nullptr;
+  if (!g_slots_made) {
+    RoundResult* mem = nullptr;
+    BGPU_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&mem), kResultSlots * sizeof(RoundResult),
+                            cudaHostAllocPortable | cudaHostAllocMapped));
+    memset(mem, 0, kResultSlots * sizeof(RoundResult));
+    for (uint32_t i = 0; i < kResultSlots; i++) g_free_slots.push_back(mem + i);
+    g_slots_made = true;
+  }
+  if (!g_free_slots.empty()) {
+    *out = g_free_slots.back();
+    g_free_slots.pop_back();
+  }
+  return BINIUS_OK;
+}
+void return_slot(RoundResult* slot) {
+  if (!slot) return;
+  std::lock_guard<std::mutex> lock(g_slots_mu);
+  slot->seq = 0;
+  g_free_slots.push_back(slot);
+}
+
 enum Kind { kBivariate = 0, kQuadraticMle = 1, kInOut = 2 };
 
 hu128 h128(const void* p) {
@@ -110,6 +219,11 @@ struct binius_sumcheck {
   bool have_coeffs = false;
   std::vector<hu128> coeffs;    // the last execute's RoundCoeffs
   hu128 last = 0;               // the running sum / evaluation claim
+  // bivariate rounds (result == nullptr: more provers alive than slots, plain reads instead)
+  RoundPartials* parts = nullptr;
+  RoundResult* result = nullptr;
+  uint64_t seq = 0;             // rounds evaluated or queued
+  bool queued = false;          // the next execute's sums are on their way
 };
 
 namespace {
@@ -155,23 +269,77 @@ int eval_with_gruen(const binius_sumcheck* p, const uint4* x, hu128& out) {
 }
 
 int make(int kind, uint32_t n_vars, void* stream, binius_sumcheck** out) {
+  int dev = 0;
+  BGPU_CUDA(cudaGetDevice(&dev));
+  if (int rc = configure_device_pool(dev)) return rc;
   binius_sumcheck* p = new binius_sumcheck();
   p->kind = kind;
   p->s = as_stream(stream);
   p->n_vars = n_vars;
-  cudaError_t e = cudaMalloc(&p->acc, 32);
-  if (e != cudaSuccess) {
-    delete p;
-    return cuda_error(e, "sumcheck round sums");
+  // the sums and, for bivariate rounds, the partial sums with their counter clear
+  cudaError_t e = cudaMallocAsync(&p->acc, 32 + sizeof(RoundPartials), p->s);
+  if (e == cudaSuccess && kind == kBivariate) {
+    p->parts = reinterpret_cast<RoundPartials*>(p->acc + 8);
+    e = cudaMemsetAsync(&p->parts->done, 0, 4, p->s);
+  }
+  int rc = e == cudaSuccess ? BINIUS_OK : cuda_error(e, "sumcheck round sums");
+  if (!rc && kind == kBivariate) rc = take_slot(&p->result);
+  if (rc) {
+    binius_sumcheck_destroy(p);
+    return rc;
   }
   *out = p;
+  return BINIUS_OK;
+}
+
+// Queues the sums of a bivariate round on the 2^n_vars values left, folding to them by r first
+// when set.
+int queue_round(binius_sumcheck* p, const uint4* r) {
+  const uint64_t L = 1ull << p->n_vars;
+  p->seq++;
+  if (L <= kRoundMax) {
+    const unsigned grid = (unsigned)std::min<uint64_t>((2 * L + kThreads - 1) / kThreads, kRoundBlocks);
+    bivariate_host_round_kernel<<<grid, kThreads, 0, p->s>>>(p->cols[0], p->cols[1], L, r != nullptr,
+                                                             r ? *r : make_uint4(0, 0, 0, 0),
+                                                             p->parts, p->result, p->seq);
+    BGPU_LAUNCH_CHECK("bivariate_host_round_kernel");
+  } else {
+    if (r) {
+      if (int rc = bivariate_fold_eval(p->cols[0], p->cols[1], 2 * L,
+                                       reinterpret_cast<const uint8_t*>(r), p->acc, p->s))
+        return rc;
+    } else {
+      if (int rc = bivariate_eval(p->cols[0], p->cols[1], L / 2, p->acc, p->s)) return rc;
+    }
+    publish_round_kernel<<<1, 1, 0, p->s>>>(reinterpret_cast<const uint4*>(p->acc), p->result,
+                                            p->seq);
+    BGPU_LAUNCH_CHECK("publish_round_kernel");
+  }
+  count_launch();
+  p->queued = true;
+  return BINIUS_OK;
+}
+
+// The queued round's sums: the host watches the result arrive for a short while (most rounds take
+// less), then waits for the stream.
+int take_round(binius_sumcheck* p, hu128& y1, hu128& yinf) {
+  const volatile uint64_t* seq = &p->result->seq;
+  for (int i = 0; i < 20000 && *seq != p->seq; i++) __builtin_ia32_pause();
+  if (*seq != p->seq) {
+    BGPU_CUDA(stream_wait(p->s));
+    if (*seq != p->seq) return set_error(BINIUS_E_CUDA, "sumcheck round left no result");
+  }
+  __atomic_thread_fence(__ATOMIC_ACQUIRE);
+  y1 = h128(&p->result->y[0]);
+  yinf = h128(&p->result->y[1]);
+  p->queued = false;
   return BINIUS_OK;
 }
 
 int build_eq(binius_sumcheck* p) {
   const uint32_t n = p->gruen_vars ? p->gruen_vars - 1 : 0;
   BGPU_ARG(n <= 32, "evaluation point longer than 33 coordinates");
-  BGPU_CUDA(cudaMalloc(&p->eq, 16ull << n));
+  BGPU_CUDA(cudaMallocAsync(&p->eq, 16ull << n, p->s));
   std::vector<uint4> pt(n);
   for (uint32_t i = 0; i < n; i++) memcpy(&pt[i], &p->point[i], 16);
   return eq_tensor(pt.data(), n, p->eq, p->s);
@@ -185,9 +353,15 @@ int do_execute(binius_sumcheck* p, int kind, void* h_coeffs, uint32_t* n_coeffs)
   const uint64_t half = 1ull << (p->n_vars - 1);
   std::vector<hu128> c;
   if (kind == kBivariate) {
-    if (int rc = bivariate_eval(p->cols[0], p->cols[1], half, p->acc, p->s)) return rc;
     hu128 y1, yinf;
-    if (int rc = read_two(p, y1, yinf)) return rc;
+    if (p->result) {
+      if (!p->queued)
+        if (int rc = queue_round(p, nullptr)) return rc;
+      if (int rc = take_round(p, y1, yinf)) return rc;
+    } else {
+      if (int rc = bivariate_eval(p->cols[0], p->cols[1], half, p->acc, p->s)) return rc;
+      if (int rc = read_two(p, y1, yinf)) return rc;
+    }
     const hu128 y0 = p->last ^ y1;  // RoundEvals2::interpolate
     c = {y0, y1 ^ y0 ^ yinf, yinf};
   } else if (kind == kQuadraticMle) {
@@ -227,6 +401,13 @@ int do_fold(binius_sumcheck* p, int kind, const void* h_challenge) {
   const uint64_t half = 1ull << (p->n_vars - 1);
   uint4 rv;
   memcpy(&rv, &r, 16);
+  if (kind == kBivariate && p->result && p->n_vars >= 2) {
+    p->n_vars--;
+    if (int rc = queue_round(p, &rv)) return rc;
+    p->last = eval_poly(p->coeffs, r);
+    p->have_coeffs = false;
+    return clear_error();
+  }
   fold_high_kernel<<<blocks_for(half), kThreads, 0, p->s>>>(p->cols[0], p->cols[1], p->cols[2],
                                                             half, rv);
   BGPU_LAUNCH_CHECK("fold_high_kernel");
@@ -337,9 +518,11 @@ int binius_sumcheck_inout_create(void* d_witness, uint32_t log_len, const void* 
 
 int binius_sumcheck_destroy(binius_sumcheck* p) {
   if (!p) return BINIUS_OK;
-  if (p->s) cudaStreamSynchronize(p->s);
-  if (p->eq) cudaFree(p->eq);
-  if (p->acc) cudaFree(p->acc);
+  // the slot and the caller's multilinears are free once the queued work is done
+  if (p->s || p->queued) cudaStreamSynchronize(p->s);
+  return_slot(p->result);
+  if (p->eq) cudaFreeAsync(p->eq, p->s);
+  if (p->acc) cudaFreeAsync(p->acc, p->s);
   delete p;
   return BINIUS_OK;
 }
