@@ -1,8 +1,9 @@
 // FRI folding, the FRI interleaved commit and FRI parameter selection.
 //
 // fold_interleaved (prover/prover/src/fri/fold.rs:260-282): each output is the inner product of a
-// 2^log_batch chunk with eq_ind(challenges).  The 256-bit carry-less products are XOR-accumulated
-// unreduced and reduced once per output (reduction is linear, so the bits are identical).
+// 2^log_batch chunk with eq_ind(challenges), on the tensor cores (fold_interleaved_tc_kernel) or,
+// for few outputs, as 256-bit carry-less products XOR-accumulated unreduced and reduced once per
+// output (reduction is linear, so the bits are identical).
 // fold_codeword (prover/prover/src/fri/fold.rs:297-318 -> verifier/verifier/src/fri/fold.rs:20-99):
 // one thread folds one coset of 2^n values in registers through all n rounds: the inverse NTT
 // butterfly with twiddle(log_len - 1 - round, index) then u + (v - u) * r.
@@ -14,6 +15,7 @@
 
 #include "gf128.cuh"
 #include "gf_reduce.cuh"
+#include "gf_tc.cuh"
 #include "internal.h"
 #include "kernels.h"
 
@@ -33,6 +35,15 @@ constexpr uint32_t kMaxChallenges = 8;
 
 struct Challenges {
   uint4 r[kMaxChallenges];
+};
+
+// A fold_codeword round in one product: with w = u + v and twiddle t,
+// u' + r (v' + u') = (1 + r) (u + w (t + rho)), rho = r / (1 + r), and the factors (1 + r) of all
+// rounds wait for one product at the end (r = 1: the round is w, without a factor).
+struct ScaledFold {
+  uint4 rho[4];
+  uint32_t ones;  // bit k: r_k = 1
+  uint4 scale;
 };
 
 unsigned grid_for(uint64_t n, unsigned threads) {
@@ -68,15 +79,153 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <int N>
+// fold_interleaved on the tensor cores (gf_tc.cuh): the 2^log_batch weights are the same for every
+// output, so an output is a sum of products by constants, which accumulate in the tensor cores'
+// sums: a thread writes its elements' operands and reads the sums once per output.  A CTA keeps
+// the matrices of 16 weights in shared memory (wider batches take a pass per 16, adding into out)
+// and two groups of 128 threads, each with a tile of 128 outputs; the products run two weights at
+// a time, on two pairs of operand slots in turn.  A sum collects up to 16 x 128 counts, so it has
+// one row, and an output's bits are formed in two parts.
+//
+// The tensor pipe would take 129 cycles per weight and tile (58 us for 2^20 outputs of 16 columns),
+// the read 42 us at the copy bandwidth; two groups of warps do not keep either busy, since a pair's
+// operands wait for the pair before last.  Measured on B200 against the kernel above: 2^20 outputs
+// of 16 columns 432 -> 140 us, of 64 columns 1666 -> 571, 2^16 of 16 38 -> 19, 2^8 of 16 22 -> 12.
+constexpr uint32_t kFoldGroups = 2;
+constexpr uint32_t kFoldThreads = kFoldGroups * tc::kGroupThreads;
+constexpr uint32_t kFoldPass = 16;  // weights per pass
+constexpr uint32_t kFoldCols = 2 * tc::kSumCols + 4 * tc::kOperandCols;  // TMEM of a group
+struct FoldTcShared {
+  uint8_t matrices[kFoldPass][tc::kMatrixBytes];
+  uint4 weights[1u << kMaxChallenges];
+  tc::MatrixRows rows[kFoldPass];
+  uint8_t ones[tc::kOnesBytes];
+  uint64_t done[kFoldGroups][2];
+  uint32_t tmem;
+};
+// Set when a wait for the tensor cores ran out (nothing more of that launch is then written).
+__device__ uint32_t g_fold_tc_stalled;
+
+__global__ void __launch_bounds__(kFoldThreads, 1)
+    fold_interleaved_tc_kernel(const uint4* __restrict__ cw, uint32_t log_len, uint32_t log_batch,
+                               Challenges ch, const uint4* __restrict__ dch,
+                               uint4* __restrict__ out) {
+  extern __shared__ __align__(128) uint8_t fold_smem[];
+  FoldTcShared& sh = *reinterpret_cast<FoldTcShared*>(fold_smem);
+  const uint32_t group = tc::uniform(threadIdx.x / tc::kGroupThreads);
+  const uint32_t gt = threadIdx.x % tc::kGroupThreads, gw = tc::uniform(gt / 32);
+  const uint32_t batch = 1u << log_batch, n_weights = min(batch, kFoldPass);
+  const uint32_t n_tiles = 1u << (log_len - 7);
+  if (threadIdx.x < 32) tc::tmem_alloc(&sh.tmem, 512);
+  if (threadIdx.x == 0) {
+    for (uint32_t g = 0; g < kFoldGroups; g++)
+      for (uint32_t b = 0; b < 2; b++) tc::mbar_init(&sh.done[g][b], 1);
+    tc::mbar_init_fence();
+  }
+  // eq_ind(r)[j] = prod_i (bit_i(j) ? r_i : 1 + r_i)
+  for (uint32_t j = threadIdx.x; j < batch; j += kFoldThreads) {
+    uint4 acc = gf_one();
+    for (uint32_t i = 0; i < log_batch; i++) {
+      uint4 f = dch ? dch[i] : ch.r[i];
+      if (!((j >> i) & 1)) f.x ^= 1u;
+      acc = gf_mul(acc, f);
+    }
+    sh.weights[j] = acc;
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tc::uniform(sh.tmem);
+  const uint32_t lanes = (gw * 32) << 16;
+  const uint32_t sums = tmem + group * kFoldCols, slots = sums + 2 * tc::kSumCols;
+  const uint32_t consts = tmem + 512 - tc::kConstCols;
+  const uint32_t matrices = tc::uniform(tc::smem_addr(sh.matrices));
+  const uint32_t ones = tc::uniform(tc::smem_addr(sh.ones));
+  if (group == 0) tc::constants_store(consts + lanes, sh.ones);
+
+  uint32_t phase[2] = {0, 0};
+  bool ok = true;
+  for (uint32_t pass = 0; pass * kFoldPass < batch; pass++) {
+    for (uint32_t x = threadIdx.x; x < n_weights * tc::kRowItems; x += kFoldThreads)
+      tc::matrix_rows(sh.rows[x / tc::kRowItems], sh.weights[pass * kFoldPass + x / tc::kRowItems],
+                      x % tc::kRowItems);
+    __syncthreads();
+    for (uint32_t w = group; w < n_weights; w += kFoldGroups)
+      tc::matrix_build(sh.matrices[w], sh.rows[w], gt);
+    tc::fence_smem_to_tensor();
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    for (uint32_t t = blockIdx.x * kFoldGroups + group; t < n_tiles; t += gridDim.x * kFoldGroups) {
+      const uint64_t i = (uint64_t)t * tc::kGroupThreads + gt;
+      const uint4* row = cw + (i << log_batch) + pass * kFoldPass;
+      const uint32_t pairs = (n_weights + 1) / 2;
+      uint4 x0 = __ldg(row), x1 = n_weights > 1 ? __ldg(row + 1) : gf_zero();
+      for (uint32_t k = 0; k < pairs; k++) {
+        const uint32_t b = k & 1;
+        if (k >= 2) {  // this pair of slots' products before last
+          ok = tc::mbar_wait(&sh.done[group][b], phase[b]) && ok;
+          phase[b] ^= 1;
+          tc::fence_after();
+        }
+        uint32_t r[16];
+        tc::operand_words(x0, r);
+        tc::operand_store(slots + 2 * b * tc::kOperandCols + lanes, r);
+        if (n_weights > 1) {
+          tc::operand_words(x1, r);
+          tc::operand_store(slots + (2 * b + 1) * tc::kOperandCols + lanes, r);
+        }
+        if (k + 1 < pairs) {
+          x0 = __ldg(row + 2 * k + 2);
+          x1 = __ldg(row + 2 * k + 3);
+        }
+        tc::wait_stores();
+        tc::fence_before();
+        // two pairs can be under way, so each pair of slots has a barrier of its own
+        const uint32_t barrier = 1 + 2 * group + b;
+        if (gw != (k & 3)) {
+          tc::group_arrive(barrier);
+          continue;
+        }
+        tc::group_wait(barrier);
+        tc::fence_after();
+        for (uint32_t part = 0; part < 2; part++) {
+          if (k == 0) tc::issue_ones(sums + part * tc::kSumCols, consts, ones);
+          for (uint32_t w = 2 * k; w < min(2 * k + 2, n_weights); w++)
+            tc::issue_part(sums + part * tc::kSumCols,
+                           slots + (2 * b + (w & 1)) * tc::kOperandCols,
+                           matrices + w * tc::kMatrixBytes, part, consts);
+        }
+        tc::commit(&sh.done[group][b]);
+      }
+      for (uint32_t k = pairs > 2 ? pairs - 2 : 0; k < pairs; k++) {
+        ok = tc::mbar_wait(&sh.done[group][k & 1], phase[k & 1]) && ok;
+        phase[k & 1] ^= 1;
+      }
+      tc::fence_after();
+      const uint2 p0 = tc::collect_part(sums + lanes);
+      const uint2 p1 = tc::collect_part(sums + tc::kSumCols + lanes);
+      uint4 y = tc::join_parts(p0, p1);
+      if (pass) gf_add_into(y, out[i]);
+      if (ok) out[i] = y;
+    }
+    tc::fence_before();
+    __syncthreads();
+  }
+  if (!ok) atomicOr(&g_fold_tc_stalled, 1u);
+  if (threadIdx.x < 32) tc::tmem_free(tmem, 512);
+}
+
+// SCALED: rounds of one product (sf), else challenges from ch or dch and two products a round.
+template <int N, bool SCALED>
 __global__ void __launch_bounds__(256)
     fold_codeword_kernel(const uint4* __restrict__ cw, uint32_t log_len,
-                         const uint4* __restrict__ tw, Challenges ch, const uint4* __restrict__ dch,
-                         uint4* __restrict__ out) {
+                         const uint4* __restrict__ tw, ScaledFold sf, Challenges ch,
+                         const uint4* __restrict__ dch, uint4* __restrict__ out) {
   const uint64_t n_chunks = 1ull << (log_len - N);
   uint4 rr[N];
 #pragma unroll
-  for (int kk = 0; kk < N; kk++) rr[kk] = dch ? dch[kk] : ch.r[kk];
+  for (int kk = 0; kk < N; kk++) rr[kk] = SCALED ? sf.rho[kk] : dch ? dch[kk] : ch.r[kk];
   for (uint64_t ci = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; ci < n_chunks;
        ci += (uint64_t)gridDim.x * blockDim.x) {
     uint4 v[1 << N];
@@ -94,14 +243,21 @@ __global__ void __launch_bounds__(256)
         const uint64_t index = (ci << (size - 1)) | (uint64_t)off;
         const uint4 t = __ldg(tw + layer_base + index);
         gf_add_into(w, u);
-        gf_add_into(u, gf_mul(w, t));
-        gf_add_into(w, u);  // w - u
-        gf_add_into(u, gf_mul(w, r));
+        if (SCALED) {
+          if ((sf.ones >> kk) & 1)
+            u = w;
+          else
+            gf_add_into(u, gf_mul(w, gf_add(t, r)));
+        } else {
+          gf_add_into(u, gf_mul(w, t));
+          gf_add_into(w, u);  // w - u
+          gf_add_into(u, gf_mul(w, r));
+        }
         v[off] = u;
       }
       cur--;
     }
-    out[ci] = v[0];
+    out[ci] = SCALED ? gf_mul(v[0], sf.scale) : v[0];
   }
 }
 
@@ -109,11 +265,12 @@ __global__ void __launch_bounds__(256)
 // nearly empty and each thread's 2 (2^N - 1) dependent multiplies are the launch's latency.  Here
 // a chunk takes P = 2^(N-1) consecutive lanes: in a round of 2^size values, lane q < 2^(size-1)
 // holds values 2q and 2q + 1, runs butterfly q and keeps its output, which lanes 2q' and 2q' + 1
-// hand to lane q' by shuffles for the next round.  The chain is N rounds of two multiplies.
-template <int N>
+// hand to lane q' by shuffles for the next round.  The chain is N rounds of two multiplies, or of
+// one and the scaling.
+template <int N, bool SCALED>
 __global__ void __launch_bounds__(256)
     fold_codeword_lanes_kernel(const uint4* __restrict__ cw, uint32_t log_len,
-                               const uint4* __restrict__ tw, Challenges ch,
+                               const uint4* __restrict__ tw, ScaledFold sf, Challenges ch,
                                const uint4* __restrict__ dch, uint4* __restrict__ out) {
   constexpr uint32_t P = 1u << (N - 1);
   const uint64_t n_chunks = 1ull << (log_len - N);
@@ -141,18 +298,25 @@ __global__ void __launch_bounds__(256)
         u = a;
       }
       if (live && q < (1u << (size - 1))) {
-        const uint4 r = dch ? dch[kk] : ch.r[kk];
+        const uint4 r = SCALED ? sf.rho[kk] : dch ? dch[kk] : ch.r[kk];
         const uint64_t layer_base = (1ull << (cur - 1)) - 1;
         const uint64_t index = (ci << (size - 1)) | (uint64_t)q;
         const uint4 t = __ldg(tw + layer_base + index);
         gf_add_into(w, u);
-        gf_add_into(u, gf_mul(w, t));
-        gf_add_into(w, u);
-        gf_add_into(u, gf_mul(w, r));
+        if (SCALED) {
+          if ((sf.ones >> kk) & 1)
+            u = w;
+          else
+            gf_add_into(u, gf_mul(w, gf_add(t, r)));
+        } else {
+          gf_add_into(u, gf_mul(w, t));
+          gf_add_into(w, u);
+          gf_add_into(u, gf_mul(w, r));
+        }
       }
       cur--;
     }
-    if (live && q == 0) out[ci] = u;
+    if (live && q == 0) out[ci] = SCALED ? gf_mul(u, sf.scale) : u;
   }
 }
 
@@ -175,15 +339,70 @@ int load_challenges(const void* h, uint32_t n, Challenges& ch) {
 // lane-parallel kernel.
 constexpr uint64_t kCompactFoldChunks = 148ull * 256;
 
+// Challenges the host knows take the scaled form: 16 products for a coset of 16 values against 30.
+// Measured on B200, four challenges, not scaled -> scaled: 2^22 values 390 -> 143 us, 2^20 141 -> 44,
+// 2^16 13 -> 10.  (For challenges in device memory the inversion would cost what it saves.)
+ScaledFold scaled_fold(const Challenges& ch, uint32_t n) {
+  ScaledFold sf;
+  memset(&sf, 0, sizeof(sf));
+  hu128 scale = 1;
+  for (uint32_t k = 0; k < n; k++) {
+    hu128 r;
+    memcpy(&r, &ch.r[k], 16);
+    if (r == 1) {
+      sf.ones |= 1u << k;
+      continue;
+    }
+    const hu128 rho = host_gf_mul(r, host_gf_inv(r ^ 1));
+    memcpy(&sf.rho[k], &rho, 16);
+    scale = host_gf_mul(scale, r ^ 1);
+  }
+  memcpy(&sf.scale, &scale, 16);
+  return sf;
+}
+
+template <int N, bool SCALED>
+void launch_fold_codeword_as(const uint4* cw, uint32_t log_len, const uint4* tw,
+                             const ScaledFold& sf, const Challenges& ch, const uint4* dch,
+                             uint4* out, cudaStream_t s) {
+  uint64_t n_chunks = 1ull << (log_len - N);
+  if (n_chunks < kCompactFoldChunks)
+    fold_codeword_lanes_kernel<N, SCALED><<<grid_for(n_chunks << (N - 1), 256), 256, 0, s>>>(
+        cw, log_len, tw, sf, ch, dch, out);
+  else
+    fold_codeword_kernel<N, SCALED><<<grid_for(n_chunks, 256), 256, 0, s>>>(cw, log_len, tw, sf,
+                                                                            ch, dch, out);
+}
+
 template <int N>
 void launch_fold_codeword(const uint4* cw, uint32_t log_len, const uint4* tw, const Challenges& ch,
                           const uint4* dch, uint4* out, cudaStream_t s) {
-  uint64_t n_chunks = 1ull << (log_len - N);
-  if (n_chunks < kCompactFoldChunks)
-    fold_codeword_lanes_kernel<N><<<grid_for(n_chunks << (N - 1), 256), 256, 0, s>>>(
-        cw, log_len, tw, ch, dch, out);
+  if (dch)
+    launch_fold_codeword_as<N, false>(cw, log_len, tw, ScaledFold{}, ch, dch, out, s);
   else
-    fold_codeword_kernel<N><<<grid_for(n_chunks, 256), 256, 0, s>>>(cw, log_len, tw, ch, dch, out);
+    launch_fold_codeword_as<N, true>(cw, log_len, tw, scaled_fold(ch, N), ch, dch, out, s);
+}
+
+int launch_fold_interleaved(const void* d_codeword, uint32_t log_len, uint32_t log_batch,
+                            const Challenges& ch, const uint4* dch, void* d_out, cudaStream_t s) {
+  // from one tile of outputs up; a batch of one element is a copy
+  if (log_batch > 0 && log_len >= 7 && log_len < 38) {
+    const void* kern = reinterpret_cast<const void*>(fold_interleaved_tc_kernel);
+    if (int rc = ensure_smem_limit(kern, sizeof(FoldTcShared))) return rc;
+    const uint64_t ctas = ((1ull << (log_len - 7)) + kFoldGroups - 1) / kFoldGroups;
+    fold_interleaved_tc_kernel<<<(unsigned)std::min<uint64_t>(ctas, 148), kFoldThreads,
+                                 sizeof(FoldTcShared), s>>>(
+        static_cast<const uint4*>(d_codeword), log_len, log_batch, ch, dch,
+        static_cast<uint4*>(d_out));
+    BGPU_LAUNCH_CHECK("fold_interleaved_tc_kernel");
+  } else {
+    fold_interleaved_kernel<<<grid_for(1ull << log_len, 256), 256, 0, s>>>(
+        static_cast<const uint4*>(d_codeword), log_len, log_batch, ch, dch,
+        static_cast<uint4*>(d_out));
+    BGPU_LAUNCH_CHECK("fold_interleaved_kernel");
+  }
+  count_launch();
+  return BINIUS_OK;
 }
 
 // ---- Scratch for binius_fri_fold_codeword_noalloc ----
@@ -280,12 +499,7 @@ int fri_fold_interleaved_dev(const void* d_codeword, uint32_t log_len, uint32_t 
   if (log_batch > kMaxChallenges) return set_error(BINIUS_E_ARG, "at most 8 folding challenges");
   Challenges none;
   memset(&none, 0, sizeof(none));
-  fold_interleaved_kernel<<<grid_for(1ull << log_len, 256), 256, 0, s>>>(
-      static_cast<const uint4*>(d_codeword), log_len, log_batch, none, d_challenges,
-      static_cast<uint4*>(d_out));
-  BGPU_LAUNCH_CHECK("fold_interleaved_kernel");
-  count_launch();
-  return BINIUS_OK;
+  return launch_fold_interleaved(d_codeword, log_len, log_batch, none, d_challenges, d_out, s);
 }
 
 int fri_fold_codeword_dev(const binius_ntt* ntt, const void* d_codeword, uint32_t log_len,
@@ -326,12 +540,9 @@ int binius_fri_fold_interleaved(const void* d_codeword, uint32_t log_len, uint32
   BGPU_ARG(log_len + log_batch <= 40, "codeword too large");
   Challenges ch;
   if (int rc = load_challenges(h_challenges, log_batch, ch)) return rc;
-  cudaStream_t s = as_stream(stream);
-  fold_interleaved_kernel<<<grid_for(1ull << log_len, 256), 256, 0, s>>>(
-      static_cast<const uint4*>(d_codeword), log_len, log_batch, ch, nullptr,
-      static_cast<uint4*>(d_out));
-  BGPU_LAUNCH_CHECK("fold_interleaved_kernel");
-  count_launch();
+  if (int rc = launch_fold_interleaved(d_codeword, log_len, log_batch, ch, nullptr, d_out,
+                                       as_stream(stream)))
+    return rc;
   return clear_error();
 }
 

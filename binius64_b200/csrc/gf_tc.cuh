@@ -71,7 +71,8 @@ __device__ __forceinline__ void fence_smem_to_tensor() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Named barrier of a group: its writes are seen by the warps that wait; the others go on.
+// Named barrier of a group: its writes are seen by the warps that wait; the others go on.  A warp
+// may arrive again only when the barrier has completed (say, because what it guarded has).
 __device__ __forceinline__ void group_arrive(uint32_t id) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kGroupThreads) : "memory");
 }
@@ -87,10 +88,11 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
 __device__ __forceinline__ void mbar_init_fence() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Waits (a bounded number of polls, far beyond any tile's time) for the phase of this parity.
+// Waits for the phase of this parity: a bounded number of polls, each of which may sleep for some
+// 20 us, far beyond any tile's time.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t a = smem_addr(bar);
-  for (uint32_t i = 0; i < (1u << 22); i++) {
+  for (uint32_t i = 0; i < (1u << 16); i++) {
     uint32_t ok;
     asm volatile(
         "{\n.reg .pred p;\n"
