@@ -5,9 +5,11 @@
 // last; node i of layer k+1 compresses nodes 2i and 2i+1 of layer k (parallel_compression.rs:79-91).
 //
 // B200 mapping: one thread hashes one leaf (its 2^log_batch elements are read as 128-bit loads);
-// the CTA's 256 leaf digests stay in shared memory and the next 8 tree layers are compressed there
-// before anything but the layer outputs touches HBM.  Upper layers run in CTAs that fuse 9 layers
-// (512 inputs -> 1).  SHA-256 is pure integer work (funnel-shift rotates, three-input logic ops, adds).
+// the CTA's 256 leaf digests stay in shared memory and the next tree layers are compressed there
+// before anything but the layer outputs touches HBM: all 8 of them in a small tree, whose time is
+// its chain of layers and launches, three in a large one, which keeps every warp full.  Upper layers
+// run in CTAs that fuse up to 9 layers (512 inputs -> 1).  SHA-256 is pure integer work
+// (funnel-shift rotates, three-input logic ops, adds).
 #include <string.h>
 
 #include <algorithm>
@@ -23,6 +25,15 @@ namespace {
 
 constexpr uint32_t kLeafFuse = 8;  // at most 2^8 leaves per CTA (Tuning::merkle_leaf_fuse)
 constexpr uint32_t kNodeFuse = 9;  // at most 2^9 inputs per CTA (Tuning::merkle_node_fuse)
+// From 2^17 inputs up a launch stops after three layers, where its 256-thread CTAs have a full warp
+// left: the ALU pipe bounds it (SHA-256's rotates and three-input logic, 1024 of its 1376
+// instructions), and the layers above would run the pipe for a warp with 16, 8, .. 1 lanes on.
+// Measured on B200, all layers of a CTA -> three, in us: 2^24 leaves of one element 3147 -> 2458
+// (13.7 G compressions/s), 2^22 819 -> 653, 2^20 237 -> 194, 2^20 of 16 elements 545 -> 471, 2^18 89
+// -> 74, 2^17 64 -> 58; at 2^16 (47 -> 46) and below (2^15 33 -> 44) the added launches cost what the
+// idle lanes do, or more.  Two or four layers are within 4% of three.
+constexpr uint32_t kFullLog = 17;
+constexpr uint32_t kFullLayers = 3;
 
 __host__ __device__ __forceinline__ uint64_t layer_offset(uint32_t L, uint32_t k) {
   return (1ull << (L + 1)) - (1ull << (L + 1 - k));
@@ -39,16 +50,18 @@ __device__ __forceinline__ void load_digest(const uint4* nodes, uint64_t i, uint
   d[4] = b.x; d[5] = b.y; d[6] = b.z; d[7] = b.w;
 }
 
-// Hashes 2^fused leaves per CTA and compresses `fused` layers above them in shared memory.
+// Hashes blockDim.x leaves per CTA and compresses `fused` layers above them in shared memory.
+template <int N>
 __global__ void __launch_bounds__(256) merkle_leaves_kernel(const uint4* __restrict__ elems,
                                                             uint32_t log_batch,
                                                             uint4* __restrict__ nodes, uint32_t L,
-                                                            uint32_t fused, NodeIV iv) {
+                                                            uint32_t fused, NodeIV iv,
+                                                            PadSchedule pad) {
   __shared__ uint32_t buf[2][256][9];  // padded rows avoid bank conflicts
   const uint32_t tid = threadIdx.x;
   const uint64_t leaf = (uint64_t)blockIdx.x * blockDim.x + tid;
   uint32_t d[8];
-  sha256_elems(elems + (leaf << log_batch), 1u << log_batch, d);
+  sha256_elems<N>(elems + (leaf << log_batch), 1u << log_batch, pad, d);
   store_digest(nodes, leaf, d);
 #pragma unroll
   for (int i = 0; i < 8; i++) buf[0][tid][i] = d[i];
@@ -71,7 +84,7 @@ __global__ void __launch_bounds__(256) merkle_leaves_kernel(const uint4* __restr
   }
 }
 
-// Compresses `fused` layers starting from layer in_level; each CTA reduces 2^fused inputs.
+// Compresses `fused` layers starting from layer in_level; a CTA has 2 blockDim.x inputs.
 __global__ void __launch_bounds__(256) merkle_nodes_kernel(uint4* __restrict__ nodes, uint32_t L,
                                                            uint32_t in_level, uint32_t fused,
                                                            NodeIV iv) {
@@ -106,6 +119,17 @@ __global__ void __launch_bounds__(256) merkle_nodes_kernel(uint4* __restrict__ n
   }
 }
 
+// The last block of a message of n_elems elements, n_elems a multiple of 4.
+PadSchedule pad_schedule(uint32_t n_elems) {
+  PadSchedule p = {{0x80000000u}};
+  p.w[15] = n_elems * 128u;
+  auto rotr = [](uint32_t x, int n) { return (x >> n) | (x << (32 - n)); };
+  for (int t = 16; t < 64; t++)
+    p.w[t] = p.w[t - 16] + (rotr(p.w[t - 15], 7) ^ rotr(p.w[t - 15], 18) ^ (p.w[t - 15] >> 3)) +
+             p.w[t - 7] + (rotr(p.w[t - 2], 17) ^ rotr(p.w[t - 2], 19) ^ (p.w[t - 2] >> 10));
+  return p;
+}
+
 }  // namespace
 
 namespace bgpu {
@@ -136,21 +160,33 @@ int merkle_commit(const void* d_elems, uint32_t log_leaves, uint32_t log_batch, 
   uint4* nodes = static_cast<uint4*>(d_nodes);
   const uint32_t leaf_fuse = std::max(5u, std::min(kLeafFuse, tuning().merkle_leaf_fuse));
   const uint32_t node_fuse = std::max(5u, std::min(kNodeFuse, tuning().merkle_node_fuse));
-  uint32_t fused = std::min(L, leaf_fuse);
-  uint64_t grid = 1ull << (L - fused);
+  const uint32_t log_cta = std::min(L, leaf_fuse);
+  const uint64_t grid = 1ull << (L - log_cta);
   BGPU_ARG(grid <= 0x7fffffffull, "too many leaves");
-  merkle_leaves_kernel<<<(unsigned)grid, 1u << fused, 0, stream>>>(
-      static_cast<const uint4*>(d_elems), log_batch, nodes, L, fused, iv);
+  auto layers = [](uint32_t log_inputs, uint32_t cta_layers) {
+    return log_inputs >= kFullLog ? std::min(cta_layers, kFullLayers) : cta_layers;
+  };
+  const auto* elems = static_cast<const uint4*>(d_elems);
+  uint32_t level = layers(L, log_cta);
+  // the last block's schedule as an argument pays for large trees only: a small one's time is the
+  // latency of a few warps, to which the reads of the argument add (1 us a launch)
+  const bool large = L >= kFullLog;
+  const PadSchedule pad = large ? pad_schedule(1u << log_batch) : PadSchedule{};
+  auto kern = !large           ? merkle_leaves_kernel<0>
+              : log_batch == 0 ? merkle_leaves_kernel<1>
+              : log_batch == 1 ? merkle_leaves_kernel<2>
+                               : merkle_leaves_kernel<4>;
+  kern<<<(unsigned)grid, 1u << log_cta, 0, stream>>>(elems, log_batch, nodes, L, level, iv, pad);
   BGPU_LAUNCH_CHECK("merkle_leaves_kernel");
   count_launch();
-  uint32_t level = fused;
   while (level < L) {
-    uint32_t f = std::min(L - level, node_fuse);
-    uint64_t g = 1ull << (L - level - f);
-    merkle_nodes_kernel<<<(unsigned)g, 1u << (f - 1), 0, stream>>>(nodes, L, level, f, iv);
+    const uint32_t f = std::min(L - level, node_fuse);
+    const uint64_t g = 1ull << (L - level - f);
+    const uint32_t fused = layers(L - level, f);
+    merkle_nodes_kernel<<<(unsigned)g, 1u << (f - 1), 0, stream>>>(nodes, L, level, fused, iv);
     BGPU_LAUNCH_CHECK("merkle_nodes_kernel");
     count_launch();
-    level += f;
+    level += fused;
   }
   return clear_error();
 }
