@@ -118,8 +118,8 @@ void prover_note_footprint(const binius_prover* P, uint64_t bytes);
 struct Tuning {
   uint32_t tail_log = 11;          // sumcheck rounds on <= 2^tail_log elements: single-CTA tail
   uint32_t ntt_pass_layers = 8;    // NTT layers fused per shared-memory pass (<= 8)
-  uint32_t merkle_leaf_fuse = 8;   // Merkle leaf CTA: 2^fuse leaves, as many layers above them
-  uint32_t merkle_node_fuse = 9;   // Merkle node CTA: 2^fuse inputs (<= 9)
+  uint32_t merkle_leaf_fuse = 8;   // Merkle leaf CTA of a tree above 2^13 leaves: 2^fuse of them
+  uint32_t merkle_node_fuse = 9;   // Merkle node CTA above it: 2^fuse inputs (<= 9)
   uint32_t ntt_tile_bits = 12;     // NTT shared-memory tile: 2^bits elements (9..12)
 };
 // The calling thread's current choices (a prove sets its prover's for its duration).

@@ -6,8 +6,9 @@
 //
 // B200 mapping: one thread hashes one leaf (its 2^log_batch elements are read as 128-bit loads);
 // the CTA's 256 leaf digests stay in shared memory and the next tree layers are compressed there
-// before anything but the layer outputs touches HBM: all 8 of them in a small tree, whose time is
-// its chain of layers and launches, three in a large one, which keeps every warp full.  Upper layers
+// before anything but the layer outputs touches HBM: all 8 of them in a tree of up to 2^16 leaves,
+// three in a larger one, which keeps every warp full.  Trees of up to 2^13 leaves, whose time is one
+// chain of compressions, run merkle_chain_kernel.  Upper layers
 // run in CTAs that fuse up to 9 layers (512 inputs -> 1).  SHA-256 is pure integer work
 // (funnel-shift rotates, three-input logic ops, adds).
 #include <string.h>
@@ -17,6 +18,7 @@
 
 #include "host_sha256.h"
 #include "internal.h"
+#include "pdl.cuh"
 #include "sha256.cuh"
 
 using namespace bgpu;
@@ -130,6 +132,204 @@ PadSchedule pad_schedule(uint32_t n_elems) {
   return p;
 }
 
+// ---- small trees
+//
+// A tree of few leaves is a chain: a leaf's blocks one after the other, then the layers.  One warp
+// alone takes 2.1 k cycles a compression (1024 instructions of the half-rate ALU pipe, 8 of 18 a
+// round for the message schedule), and two warps on one scheduler twice that.  Here a CTA has 32
+// nodes, one to a lane, and only warp 0, alone on its scheduler, runs their rounds; warps 1, 2 and
+// 3 prepare the schedules, block b on warp 1 + b mod 3, 16 words at a time through shared memory.
+// A layer's schedule starts from the digests that warp 0 leaves in shared memory, while warp 0 runs
+// the first 16 rounds from the same words.
+//
+// Measured on B200 against a thread per leaf and 256 leaves per CTA, in us with the launches: 2^8
+// leaves of 64 elements 62 -> 37, 2^10 of 16 37 -> 24, 2^12 of 16 40 -> 29, 2^13 of one 30 -> 26 and
+// of 16 42 -> 33; at 2^14 they meet (32 -> 31, 43 -> 42), where several of these CTAs share an SM and
+// their first warps its scheduler, and above it loses (2^15 33 -> 47).  A compression of the chain
+// takes 1.3 us, 39 cycles a round, of which the 14 instructions of the half-rate pipes are 28.
+constexpr uint32_t kChainMaxLog = 13;
+constexpr uint32_t kChainLog = 5;  // a CTA's nodes
+constexpr uint32_t kChainThreads = 128;
+struct ChainShared {
+  uint32_t kw[3][64][32];  // K[t] + W[t] of block b mod 3, a column a lane
+  uint4 digests[2][32][2];
+};
+// Named barriers of warp 0 and a buffer's warp: words 16 c .. written (c < 4; c = 0 of a layer: its
+// digests written, by warp 0), all words read (c = 4).
+__device__ __forceinline__ uint32_t chain_bar(uint32_t buffer, uint32_t c) {
+  return 1 + 5 * buffer + c;
+}
+__device__ __forceinline__ void chain_arrive(uint32_t id) {
+  asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
+__device__ __forceinline__ void chain_wait(uint32_t id) {
+  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+
+// Rounds t0 .. t0 + 15 from their words; the eight state words rotate through v.
+__device__ __forceinline__ void chain_rounds(uint32_t (&v)[8], const uint32_t (&k)[16]) {
+  uint32_t a = v[0], b = v[1], c = v[2], d = v[3], e = v[4], f = v[5], g = v[6], h = v[7];
+#pragma unroll
+  for (int t = 0; t < 16; t++) {
+    const uint32_t S1 = rotr32(e, 6) ^ rotr32(e, 11) ^ rotr32(e, 25);
+    const uint32_t ch = (e & f) ^ (~e & g);
+    const uint32_t S0 = rotr32(a, 2) ^ rotr32(a, 13) ^ rotr32(a, 22);
+    const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
+    const uint32_t y = ch + (h + k[t]);
+    const uint32_t ne = (d + y) + S1, na = (y + S1) + (S0 + mj);
+    h = g;
+    g = f;
+    f = e;
+    e = ne;
+    d = c;
+    c = b;
+    b = a;
+    a = na;
+  }
+  v[0] = a;
+  v[1] = b;
+  v[2] = c;
+  v[3] = d;
+  v[4] = e;
+  v[5] = f;
+  v[6] = g;
+  v[7] = h;
+}
+
+// The words of lane's node of a layer above: the digests of nodes 2 lane and 2 lane + 1 below (lanes
+// past the layer's end take others').
+__device__ __forceinline__ void chain_children(const uint4 (&d)[32][2], uint32_t (&w)[16]) {
+  const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint4 v = d[(2 * lane + i / 2) & 31][i & 1];
+    w[4 * i + 0] = bswap32(v.x);
+    w[4 * i + 1] = bswap32(v.y);
+    w[4 * i + 2] = bswap32(v.z);
+    w[4 * i + 3] = bswap32(v.w);
+  }
+}
+
+// NODES = false: hashes 2^log_n leaves per CTA (log_n <= 5) and compresses the log_n layers above
+// them.  NODES = true: compresses the log_n + 1 layers above layer in_level, 2^(log_n + 1) of its
+// nodes per CTA.
+template <bool NODES>
+__global__ void __launch_bounds__(kChainThreads)
+    merkle_chain_kernel(const uint4* __restrict__ elems, uint32_t log_batch,
+                        uint4* __restrict__ nodes, uint32_t L, uint32_t in_level, uint32_t log_n,
+                        NodeIV iv) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ ChainShared sh;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x / 32, n = 1u << log_n;
+  const uint32_t n_elems = 1u << log_batch;
+  const uint32_t n_blocks = NODES ? 1 : n_elems / 4 + 1, total = n_blocks + log_n;
+  const uint64_t first = (uint64_t)blockIdx.x << log_n;  // of this CTA's nodes of the lowest layer
+  const uint64_t mine = first + (lane & (n - 1));
+  if (warp) {
+    for (uint32_t b = warp - 1; b < total; b += 3) {
+      const uint32_t buf = warp - 1;
+      // warp 0 is through with the buffer's last block, and so with that one's barriers
+      if (b >= 3) chain_wait(chain_bar(buf, 4));
+      uint32_t w[16];
+      if (b >= n_blocks) {
+        chain_wait(chain_bar(buf, 0));
+        chain_children(sh.digests[(b - n_blocks) & 1], w);
+      } else if (NODES) {
+        const uint4* src = nodes + 2 * (layer_offset(L, in_level) + 2 * mine);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const uint4 v = src[i];
+          w[4 * i + 0] = bswap32(v.x);
+          w[4 * i + 1] = bswap32(v.y);
+          w[4 * i + 2] = bswap32(v.z);
+          w[4 * i + 3] = bswap32(v.w);
+        }
+      } else {
+        const uint4* src = elems + (mine << log_batch);
+        const uint32_t end = b + 1 == n_blocks;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const uint32_t e = 4 * b + i;
+          uint4 v = make_uint4(e == n_elems ? 0x80u : 0u, 0u, 0u, 0u);
+          if (e < n_elems) v = __ldg(src + e);
+          w[4 * i + 0] = bswap32(v.x);
+          w[4 * i + 1] = bswap32(v.y);
+          w[4 * i + 2] = bswap32(v.z);
+          w[4 * i + 3] = bswap32(v.w);
+        }
+        if (end) w[15] = n_elems * 128u;
+      }
+#pragma unroll 1
+      for (uint32_t c = 0; c < 4; c++) {
+        if (c) {
+#pragma unroll
+          for (int t = 0; t < 16; t++) {
+            const uint32_t w15 = w[(t + 1) & 15], w2 = w[(t + 14) & 15];
+            const uint32_t s0 = rotr32(w15, 7) ^ rotr32(w15, 18) ^ (w15 >> 3);
+            const uint32_t s1 = rotr32(w2, 17) ^ rotr32(w2, 19) ^ (w2 >> 10);
+            w[t] = w[t] + s0 + w[(t + 9) & 15] + s1;
+          }
+        } else if (b >= n_blocks) {
+          continue;  // warp 0 has these words
+        }
+#pragma unroll
+        for (int t = 0; t < 16; t++) sh.kw[buf][16 * c + t][lane] = w[t] + kSha256K[16 * c + t];
+        chain_arrive(chain_bar(buf, c));
+      }
+    }
+    return;
+  }
+  uint32_t s[8], buf = 0;
+  if (NODES) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] = iv.w[i];
+  } else {
+    sha256_init(s);
+  }
+  for (uint32_t b = 0; b < total; b++, buf = buf == 2 ? 0 : buf + 1) {
+    const bool layer = b >= n_blocks;
+    uint32_t k[16];
+    if (layer) {
+      chain_children(sh.digests[(b - n_blocks) & 1], k);
+#pragma unroll
+      for (int t = 0; t < 16; t++) k[t] += kSha256K[t];
+#pragma unroll
+      for (int i = 0; i < 8; i++) s[i] = iv.w[i];
+    }
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = s[i];
+#pragma unroll 1
+    for (uint32_t c = 0; c < 4; c++) {
+      if (c || !layer) {
+        chain_wait(chain_bar(buf, c));
+#pragma unroll
+        for (int t = 0; t < 16; t++) k[t] = sh.kw[buf][16 * c + t][lane];
+      }
+      chain_rounds(v, k);
+    }
+    if (b + 3 < total) chain_arrive(chain_bar(buf, 4));
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] += v[i];
+    if (b + 1 < n_blocks) continue;
+    uint32_t o[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i] = NODES || layer ? s[i] : bswap32(s[i]);
+    const uint32_t up = b + 1 - n_blocks;
+    if (up < log_n) {
+      sh.digests[up & 1][lane][0] = make_uint4(o[0], o[1], o[2], o[3]);
+      sh.digests[up & 1][lane][1] = make_uint4(o[4], o[5], o[6], o[7]);
+      __syncwarp();
+      chain_arrive(chain_bar(buf == 2 ? 0 : buf + 1, 0));
+    }
+    if (lane < n >> up)
+      store_digest(nodes, layer_offset(L, in_level + up + (NODES ? 1 : 0)) + (first >> up) + lane,
+                   o);
+    __syncwarp();
+  }
+}
+
 }  // namespace
 
 namespace bgpu {
@@ -158,6 +358,24 @@ int merkle_commit(const void* d_elems, uint32_t log_leaves, uint32_t log_batch, 
   const uint32_t L = log_leaves;
   const NodeIV iv = node_iv();
   uint4* nodes = static_cast<uint4*>(d_nodes);
+  if (L <= kChainMaxLog) {
+    uint32_t level = std::min(L, kChainLog);
+    auto launch = [&](auto kern, uint32_t grid_log, uint32_t in_level, uint32_t log_n) {
+      cudaError_t e = launch_pdl(kern, 1u << grid_log, kChainThreads, 0, stream,
+                                 static_cast<const uint4*>(d_elems), log_batch, nodes, L, in_level,
+                                 log_n, iv);
+      if (e != cudaSuccess) return cuda_error(e, "merkle_chain_kernel");
+      count_launch();
+      return (int)BINIUS_OK;
+    };
+    if (int rc = launch(merkle_chain_kernel<false>, L - level, 0, level)) return rc;
+    while (level < L) {
+      const uint32_t f = std::min(L - level, kChainLog + 1);
+      if (int rc = launch(merkle_chain_kernel<true>, L - level - f, level, f - 1)) return rc;
+      level += f;
+    }
+    return clear_error();
+  }
   const uint32_t leaf_fuse = std::max(5u, std::min(kLeafFuse, tuning().merkle_leaf_fuse));
   const uint32_t node_fuse = std::max(5u, std::min(kNodeFuse, tuning().merkle_node_fuse));
   const uint32_t log_cta = std::min(L, leaf_fuse);

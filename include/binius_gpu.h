@@ -307,8 +307,9 @@ int binius_prove(const binius_prover* prover, const uint64_t* h_words, size_t n_
 /* Launch-shape choices of a prover's proofs, none of which changes a result (the arithmetic is
  * exact): h5 = {tail_log: sumcheck rounds on at most 2^tail_log elements run in one single-CTA
  * kernel (8..12, default 11); ntt_pass_layers: NTT layers fused per shared-memory pass (4..8,
- * default 8); merkle_leaf_fuse: a Merkle leaf CTA hashes 2^k leaves and compresses k layers above
- * them (5..8, default 8); merkle_node_fuse: a node CTA reduces 2^k inputs (5..9, default 9);
+ * default 8); merkle_leaf_fuse: a Merkle leaf CTA hashes 2^k leaves and compresses up to k layers
+ * above them (5..8, default 8); merkle_node_fuse: a node CTA has 2^k inputs (5..9, default 9; both
+ * for trees of more than 2^13 leaves);
  * ntt_tile_bits: an NTT pass works on tiles of 2^k elements (9..12, default 12)}.
  * No reference counterpart (the reference's rayon code has no launch shapes).  Not while a prove
  * on the prover is in flight.

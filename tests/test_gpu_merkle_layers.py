@@ -1,7 +1,6 @@
-"""SHA-256 trees against the CPU oracle, every digest: the sizes around the one from which a launch
-stops after three layers (and those whose last launch then has one, two or three), and leaves of
-one element, two, one block and several, whose last blocks are formed differently in large trees
-and in small ones."""
+"""SHA-256 trees against the CPU oracle, every digest: the sizes around those where another kernel or
+another split of the layers over the launches begins, and leaves of one element, two, one block and
+several, whose last blocks are formed differently by each kernel."""
 import numpy as np
 import pytest
 
@@ -17,7 +16,8 @@ import binius64_b200 as bg  # noqa: E402
 
 
 @pytest.mark.parametrize("log_leaves,log_batch", [
-    (0, 0), (3, 1), (9, 2), (16, 0), (17, 0), (17, 1), (18, 2), (19, 0), (20, 1), (17, 3), (7, 7),
+    (0, 0), (0, 3), (1, 7), (2, 2), (3, 1), (4, 4), (5, 0), (6, 3), (8, 4), (9, 2), (11, 0), (12, 1),
+    (13, 2), (14, 0), (16, 0), (17, 0), (17, 1), (18, 2), (19, 0), (20, 1), (17, 3), (7, 7),
 ])
 def test_trees(log_leaves, log_batch):
     r = np.random.default_rng(10 * log_leaves + log_batch)
