@@ -143,15 +143,14 @@ PadSchedule pad_schedule(uint32_t n_elems) {
 // the first 16 rounds from the same words.
 //
 // Measured on B200 against a thread per leaf and 256 leaves per CTA, in us with the launches: 2^8
-// leaves of 64 elements 62 -> 37, 2^10 of 16 37 -> 24, 2^12 of 16 40 -> 29, 2^13 of one 30 -> 26 and
-// of 16 42 -> 33; at 2^14 they meet (32 -> 31, 43 -> 42), where several of these CTAs share an SM and
-// their first warps its scheduler, and above it loses (2^15 33 -> 47).  A compression of the chain
-// takes 1.3 us, 39 cycles a round, of which the 14 instructions of the half-rate pipes are 28.
+// leaves of 64 elements 62 -> 29, 2^10 of 16 37 -> 20, 2^12 of 16 40 -> 24, 2^13 of 16 42 -> 28; at
+// 2^14 they meet, where several of these CTAs share an SM and their first warps its scheduler, and
+// above it loses (2^15 of one element 33 -> 47).  A compression of the chain takes 1.0 us.
 constexpr uint32_t kChainMaxLog = 13;
 constexpr uint32_t kChainLog = 5;  // a CTA's nodes
 constexpr uint32_t kChainThreads = 128;
 struct ChainShared {
-  uint32_t kw[3][64][32];  // K[t] + W[t] of block b mod 3, a column a lane
+  uint4 kw[3][16][32];  // K[t] + W[t] of block b mod 3, four words to a lane's element
   uint4 digests[2][32][2];
 };
 // Named barriers of warp 0 and a buffer's warp: words 16 c .. written (c < 4; c = 0 of a layer: its
@@ -164,36 +163,6 @@ __device__ __forceinline__ void chain_arrive(uint32_t id) {
 }
 __device__ __forceinline__ void chain_wait(uint32_t id) {
   asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
-}
-
-// Rounds t0 .. t0 + 15 from their words; the eight state words rotate through v.
-__device__ __forceinline__ void chain_rounds(uint32_t (&v)[8], const uint32_t (&k)[16]) {
-  uint32_t a = v[0], b = v[1], c = v[2], d = v[3], e = v[4], f = v[5], g = v[6], h = v[7];
-#pragma unroll
-  for (int t = 0; t < 16; t++) {
-    const uint32_t S1 = rotr32(e, 6) ^ rotr32(e, 11) ^ rotr32(e, 25);
-    const uint32_t ch = (e & f) ^ (~e & g);
-    const uint32_t S0 = rotr32(a, 2) ^ rotr32(a, 13) ^ rotr32(a, 22);
-    const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
-    const uint32_t y = ch + (h + k[t]);
-    const uint32_t ne = (d + y) + S1, na = (y + S1) + (S0 + mj);
-    h = g;
-    g = f;
-    f = e;
-    e = ne;
-    d = c;
-    c = b;
-    b = a;
-    a = na;
-  }
-  v[0] = a;
-  v[1] = b;
-  v[2] = c;
-  v[3] = d;
-  v[4] = e;
-  v[5] = f;
-  v[6] = g;
-  v[7] = h;
 }
 
 // The words of lane's node of a layer above: the digests of nodes 2 lane and 2 lane + 1 below (lanes
@@ -274,7 +243,11 @@ __global__ void __launch_bounds__(kChainThreads)
           continue;  // warp 0 has these words
         }
 #pragma unroll
-        for (int t = 0; t < 16; t++) sh.kw[buf][16 * c + t][lane] = w[t] + kSha256K[16 * c + t];
+        for (int i = 0; i < 4; i++)
+          sh.kw[buf][4 * c + i][lane] = make_uint4(
+              w[4 * i] + kSha256K[16 * c + 4 * i], w[4 * i + 1] + kSha256K[16 * c + 4 * i + 1],
+              w[4 * i + 2] + kSha256K[16 * c + 4 * i + 2],
+              w[4 * i + 3] + kSha256K[16 * c + 4 * i + 3]);
         chain_arrive(chain_bar(buf, c));
       }
     }
@@ -289,25 +262,33 @@ __global__ void __launch_bounds__(kChainThreads)
   }
   for (uint32_t b = 0; b < total; b++, buf = buf == 2 ? 0 : buf + 1) {
     const bool layer = b >= n_blocks;
-    uint32_t k[16];
-    if (layer) {
-      chain_children(sh.digests[(b - n_blocks) & 1], k);
+    uint4 x[4];
+    auto load = [&](uint32_t c) {
+      chain_wait(chain_bar(buf, c));
 #pragma unroll
-      for (int t = 0; t < 16; t++) k[t] += kSha256K[t];
+      for (int i = 0; i < 4; i++) x[i] = sh.kw[buf][4 * c + i][lane];
+    };
+    if (layer) {
+      uint32_t w[16];
+      chain_children(sh.digests[(b - n_blocks) & 1], w);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        x[i] = make_uint4(w[4 * i] + kSha256K[4 * i], w[4 * i + 1] + kSha256K[4 * i + 1],
+                          w[4 * i + 2] + kSha256K[4 * i + 2], w[4 * i + 3] + kSha256K[4 * i + 3]);
 #pragma unroll
       for (int i = 0; i < 8; i++) s[i] = iv.w[i];
+    } else {
+      load(0);
     }
     uint32_t v[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = s[i];
-#pragma unroll 1
-    for (uint32_t c = 0; c < 4; c++) {
-      if (c || !layer) {
-        chain_wait(chain_bar(buf, c));
+    // unrolled, which lets the words' reads in among the rounds before: 1957 cycles a block, a loop of
+    // four steps 2294, of two with the next step's words read ahead 2894
 #pragma unroll
-        for (int t = 0; t < 16; t++) k[t] = sh.kw[buf][16 * c + t][lane];
-      }
-      chain_rounds(v, k);
+    for (uint32_t c = 0; c < 4; c++) {
+      if (c) load(c);
+      sha256_rounds16(v, reinterpret_cast<const uint32_t*>(x));
     }
     if (b + 3 < total) chain_arrive(chain_bar(buf, 4));
 #pragma unroll
