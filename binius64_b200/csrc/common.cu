@@ -117,6 +117,39 @@ thread_local PinnedStage t_stage;
 // synchronise with the device, which would stall every concurrent proof.  Reads that do not fit
 // go straight to pageable memory.
 constexpr size_t kStageBytes = 4u << 20;
+
+// Copies up to kGatherSegments pieces of device memory into the stage, one CTA a piece.  A read of
+// a proof's results is several small pieces (the transcript, its bytes, the challenges, the last
+// values); as copies each takes 6 us of the stream, 3 of them between two copies, and one launch
+// takes about that for all of them.  Measured on B200, copies -> launches: a proof of 2^12 words 1707
+// -> 1614 us, of 2^16 from the host 1325 -> 1277, of 2^20 2640 -> 2581.
+constexpr uint32_t kGatherSegments = 8, kGatherThreads = 256;
+constexpr size_t kGatherBytes = 64u << 10;  // a larger or an odd piece is left to the copy engine
+struct GatherSegment {
+  const uint8_t* src;
+  uint8_t* dst;  // 16-byte aligned
+  uint64_t pitch;
+  uint32_t width, height;
+};
+struct GatherSegments {
+  GatherSegment seg[kGatherSegments];
+};
+template <class T>
+__device__ __forceinline__ void gather_rows(const GatherSegment& g) {
+  const uint32_t w = g.width / sizeof(T), n = w * g.height;
+  for (uint32_t i = threadIdx.x; i < n; i += kGatherThreads)
+    reinterpret_cast<T*>(g.dst)[i] =
+        reinterpret_cast<const T*>(g.src + (uint64_t)(i / w) * g.pitch)[i % w];
+}
+__global__ void __launch_bounds__(kGatherThreads) gather_reads_kernel(GatherSegments a) {
+  pdl_wait();
+  pdl_trigger();
+  const GatherSegment g = a.seg[blockIdx.x];
+  if (((uint64_t)(uintptr_t)g.src | g.pitch | g.width) % 16 == 0)
+    gather_rows<uint4>(g);
+  else
+    gather_rows<uint32_t>(g);
+}
 }  // namespace
 
 StagedReads::StagedReads(cudaStream_t s) : s_(s) {}
@@ -134,41 +167,66 @@ int StagedReads::reserve(size_t bytes, uint8_t** at) {
 }
 
 int StagedReads::add(void* dst, const void* src, size_t bytes) {
-  uint8_t* at = nullptr;
-  if (int rc = reserve(bytes, &at)) return rc;
-  if (!at) {  // larger than the stage: a pageable copy, complete when the call returns
-    BGPU_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s_));
-    return BINIUS_OK;
-  }
-  BGPU_CUDA(cudaMemcpyAsync(at, src, bytes, cudaMemcpyDeviceToHost, s_));
-  pending_.push_back({dst, at, bytes, 0, 0, 0});
-  return BINIUS_OK;
+  return add2d(dst, bytes, src, bytes, bytes, 1);
 }
 
 int StagedReads::add2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width,
                        size_t height) {
+  if (width * height == 0) return BINIUS_OK;
   uint8_t* at = nullptr;
   if (int rc = reserve(width * height, &at)) return rc;
-  if (!at) {
-    BGPU_CUDA(cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, height, cudaMemcpyDeviceToHost,
-                                s_));
-    return BINIUS_OK;
+  Pending p{dst, at, src, dpitch, spitch, width, height};
+  if (!at) {  // larger than the stage: a pageable copy, complete when the call returns
+    p.stage = static_cast<uint8_t*>(dst);
+    return copy(p, dpitch);
   }
-  BGPU_CUDA(cudaMemcpy2DAsync(at, width, src, spitch, width, height, cudaMemcpyDeviceToHost, s_));
-  pending_.push_back({dst, at, width, dpitch, width, height});
+  pending_.push_back(p);
   return BINIUS_OK;
 }
 
-int StagedReads::wait() {
-  BGPU_CUDA(stream_wait(s_));
+int StagedReads::copy(const Pending& p, size_t dpitch) {
+  if (p.height == 1)
+    BGPU_CUDA(cudaMemcpyAsync(p.stage, p.src, p.width, cudaMemcpyDeviceToHost, s_));
+  else
+    BGPU_CUDA(cudaMemcpy2DAsync(p.stage, dpitch, p.src, p.spitch, p.width, p.height,
+                                cudaMemcpyDeviceToHost, s_));
+  return BINIUS_OK;
+}
+
+// Queues the reads: small pieces in launches of kGatherSegments, a large or a lone one as a copy.
+int StagedReads::queue() {
+  GatherSegments g;
+  uint32_t n = 0;
+  const Pending* lone = nullptr;
+  auto launch = [&]() -> int {
+    if (n == 1) return copy(*lone, lone->width);
+    BGPU_CUDA(launch_pdl(gather_reads_kernel, n, kGatherThreads, 0, s_, g));
+    count_launch();
+    return BINIUS_OK;
+  };
   for (const auto& p : pending_) {
-    if (p.height == 0) {
-      memcpy(p.dst, p.stage, p.bytes);
-    } else {
-      for (size_t r = 0; r < p.height; r++)
-        memcpy(static_cast<uint8_t*>(p.dst) + r * p.dpitch, p.stage + r * p.width, p.width);
+    if (p.width * p.height > kGatherBytes ||
+        ((uint64_t)(uintptr_t)p.src | p.spitch | p.width) % 4 != 0) {
+      if (int rc = copy(p, p.width)) return rc;
+      continue;
+    }
+    lone = &p;
+    g.seg[n++] = {static_cast<const uint8_t*>(p.src), p.stage, p.height == 1 ? 0 : p.spitch,
+                  (uint32_t)p.width, (uint32_t)p.height};
+    if (n == kGatherSegments) {
+      if (int rc = launch()) return rc;
+      n = 0;
     }
   }
+  return n ? launch() : BINIUS_OK;
+}
+
+int StagedReads::wait() {
+  if (int rc = queue()) return rc;
+  BGPU_CUDA(stream_wait(s_));
+  for (const auto& p : pending_)
+    for (size_t r = 0; r < p.height; r++)
+      memcpy(static_cast<uint8_t*>(p.dst) + r * p.dpitch, p.stage + r * p.width, p.width);
   pending_.clear();
   used_ = 0;
   return BINIUS_OK;

@@ -42,9 +42,9 @@ cudaError_t stream_mark(cudaStream_t s);
 cudaError_t mark_wait();
 void set_blocking_waits(bool on, double poll_micros = 100.0);
 
-// Device-to-host reads through a per-thread pinned staging buffer: add() queues copies on the
-// stream, wait() synchronises once and scatters them to their destinations.  Small reads from
-// pinned memory are truly asynchronous, unlike copies into pageable memory.
+// Device-to-host reads through a per-thread pinned staging buffer: add() notes them, wait() queues
+// them on the stream (small ones together as one launch, which writes the stage), synchronises once
+// and scatters them to their destinations.  The sources stay as they are from add() to wait().
 class StagedReads {
  public:
   explicit StagedReads(cudaStream_t s);
@@ -60,9 +60,12 @@ class StagedReads {
   struct Pending {
     void* dst;
     uint8_t* stage;
-    size_t bytes, dpitch, width, height;
+    const void* src;
+    size_t dpitch, spitch, width, height;
   };
   int reserve(size_t bytes, uint8_t** at);
+  int copy(const Pending& p, size_t dpitch);
+  int queue();
   cudaStream_t s_;
   size_t used_ = 0;
   std::vector<Pending> pending_;
