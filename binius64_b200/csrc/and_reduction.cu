@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(kUniThreads, 1)
                             const uint64_t* __restrict__ wc, const uint4* __restrict__ eq_big,
                             uint64_t n_chunks, DevAndTables tab, PhiPowers phi,
                             uint32_t* __restrict__ out) {
+  pdl_wait();
   extern __shared__ uint4 smem4[];
   uint32_t* sT = reinterpret_cast<uint32_t*>(smem4);
   const uint2* sT2 = reinterpret_cast<const uint2*>(sT);
@@ -296,6 +297,7 @@ struct Lag64 {
 __global__ void __launch_bounds__(256)
     fold_words_kernel(const uint64_t* __restrict__ words, uint64_t n, Lag64 lag,
                       uint4* __restrict__ out) {
+  pdl_wait();
   __shared__ uint4 tab[8][256];
   for (uint32_t i = threadIdx.x; i < 8 * 256; i += blockDim.x) {
     const uint32_t bi = i >> 8, bv = i & 255;
@@ -358,6 +360,7 @@ __global__ void __launch_bounds__(256)
     and_mle_eval_kernel(const uint4* __restrict__ fa, const uint4* __restrict__ fb,
                         const uint4* __restrict__ fc, const uint4* __restrict__ eq, uint64_t half,
                         uint32_t* __restrict__ out) {
+  pdl_wait();
   u256 s1 = {0, 0, 0, 0}, sinf = {0, 0, 0, 0};
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < half;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -637,7 +640,8 @@ hu128 phi_elem(uint32_t b) { return and_constants().phi[b & 255]; }
 int and_mle_eval(const uint4* d_a, const uint4* d_b, const uint4* d_c, const uint4* d_eq,
                  uint64_t half, uint32_t* d_out8, cudaStream_t s) {
   BGPU_CUDA(cudaMemsetAsync(d_out8, 0, 32, s));
-  and_mle_eval_kernel<<<grid_for(half, 256), 256, 0, s>>>(d_a, d_b, d_c, d_eq, half, d_out8);
+  launch_pdl(and_mle_eval_kernel, grid_for(half, 256), 256, 0, s, d_a, d_b, d_c, d_eq, half,
+             d_out8);
   BGPU_LAUNCH_CHECK("and_mle_eval_kernel");
   count_launch();
   return BINIUS_OK;
@@ -648,7 +652,7 @@ int fold_words64(const uint64_t* d_words, uint64_t n, const hu128* vec64, uint4*
   if (n == 0) return BINIUS_OK;
   Lag64 l64;
   for (int i = 0; i < 64; i++) l64.l[i] = to_uint4(vec64[i]);
-  fold_words_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_words, n, l64, d_out);
+  launch_pdl(fold_words_kernel, grid_for(n, 256), 256, 0, s, d_words, n, l64, d_out);
   BGPU_LAUNCH_CHECK("fold_words_kernel");
   count_launch();
   return BINIUS_OK;
@@ -724,8 +728,8 @@ int and_reduction_finish(const binius_cs* cs, AndPrep& p, Transcript& t, AndResu
     for (int i = 0; i < 8; i++) pw.p[i] = to_uint4(C.phi[1u << i]);
     cudaError_t e = cudaMemsetAsync(d_acc, 0, 16 * (64 + 2 * (log_n + 1)), s);
     if (e != cudaSuccess) { rc = cuda_error(e, "memset"); break; }
-    univariate_round_kernel<<<148, kUniThreads, kUniSmem, s>>>(words, words + N, words + 2 * N,
-                                                              eq_big, n_chunks, tab, pw, d_acc);
+    launch_pdl(univariate_round_kernel, 148, kUniThreads, kUniSmem, s, words, words + N,
+               words + 2 * N, eq_big, n_chunks, tab, pw, d_acc);
     e = cudaGetLastError();
     if (e != cudaSuccess) { rc = cuda_error(e, "univariate_round_kernel"); break; }
     count_launch();
@@ -741,7 +745,7 @@ int and_reduction_finish(const binius_cs* cs, AndPrep& p, Transcript& t, AndResu
     lagrange_b128(6, z, lag);
     Lag64 l64;
     for (int i = 0; i < 64; i++) l64.l[i] = to_uint4(lag[i]);
-    fold_words_kernel<<<grid_for(3 * N, 256), 256, 0, s>>>(words, 3 * N, l64, fcols);
+    launch_pdl(fold_words_kernel, grid_for(3 * N, 256), 256, 0, s, words, 3 * N, l64, fcols);
     e = cudaGetLastError();
     if (e != cudaSuccess) { rc = cuda_error(e, "fold_words_kernel"); break; }
     count_launch();
@@ -787,8 +791,8 @@ int and_reduction_finish(const binius_cs* cs, AndPrep& p, Transcript& t, AndResu
       uint32_t* acc = d_acc + 4 * (64 + 2 * k);
       const uint64_t size = 1ull << n_rem;
       if (n_rem == log_n) {
-        and_mle_eval_kernel<<<grid_for(size / 2, 256), 256, 0, s>>>(fa, fb, fc, eq, size / 2,
-                                                                    acc);
+        launch_pdl(and_mle_eval_kernel, grid_for(size / 2, 256), 256, 0, s, fa, fb, fc, eq,
+                   size / 2, acc);
         e = cudaGetLastError();
       } else if (size * 2 >= kMulTableMinSize) {
         // two lanes per folded position (size of them)

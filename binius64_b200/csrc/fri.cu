@@ -17,6 +17,7 @@
 #include "gf_reduce.cuh"
 #include "gf_tc.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 #include "kernels.h"
 
 using namespace bgpu;
@@ -56,6 +57,7 @@ unsigned grid_for(uint64_t n, unsigned threads) {
 __global__ void __launch_bounds__(256)
     fold_interleaved_kernel(const uint4* __restrict__ cw, uint32_t log_len, uint32_t log_batch,
                             Challenges ch, const uint4* __restrict__ dch, uint4* __restrict__ out) {
+  pdl_wait();
   __shared__ uint4 tensor[1u << kMaxChallenges];
   const uint32_t batch = 1u << log_batch;
   // eq_ind(r)[j] = prod_i (bit_i(j) ? r_i : 1 + r_i)  (multilinear/eq.rs:39-71)
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
     fold_interleaved_tc_kernel(const uint4* __restrict__ cw, uint32_t log_len, uint32_t log_batch,
                                Challenges ch, const uint4* __restrict__ dch,
                                uint4* __restrict__ out) {
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t fold_smem[];
   FoldTcShared& sh = *reinterpret_cast<FoldTcShared*>(fold_smem);
   const uint32_t group = tc::uniform(threadIdx.x / tc::kGroupThreads);
@@ -222,6 +225,7 @@ __global__ void __launch_bounds__(256)
     fold_codeword_kernel(const uint4* __restrict__ cw, uint32_t log_len,
                          const uint4* __restrict__ tw, ScaledFold sf, Challenges ch,
                          const uint4* __restrict__ dch, uint4* __restrict__ out) {
+  pdl_wait();
   const uint64_t n_chunks = 1ull << (log_len - N);
   uint4 rr[N];
 #pragma unroll
@@ -272,6 +276,7 @@ __global__ void __launch_bounds__(256)
     fold_codeword_lanes_kernel(const uint4* __restrict__ cw, uint32_t log_len,
                                const uint4* __restrict__ tw, ScaledFold sf, Challenges ch,
                                const uint4* __restrict__ dch, uint4* __restrict__ out) {
+  pdl_wait();
   constexpr uint32_t P = 1u << (N - 1);
   const uint64_t n_chunks = 1ull << (log_len - N);
   const uint32_t q = threadIdx.x & (P - 1);
@@ -367,11 +372,11 @@ void launch_fold_codeword_as(const uint4* cw, uint32_t log_len, const uint4* tw,
                              uint4* out, cudaStream_t s) {
   uint64_t n_chunks = 1ull << (log_len - N);
   if (n_chunks < kCompactFoldChunks)
-    fold_codeword_lanes_kernel<N, SCALED><<<grid_for(n_chunks << (N - 1), 256), 256, 0, s>>>(
-        cw, log_len, tw, sf, ch, dch, out);
+    launch_pdl(fold_codeword_lanes_kernel<N, SCALED>, grid_for(n_chunks << (N - 1), 256), 256, 0, s,
+               cw, log_len, tw, sf, ch, dch, out);
   else
-    fold_codeword_kernel<N, SCALED><<<grid_for(n_chunks, 256), 256, 0, s>>>(cw, log_len, tw, sf,
-                                                                            ch, dch, out);
+    launch_pdl(fold_codeword_kernel<N, SCALED>, grid_for(n_chunks, 256), 256, 0, s, cw, log_len, tw,
+               sf, ch, dch, out);
 }
 
 template <int N>
@@ -390,15 +395,14 @@ int launch_fold_interleaved(const void* d_codeword, uint32_t log_len, uint32_t l
     const void* kern = reinterpret_cast<const void*>(fold_interleaved_tc_kernel);
     if (int rc = ensure_smem_limit(kern, sizeof(FoldTcShared))) return rc;
     const uint64_t ctas = ((1ull << (log_len - 7)) + kFoldGroups - 1) / kFoldGroups;
-    fold_interleaved_tc_kernel<<<(unsigned)std::min<uint64_t>(ctas, 148), kFoldThreads,
-                                 sizeof(FoldTcShared), s>>>(
-        static_cast<const uint4*>(d_codeword), log_len, log_batch, ch, dch,
-        static_cast<uint4*>(d_out));
+    launch_pdl(fold_interleaved_tc_kernel, (unsigned)std::min<uint64_t>(ctas, 148), kFoldThreads,
+               sizeof(FoldTcShared), s, static_cast<const uint4*>(d_codeword), log_len, log_batch,
+               ch, dch, static_cast<uint4*>(d_out));
     BGPU_LAUNCH_CHECK("fold_interleaved_tc_kernel");
   } else {
-    fold_interleaved_kernel<<<grid_for(1ull << log_len, 256), 256, 0, s>>>(
-        static_cast<const uint4*>(d_codeword), log_len, log_batch, ch, dch,
-        static_cast<uint4*>(d_out));
+    launch_pdl(fold_interleaved_kernel, grid_for(1ull << log_len, 256), 256, 0, s,
+               static_cast<const uint4*>(d_codeword), log_len, log_batch, ch, dch,
+               static_cast<uint4*>(d_out));
     BGPU_LAUNCH_CHECK("fold_interleaved_kernel");
   }
   count_launch();

@@ -61,6 +61,8 @@ unsigned blocks_for(uint64_t n, unsigned cap = 148 * 4) {
 // out[(i) * stride + x] = bit_i(e[x]) ? pw[i] : 1 for i < 64.
 __global__ void const_leaves_kernel(const uint64_t* __restrict__ e, uint64_t n, Pow64 pw,
                                     uint4* __restrict__ out, uint64_t stride) {
+  pdl_wait();
+  pdl_trigger();
   for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < n;
        x += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t w = e[x];
@@ -73,6 +75,8 @@ __global__ void const_leaves_kernel(const uint64_t* __restrict__ e, uint64_t n, 
 __global__ void var_leaves_kernel(const uint64_t* __restrict__ e, uint64_t n,
                                   const uint4* __restrict__ base, uint4* __restrict__ out,
                                   uint64_t stride) {
+  pdl_wait();
+  pdl_trigger();
   for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < n;
        x += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t w = e[x];
@@ -87,6 +91,8 @@ __global__ void var_leaves_kernel(const uint64_t* __restrict__ e, uint64_t n,
 // parent[q] = child[2q] * child[2q + 1] for q < count.
 __global__ void tree_layer_kernel(const uint4* __restrict__ child, uint4* __restrict__ parent,
                                   uint32_t count, uint64_t n, uint64_t stride) {
+  pdl_wait();
+  pdl_trigger();
   const uint64_t total = (uint64_t)count * n;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -98,6 +104,8 @@ __global__ void tree_layer_kernel(const uint4* __restrict__ child, uint4* __rest
 // out[k * stride + x] = bit (k + first) of e[x] as 0 / 1 for k < count.
 __global__ void bit_columns_kernel(const uint64_t* __restrict__ e, uint64_t n, uint32_t first,
                                    uint32_t count, uint4* __restrict__ out, uint64_t stride) {
+  pdl_wait();
+  pdl_trigger();
   const uint64_t total = (uint64_t)count * n;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -319,6 +327,8 @@ __global__ void fold_set_kernel(uint4* __restrict__ set, uint32_t count, uint64_
 // out[k * stride + (2^m' - 1) + i] = prod_{j < m'} (bit_j(i) ? p_kj : 1 + p_kj).
 __global__ void eq_levels_kernel(const uint4* __restrict__ points, uint32_t count, uint32_t m,
                                  uint4* __restrict__ out, uint64_t stride) {
+  pdl_wait();
+  pdl_trigger();
   const uint64_t per = (2ull << m) - 1, total = (uint64_t)count * per;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -347,6 +357,8 @@ __global__ void eq_levels_kernel(const uint4* __restrict__ points, uint32_t coun
 __global__ void __launch_bounds__(kT)
     dot_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
                const uint4* __restrict__ eq, uint64_t n, uint32_t* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   u256 s = {0, 0, 0, 0};
   for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < n;
        x += (uint64_t)gridDim.x * blockDim.x) {
@@ -482,6 +494,8 @@ constexpr size_t kLayerTape = (sizeof(LayerResult) + 15) & ~size_t(15);
 // eq tensor levels 0 .. n - 1 of the layer's point (as eq_levels_kernel), and the layer's state.
 __global__ void __launch_bounds__(kT)
     intmul_layer_begin_kernel(LayerArgs a, LayerState* __restrict__ st, uint4* __restrict__ eq) {
+  pdl_wait();
+  pdl_trigger();
   const uint64_t total = (1ull << a.n) - 1;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -1040,7 +1054,8 @@ class IntMulDevice {
       if (int rc = alloc(&d_pts, h.size())) return rc;
       BGPU_CUDA(cudaMemcpyAsync(d_pts, h.data(), 16 * h.size(), cudaMemcpyHostToDevice, s_));
     }
-    eq_levels_kernel<<<blocks_for((uint64_t)count << (m + 1)), kT, 0, s_>>>(d_pts, count, m, out, N_);
+    launch_pdl(eq_levels_kernel, blocks_for((uint64_t)count << (m + 1)), kT, 0, s_, d_pts, count, m,
+               out, N_);
     return check("eq_levels_kernel");
   }
   static const uint4* level(const uint4* eqs, uint32_t lvl) { return eqs + ((1ull << lvl) - 1); }
@@ -1111,7 +1126,7 @@ int IntMulDevice::layer(uint4* set, uint32_t pairs, std::vector<hu128>& point,
     uint4* mem = nullptr;
     if (int rc = alloc(&mem, (sizeof(LayerState) + 15) / 16)) return rc;
     ls = reinterpret_cast<LayerState*>(mem);
-    intmul_layer_begin_kernel<<<blocks_for(1ull << n), kT, 0, s_>>>(a, ls, eq_);
+    launch_pdl(intmul_layer_begin_kernel, blocks_for(1ull << n), kT, 0, s_, a, ls, eq_);
     if (int rc = check("intmul_layer_begin_kernel")) return rc;
     for (uint32_t t = 0; t < t0; t++) {
       if (int rc = biv_round(set, pairs, 1ull << (n - t), level(eq_, n - t - 1),
@@ -1182,15 +1197,15 @@ int IntMulDevice::run_single(uint4* acl, uint4* btree, uint4* bcols, uint4* lo0,
                              const uint64_t* d_a, const uint64_t* d_b, const uint64_t* d_lo,
                              IntMulResult& res) {
   constexpr int kAcl = 3 * 127 + 2, kB = 127;
-  bit_columns_kernel<<<1, kT, 0, s_>>>(d_b, 1, 0, 64, bcols, 1);
-  bit_columns_kernel<<<1, kT, 0, s_>>>(d_a, 1, 0, 1, acl + 3 * 127, 1);
-  bit_columns_kernel<<<1, kT, 0, s_>>>(d_b, 1, 0, 1, acl + 3 * 127 + 1, 1);
-  bit_columns_kernel<<<1, kT, 0, s_>>>(d_lo, 1, 0, 1, lo0, 1);
+  launch_pdl(bit_columns_kernel, 1, kT, 0, s_, d_b, 1, 0, 64, bcols, 1);
+  launch_pdl(bit_columns_kernel, 1, kT, 0, s_, d_a, 1, 0, 1, acl + 3 * 127, 1);
+  launch_pdl(bit_columns_kernel, 1, kT, 0, s_, d_b, 1, 0, 1, acl + 3 * 127 + 1, 1);
+  launch_pdl(bit_columns_kernel, 1, kT, 0, s_, d_lo, 1, 0, 1, lo0, 1);
   if (int rc = check("bit_columns_kernel", 4)) return rc;
   // c_root = c_lo_root * c_hi_root (acl nodes 1 and 2), through the dot kernel with eq = [1]
   if (int rc = eq_single({}, 0, eq_)) return rc;
   BGPU_CUDA(cudaMemsetAsync(acc_, 0, 16, s_));
-  dot_kernel<<<1, kT, 0, s_>>>(acl + 1, acl + 2, eq_, 1, acc_);
+  launch_pdl(dot_kernel, 1, kT, 0, s_, acl + 1, acl + 2, eq_, 1, acc_);
   if (int rc = check("dot_kernel")) return rc;
   std::vector<hu128> hacl(kAcl), hb(kB), hcols(64);
   hu128 c_root = 0, lo_bit = 0;
@@ -1235,18 +1250,21 @@ int IntMulDevice::run(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* 
     Pow64 pw;
     hu128 b = bases[t];
     for (int i = 0; i < 64; i++, b = host_gf_mul(b, b)) pw.p[i] = u4(b);
-    const_leaves_kernel<<<blocks_for(N), kT, 0, s_>>>(exps[t], N, pw, acl_layer(6) + 64 * t * N, N);
+    launch_pdl(const_leaves_kernel, blocks_for(N), kT, 0, s_, exps[t], N, pw,
+               acl_layer(6) + 64 * t * N, N);
     if (int rc = check("const_leaves_kernel")) return rc;
   }
   for (int k = 5; k >= 0; k--) {
     const uint32_t count = 3u << k;
-    tree_layer_kernel<<<blocks_for(count * N), kT, 0, s_>>>(acl_layer(k + 1), acl_layer(k), count, N, N);
+    launch_pdl(tree_layer_kernel, blocks_for(count * N), kT, 0, s_, acl_layer(k + 1), acl_layer(k),
+               count, N, N);
     if (int rc = check("tree_layer_kernel")) return rc;
   }
-  var_leaves_kernel<<<blocks_for(N), kT, 0, s_>>>(d_b, N, acl_layer(0), b_layer(6), N);
+  launch_pdl(var_leaves_kernel, blocks_for(N), kT, 0, s_, d_b, N, acl_layer(0), b_layer(6), N);
   if (int rc = check("var_leaves_kernel")) return rc;
   for (int k = 5; k >= 0; k--) {
-    tree_layer_kernel<<<blocks_for((1u << k) * N), kT, 0, s_>>>(b_layer(k + 1), b_layer(k), 1u << k, N, N);
+    launch_pdl(tree_layer_kernel, blocks_for((1u << k) * N), kT, 0, s_, b_layer(k + 1), b_layer(k),
+               1u << k, N, N);
     if (int rc = check("tree_layer_kernel")) return rc;
   }
 
@@ -1257,8 +1275,9 @@ int IntMulDevice::run(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* 
   for (auto& v : point0) v = sample(t_);
   if (int rc = eq_single(point0, n_, eq_)) return rc;
   BGPU_CUDA(cudaMemsetAsync(acc, 0, 32, s_));
-  dot_kernel<<<blocks_for(N), kT, 0, s_>>>(b_layer(0), nullptr, eq_, N, acc);
-  dot_kernel<<<blocks_for(N), kT, 0, s_>>>(acl_layer(0) + N, acl_layer(0) + 2 * N, eq_, N, acc + 4);
+  launch_pdl(dot_kernel, blocks_for(N), kT, 0, s_, b_layer(0), nullptr, eq_, N, acc);
+  launch_pdl(dot_kernel, blocks_for(N), kT, 0, s_, acl_layer(0) + N, acl_layer(0) + 2 * N, eq_, N,
+             acc + 4);
   if (int rc = check("dot_kernel", 2)) return rc;
   uint8_t bc[32];
   if (int rc = sync_read(bc, acc, 32)) return rc;
@@ -1291,7 +1310,7 @@ int IntMulDevice::run(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* 
   std::vector<hu128> p3, b_exp_evals;
   hu128 selector_eval, c_lo_root_eval, c_hi_root_eval;
   {
-    bit_columns_kernel<<<blocks_for(64 * N), kT, 0, s_>>>(d_b, N, 0, 64, bcols, N);
+    launch_pdl(bit_columns_kernel, blocks_for(64 * N), kT, 0, s_, d_b, N, 0, 64, bcols, N);
     if (int rc = check("bit_columns_kernel")) return rc;
     std::vector<const std::vector<hu128>*> tw_ptrs;
     for (int i = 0; i < 64; i++) tw_ptrs.push_back(&tw_points[i]);
@@ -1356,14 +1375,14 @@ int IntMulDevice::run(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* 
   // ---- phase 5: the leaf layers with a_0 * b_0 = c_lo_0 and the b rerandomisation
   {
     uint4* leaves = acl_layer(6);
-    bit_columns_kernel<<<blocks_for(N), kT, 0, s_>>>(d_a, N, 0, 1, leaves + 192 * N, N);
-    bit_columns_kernel<<<blocks_for(N), kT, 0, s_>>>(d_b, N, 0, 1, leaves + 193 * N, N);
-    bit_columns_kernel<<<blocks_for(N), kT, 0, s_>>>(d_lo, N, 0, 1, lo0, N);
-    bit_columns_kernel<<<blocks_for(64 * N), kT, 0, s_>>>(d_b, N, 0, 64, bcols, N);
+    launch_pdl(bit_columns_kernel, blocks_for(N), kT, 0, s_, d_a, N, 0, 1, leaves + 192 * N, N);
+    launch_pdl(bit_columns_kernel, blocks_for(N), kT, 0, s_, d_b, N, 0, 1, leaves + 193 * N, N);
+    launch_pdl(bit_columns_kernel, blocks_for(N), kT, 0, s_, d_lo, N, 0, 1, lo0, N);
+    launch_pdl(bit_columns_kernel, blocks_for(64 * N), kT, 0, s_, d_b, N, 0, 64, bcols, N);
     if (int rc = check("bit_columns_kernel", 4)) return rc;
     if (int rc = eq_single(pt, n_, eq_)) return rc;
     BGPU_CUDA(cudaMemsetAsync(acc, 0, 16, s_));
-    dot_kernel<<<blocks_for(N), kT, 0, s_>>>(lo0, nullptr, eq_, N, acc);
+    launch_pdl(dot_kernel, blocks_for(N), kT, 0, s_, lo0, nullptr, eq_, N, acc);
     if (int rc = check("dot_kernel")) return rc;
     uint8_t cb[16];
     if (int rc = sync_read(cb, acc, 16)) return rc;

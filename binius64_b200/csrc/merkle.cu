@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(256) merkle_leaves_kernel(const uint4* __restr
                                                             uint4* __restrict__ nodes, uint32_t L,
                                                             uint32_t fused, NodeIV iv,
                                                             PadSchedule pad) {
+  pdl_wait();
   __shared__ uint32_t buf[2][256][9];  // padded rows avoid bank conflicts
   const uint32_t tid = threadIdx.x;
   const uint64_t leaf = (uint64_t)blockIdx.x * blockDim.x + tid;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(256) merkle_leaves_kernel(const uint4* __restr
 __global__ void __launch_bounds__(256) merkle_nodes_kernel(uint4* __restrict__ nodes, uint32_t L,
                                                            uint32_t in_level, uint32_t fused,
                                                            NodeIV iv) {
+  pdl_wait();
   __shared__ uint32_t buf[2][256][9];
   const uint32_t tid = threadIdx.x;
   const uint64_t in_off = layer_offset(L, in_level);
@@ -375,14 +377,16 @@ int merkle_commit(const void* d_elems, uint32_t log_leaves, uint32_t log_batch, 
               : log_batch == 0 ? merkle_leaves_kernel<1>
               : log_batch == 1 ? merkle_leaves_kernel<2>
                                : merkle_leaves_kernel<4>;
-  kern<<<(unsigned)grid, 1u << log_cta, 0, stream>>>(elems, log_batch, nodes, L, level, iv, pad);
+  launch_pdl(kern, (unsigned)grid, 1u << log_cta, 0, stream, elems, log_batch, nodes, L, level, iv,
+             pad);
   BGPU_LAUNCH_CHECK("merkle_leaves_kernel");
   count_launch();
   while (level < L) {
     const uint32_t f = std::min(L - level, node_fuse);
     const uint64_t g = 1ull << (L - level - f);
     const uint32_t fused = layers(L - level, f);
-    merkle_nodes_kernel<<<(unsigned)g, 1u << (f - 1), 0, stream>>>(nodes, L, level, fused, iv);
+    launch_pdl(merkle_nodes_kernel, (unsigned)g, 1u << (f - 1), 0, stream, nodes, L, level, fused,
+               iv);
     BGPU_LAUNCH_CHECK("merkle_nodes_kernel");
     count_launch();
     level += fused;

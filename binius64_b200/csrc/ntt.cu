@@ -18,6 +18,7 @@
 #include "gf128.cuh"
 #include "gf_tc.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 
 using namespace bgpu;
 
@@ -62,6 +63,7 @@ template <bool INVERSE, bool RS>
 __global__ void __launch_bounds__(kNttThreads)
     ntt_pass_kernel(uint4* __restrict__ data, const uint4* __restrict__ src,
                     const uint4* __restrict__ tw, NttPass p) {
+  pdl_wait();
   extern __shared__ uint4 smem[];
   const uint32_t k = p.k, c = p.c;
   const uint32_t tile_elems = 1u << (k + c);
@@ -325,6 +327,7 @@ template <bool INVERSE, bool RS>
 __global__ void __launch_bounds__(kTcThreads, 1)
     ntt_tc_pass_kernel(uint4* __restrict__ data, const uint4* __restrict__ src,
                        const uint4* __restrict__ tw, NttPass p, uint32_t n_tiles) {
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t tc_smem[];
   NttTcShared& sh = *reinterpret_cast<NttTcShared*>(tc_smem);
   const uint32_t k = p.k, c = p.c;
@@ -545,8 +548,8 @@ int launch_tc_pass(const NttPass& p, uint4* data, const uint4* src, const uint4*
   if (int rc = ensure_smem_limit(reinterpret_cast<const void*>(kern), sizeof(NttTcShared))) return rc;
   const uint64_t n_tiles = 1ull << (p.log_d - p.k - p.c);
   if (n_tiles > 0x7fffffffull) return set_error(BINIUS_E_ARG, "ntt: buffer too large");
-  kern<<<(unsigned)std::min<uint64_t>(n_tiles, 148), kTcThreads, sizeof(NttTcShared), stream>>>(
-      data, src, tw, p, (uint32_t)n_tiles);
+  launch_pdl(kern, (unsigned)std::min<uint64_t>(n_tiles, 148), kTcThreads, sizeof(NttTcShared),
+             stream, data, src, tw, p, (uint32_t)n_tiles);
   BGPU_LAUNCH_CHECK("ntt_tc_pass_kernel");
   count_launch();
   return BINIUS_OK;
@@ -564,7 +567,7 @@ int launch_pass(const NttPass& p, uint4* data, const uint4* src, const uint4* tw
   if (int rc = ensure_smem_limit(reinterpret_cast<const void*>(kern), kMaxSmem)) return rc;
   uint64_t n_tiles = 1ull << (p.log_d - p.k - p.c);
   if (n_tiles > 0x7fffffffull) return set_error(BINIUS_E_ARG, "ntt: buffer too large");
-  kern<<<(unsigned)n_tiles, kNttThreads, smem, stream>>>(data, src, tw, p);
+  launch_pdl(kern, (unsigned)n_tiles, kNttThreads, smem, stream, data, src, tw, p);
   BGPU_LAUNCH_CHECK("ntt_pass_kernel");
   count_launch();
   return BINIUS_OK;

@@ -14,6 +14,7 @@
 
 #include "dev_transcript.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 #include "kernels.h"
 #include "transcript.h"
 
@@ -94,6 +95,8 @@ struct QueryLayout {
 // the leaf layer up), so the host appends the buffer as it is.
 __global__ void fri_query_gather_kernel(QueryLayout lay, const uint64_t* __restrict__ idx,
                                         uint32_t n_queries, uint8_t* __restrict__ dst) {
+  pdl_wait();
+  pdl_trigger();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= n_queries) return;
@@ -255,8 +258,8 @@ struct DevFri {
           break;
         }
         const unsigned per_block = 4;  // warps (queries) per CTA
-        fri_query_gather_kernel<<<(P.n_queries + per_block - 1) / per_block, 32 * per_block, 0,
-                                  s>>>(lay, d_idx, P.n_queries, d_dst + off);
+        launch_pdl(fri_query_gather_kernel, (P.n_queries + per_block - 1) / per_block,
+                   32 * per_block, 0, s, lay, d_idx, P.n_queries, d_dst + off);
         if ((e = cudaGetLastError()) != cudaSuccess) {
           rc = cuda_error(e, "fri_query_gather_kernel");
           break;

@@ -1,4 +1,4 @@
-// Programmatic dependent launch for the chains of dependent kernels in the sumcheck round loops.
+// Programmatic dependent launch for the chains of dependent kernels of a proof.
 //
 // A kernel launched through launch_pdl may be scheduled while the previous kernel on its stream is
 // still running, which hides most of the ~3 us gap between dependent launches.  Such a kernel
@@ -7,6 +7,12 @@
 // kernel launched without the attribute it returns at once).  pdl_trigger() lets the next kernel
 // of the stream be launched early; it does not release the next kernel's pdl_wait(), so it may be
 // called anywhere.
+//
+// Kernels that take tens of microseconds on many SMs only wait: their CTAs end at different times,
+// and the next grid's, launched early, would settle on the SMs that are free first.  Measured on
+// B200: a tree's 256 leaf CTAs after a 148-CTA transform pass 56 -> 99 us when the pass triggered.
+// With the rest of a proof's kernels launched so: 2^12 words 1654 -> 1601 us, with multiplications
+// 3662 -> 3603, 2^16 from the host 1298 -> 1279.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kTile)
                    const uint16_t* __restrict__ keys, uint64_t n,
                    const uint64_t* __restrict__ words, const uint4* __restrict__ eq_and,
                    const uint4* __restrict__ eq_mul, uint32_t* __restrict__ g_raw) {
+  pdl_wait();
   __shared__ uint4 s_eq[kTile + kChunks];
   __shared__ uint64_t s_w[kTile + kChunks];
   __shared__ uint32_t s_key[kTile];
@@ -202,6 +203,8 @@ __global__ void __launch_bounds__(kTile)
 // g[(s*64 + j)*8 + v] = sum over classes of lambda_class * g_raw[((v*64 + s)*8 + class)*64 + j].
 __global__ void shift_g_combine_kernel(const uint4* __restrict__ g_raw, ClassPowers pw,
                                        uint4* __restrict__ g) {
+  pdl_wait();
+  pdl_trigger();
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= kFlat) return;
   const uint32_t v = idx & 7, s = (idx >> 3) >> 6, j = (idx >> 3) & 63;
@@ -217,6 +220,8 @@ __global__ void shift_g_combine_kernel(const uint4* __restrict__ g_raw, ClassPow
 
 // build_h_parts (monster.rs:34-104) from l_tilde, interleaved layout.
 __global__ void shift_h_kernel(Lag64 L, uint4* __restrict__ h) {
+  pdl_wait();
+  pdl_trigger();
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= kFlat) return;
   const uint32_t v = idx & 7, s = (idx >> 3) >> 6, j = (idx >> 3) & 63;
@@ -267,6 +272,8 @@ constexpr int kHopsBlocks = 64;
 __global__ void __launch_bounds__(256)
     shift_h_ops_kernel(const uint4* __restrict__ h, const uint4* __restrict__ eq,
                        uint32_t* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ uint4 part[256];
   const uint32_t v = threadIdx.x & 7;
   constexpr uint32_t kSlice = kLen / kHopsBlocks;
@@ -285,6 +292,8 @@ __global__ void __launch_bounds__(256)
 // T[key] = lambda_class * h_op(kind)[v] * eq(r_s)[s] (the monster scalars, monster.rs:168-190).
 __global__ void shift_scalars_kernel(ClassPowers pw, Lag64 eq_rs, const uint4* __restrict__ h_ops,
                                      uint32_t mul_offset, uint4* __restrict__ T) {
+  pdl_wait();
+  pdl_trigger();
   const uint32_t key = blockIdx.x * blockDim.x + threadIdx.x;
   if (key >= kShiftKeys) return;
   const uint32_t cls = key & 7, id = key >> 3, v = id >> 6, s = id & 63;
@@ -308,6 +317,7 @@ __global__ void __launch_bounds__(256)
                          uint64_t n, const uint4* __restrict__ eq_and,
                          const uint4* __restrict__ eq_mul, const uint4* __restrict__ T,
                          uint4* __restrict__ M) {
+  pdl_wait();
   const uint64_t n_chunks = (n + kMonsterChunk - 1) / kMonsterChunk;
   for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n_chunks;
        j += (uint64_t)gridDim.x * blockDim.x) {
@@ -670,11 +680,12 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
   // ---- phase 1: g and h parts
   BGPU_CUDA(cudaMemsetAsync(g_raw, 0, 16ull * kShiftKeys * 64, s));
   if (terms.n) {
-    shift_g_kernel<<<grid_for(terms.n, kTile, 148 * 8), kTile, 0, s>>>(
-        terms.vi, terms.c, terms.key, terms.n, d_witness, eq_and, eq_mul, g_raw);
+    launch_pdl(shift_g_kernel, grid_for(terms.n, kTile, 148 * 8), kTile, 0, s, terms.vi, terms.c,
+               terms.key, terms.n, d_witness, eq_and, eq_mul, g_raw);
     SHIFT_TRY(launched("shift_g_kernel"));
   }
-  shift_g_combine_kernel<<<kFlat / 256, 256, 0, s>>>(reinterpret_cast<const uint4*>(g_raw), pw, g);
+  launch_pdl(shift_g_combine_kernel, kFlat / 256, 256, 0, s, reinterpret_cast<const uint4*>(g_raw),
+             pw, g);
   SHIFT_TRY(launched("shift_g_combine_kernel"));
   const bool same_z = band.r_zhat == bmul.r_zhat;
   for (int kind = 0; kind < (same_z ? 1 : 2); kind++) {
@@ -682,7 +693,7 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
     lagrange_phi(6, kind == 0 ? band.r_zhat : bmul.r_zhat, lt);
     Lag64 L;
     for (int i = 0; i < 64; i++) L.l[i] = u4(lt[i]);
-    shift_h_kernel<<<kFlat / 256, 256, 0, s>>>(L, h_keep + kind * kFlat);
+    launch_pdl(shift_h_kernel, kFlat / 256, 256, 0, s, L, h_keep + kind * kFlat);
     SHIFT_TRY(launched("shift_h_kernel"));
   }
   BGPU_CUDA(cudaMemcpyAsync(h, h_keep, 16ull * kFlat, cudaMemcpyDeviceToDevice, s));
@@ -702,7 +713,7 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
 
   // the provers' claims: sum_v <g_v, h_v> (phase_1.rs:96-101)
   BGPU_CUDA(cudaMemsetAsync(acc + 8, 0, 32, s));
-  dot2_kernel<<<grid_for(kFlat, 256, 148), 256, 0, s>>>(g, 0, 0, h, kFlat, acc + 8);
+  launch_pdl(dot2_kernel, grid_for(kFlat, 256, 148), 256, 0, s, g, 0, 0, h, kFlat, acc + 8);
   SHIFT_TRY(launched("dot2_kernel"));
   DeviceTranscript dt;
   SHIFT_TRY(dt.begin(t, s));
@@ -754,20 +765,20 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
   SHIFT_TRY(eq_tensor(to_u4(rev).data(), 12, eq_rjs, s));
   BGPU_CUDA(cudaMemsetAsync(h_ops, 0, 16 * 16, s));
   for (int kind = 0; kind < (same_z ? 1 : 2); kind++) {
-    shift_h_ops_kernel<<<kHopsBlocks, 256, 0, s>>>(h_keep + kind * kFlat, eq_rjs,
-                                                   reinterpret_cast<uint32_t*>(h_ops + 8 * kind));
+    launch_pdl(shift_h_ops_kernel, kHopsBlocks, 256, 0, s, h_keep + kind * kFlat, eq_rjs,
+               reinterpret_cast<uint32_t*>(h_ops + 8 * kind));
     SHIFT_TRY(launched("shift_h_ops_kernel"));
   }
   Lag64 ers;
   for (int i = 0; i < 64; i++) ers.l[i] = u4(eq_rs[i]);
-  shift_scalars_kernel<<<kShiftKeys / 256, 256, 0, s>>>(pw, ers, h_ops, same_z ? 0 : 8, T);
+  launch_pdl(shift_scalars_kernel, kShiftKeys / 256, 256, 0, s, pw, ers, h_ops, same_z ? 0 : 8, T);
   SHIFT_TRY(launched("shift_scalars_kernel"));
   if (terms.n_words != n_words) return set_error(BINIUS_E_ARG, "shift term table of another size");
   BGPU_CUDA(cudaMemsetAsync(M, 0, 16ull * n_words, s));
   if (terms.n) {
     const uint64_t n_chunks = (terms.n + kMonsterChunk - 1) / kMonsterChunk;
-    shift_monster_kernel<<<grid_for(n_chunks, 256, 148 * 32), 256, 0, s>>>(
-        terms.w_off, terms.w_chunk, terms.w_c, terms.w_key, terms.n, eq_and, eq_mul, T, M);
+    launch_pdl(shift_monster_kernel, grid_for(n_chunks, 256, 148 * 32), 256, 0, s, terms.w_off,
+               terms.w_chunk, terms.w_c, terms.w_key, terms.n, eq_and, eq_mul, T, M);
     SHIFT_TRY(launched("shift_monster_kernel"));
   }
 
@@ -785,7 +796,8 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
       BGPU_CUDA(launch_pdl(dot2_kernel, grid, 256, 0, s, (const uint4*)W, off0, off1,
                            (const uint4*)eq_pub, len, reinterpret_cast<uint32_t*>(out)));
     else
-      dot2_kernel<<<grid, 256, 0, s>>>(W, off0, off1, eq_pub, len, reinterpret_cast<uint32_t*>(out));
+      launch_pdl(dot2_kernel, grid, 256, 0, s, W, off0, off1, eq_pub, len,
+                 reinterpret_cast<uint32_t*>(out));
     SHIFT_TRY(launched("dot2_kernel"));
     return BINIUS_OK;
   };

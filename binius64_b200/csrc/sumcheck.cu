@@ -91,6 +91,7 @@ constexpr int kRowTile = 256;
 __global__ void __launch_bounds__(128)
     fold_rows_kernel(const uint4* __restrict__ mat, const uint4* __restrict__ vec, uint64_t n,
                      uint32_t* __restrict__ out) {
+  pdl_wait();
   __shared__ uint32_t s_mat[kRowTile][4];
   __shared__ uint4 s_vec[kRowTile];
   const uint32_t k = threadIdx.x;  // bit column
@@ -123,6 +124,8 @@ __global__ void __launch_bounds__(128)
 
 // tables[p][b] = sum over the set bits j of b of vec[8p + j].
 __global__ void build_fold_tables_kernel(const uint4* __restrict__ vec, uint4* __restrict__ tables) {
+  pdl_wait();
+  pdl_trigger();
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= 16 * 256) return;
   const uint32_t p = idx >> 8, b = idx & 255;
@@ -140,6 +143,7 @@ __device__ __forceinline__ uint32_t byte_of(uint4 v, uint32_t p) {
 __global__ void __launch_bounds__(kThreads)
     fold_elems_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, uint64_t n,
                       const uint4* __restrict__ tables) {
+  pdl_wait();
   extern __shared__ uint4 s_tab[];  // 16 x 256
   for (uint32_t i = threadIdx.x; i < 16 * 256; i += blockDim.x) s_tab[i] = tables[i];
   __syncthreads();
@@ -157,6 +161,7 @@ __global__ void __launch_bounds__(kThreads)
 __global__ void __launch_bounds__(kThreads)
     bivariate_eval_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, uint64_t half,
                           uint32_t* __restrict__ out) {
+  pdl_wait();
   u256 s1 = {0, 0, 0, 0}, sinf = {0, 0, 0, 0};
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < half;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -400,7 +405,7 @@ int fold_1b_rows(const uint4* d_mat, const uint4* d_vec, uint64_t n, uint32_t* d
   BGPU_CUDA(cudaMemsetAsync(d_out512, 0, 128 * 16, s));
   unsigned blocks = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>((n + kRowTile - 1) / kRowTile, 148 * 4));
-  fold_rows_kernel<<<blocks, 128, 0, s>>>(d_mat, d_vec, n, d_out512);
+  launch_pdl(fold_rows_kernel, blocks, 128, 0, s, d_mat, d_vec, n, d_out512);
   BGPU_LAUNCH_CHECK("fold_rows_kernel");
   count_launch();
   return BINIUS_OK;
@@ -410,13 +415,14 @@ int fold_b128_elems(const uint4* d_in, uint4* d_out, uint64_t n, const uint4* d_
                     cudaStream_t s) {
   uint4* tables = nullptr;
   BGPU_CUDA(dev_alloc(&tables, 16 * 16 * 256, s));
-  build_fold_tables_kernel<<<16, 256, 0, s>>>(d_vec128, tables);
+  launch_pdl(build_fold_tables_kernel, 16, 256, 0, s, d_vec128, tables);
   const size_t smem = 16 * 256 * sizeof(uint4);
   cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(fold_elems_kernel), smem)
                       ? cudaErrorInvalidValue
                       : cudaSuccess;
   if (e == cudaSuccess) {
-    fold_elems_kernel<<<grid_for(n, kThreads, 148 * 2), kThreads, smem, s>>>(d_in, d_out, n, tables);
+    launch_pdl(fold_elems_kernel, grid_for(n, kThreads, 148 * 2), kThreads, smem, s, d_in, d_out, n,
+               tables);
     e = cudaGetLastError();
   }
   dev_free(tables, s);
@@ -428,7 +434,8 @@ int fold_b128_elems(const uint4* d_in, uint4* d_out, uint64_t n, const uint4* d_
 int bivariate_eval(const uint4* d_a, const uint4* d_b, uint64_t half, uint32_t* d_out8,
                    cudaStream_t s) {
   BGPU_CUDA(cudaMemsetAsync(d_out8, 0, 32, s));
-  bivariate_eval_kernel<<<grid_for(half, kThreads), kThreads, 0, s>>>(d_a, d_b, half, d_out8);
+  launch_pdl(bivariate_eval_kernel, grid_for(half, kThreads), kThreads, 0, s, d_a, d_b, half,
+             d_out8);
   BGPU_LAUNCH_CHECK("bivariate_eval_kernel");
   count_launch();
   return BINIUS_OK;
@@ -442,13 +449,14 @@ int bivariate_fold_eval(uint4* d_a, uint4* d_b, uint64_t size, const uint8_t r[1
   BGPU_CUDA(cudaMemsetAsync(d_out8, 0, 32, s));
   const unsigned grid = grid_for(size / 2, kThreads);  // two lanes per folded position
   if (size >= kMulTableMinSize) {
-    bivariate_fold_eval_kernel<<<grid, kThreads, 0, s>>>(d_a, d_b, size, rv, nullptr, d_out8);
+    launch_pdl(bivariate_fold_eval_kernel, grid, kThreads, 0, s, d_a, d_b, size, rv, nullptr,
+               d_out8);
     BGPU_LAUNCH_CHECK("bivariate_fold_eval_kernel");
     count_launch();
     return BINIUS_OK;
   }
-  bivariate_fold_eval_lanes_kernel<<<grid_for(size, kThreads), kThreads, 0, s>>>(
-      d_a, d_b, size, rv, nullptr, d_out8);
+  launch_pdl(bivariate_fold_eval_lanes_kernel, grid_for(size, kThreads), kThreads, 0, s, d_a, d_b,
+             size, rv, nullptr, d_out8);
   BGPU_LAUNCH_CHECK("bivariate_fold_eval_lanes_kernel");
   count_launch();
   return BINIUS_OK;

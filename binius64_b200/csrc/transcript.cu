@@ -5,6 +5,7 @@
 
 #include "dev_transcript.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 #include "transcript.h"
 
 using namespace bgpu;
@@ -12,11 +13,15 @@ using namespace bgpu;
 namespace {
 
 __global__ void transcript_load_kernel(TranscriptState st, TranscriptState* dst) {
+  pdl_wait();
+  pdl_trigger();
   if (threadIdx.x == 0 && blockIdx.x == 0) *dst = st;
 }
 
 __global__ void transcript_message_kernel(TranscriptState* ts, uint8_t* tape,
                                           const uint32_t* __restrict__ words, uint32_t n) {
+  pdl_wait();
+  pdl_trigger();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   DevTr st;
   st.load(ts);
@@ -38,7 +43,7 @@ int DeviceTranscript::begin(const Transcript& t, cudaStream_t s) {
   TranscriptState st;
   t.save(st);
   st.tape_cap = kTapeCap;
-  transcript_load_kernel<<<1, 32, 0, s>>>(st, state());
+  launch_pdl(transcript_load_kernel, 1, 32, 0, s, st, state());
   BGPU_LAUNCH_CHECK("transcript_load_kernel");
   count_launch();
   return BINIUS_OK;
@@ -47,8 +52,8 @@ int DeviceTranscript::begin(const Transcript& t, cudaStream_t s) {
 int DeviceTranscript::message_device(const void* d_bytes, uint32_t n_bytes, cudaStream_t s) {
   if (n_bytes % 4 || reinterpret_cast<uintptr_t>(d_bytes) % 4)
     return set_error(BINIUS_E_ARG, "device message: whole aligned words only");
-  transcript_message_kernel<<<1, 32, 0, s>>>(state(), tape(),
-                                             static_cast<const uint32_t*>(d_bytes), n_bytes / 4);
+  launch_pdl(transcript_message_kernel, 1, 32, 0, s, state(), tape(),
+             static_cast<const uint32_t*>(d_bytes), n_bytes / 4);
   BGPU_LAUNCH_CHECK("transcript_message_kernel");
   count_launch();
   return BINIUS_OK;

@@ -31,6 +31,7 @@
 
 #include "gf128.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 #include "kernels.h"
 
 using namespace bgpu;
@@ -573,6 +574,7 @@ __global__ void __launch_bounds__(kGroupLanes << kWarpFuse)
     vision4_leaves_warp_kernel(const uint4* __restrict__ img, const uint4* __restrict__ elems,
                                uint32_t log_batch, uint4* __restrict__ nodes, uint32_t L,
                                uint32_t fused) {
+  pdl_wait();
   v4w_load_image(img);
   const uint32_t group = threadIdx.x / kGroupLanes, e = (threadIdx.x / 32) & 3;
   uint4* mix = v4_img + kWarpImageBytes / 16 + 8 * group;
@@ -609,6 +611,7 @@ __global__ void __launch_bounds__(kGroupLanes << kWarpFuse)
 __global__ void __launch_bounds__(kGroupLanes << kWarpFuse)
     vision4_nodes_warp_kernel(const uint4* __restrict__ img, uint4* __restrict__ nodes, uint32_t L,
                               uint32_t in_level, uint32_t fused) {
+  pdl_wait();
   v4w_load_image(img);
   const uint32_t group = threadIdx.x / kGroupLanes, e = (threadIdx.x / 32) & 3;
   uint4* mix = v4_img + kWarpImageBytes / 16 + 8 * group;
@@ -626,14 +629,14 @@ int vision4_commit_warps(const uint4* elems, uint32_t L, uint32_t log_batch, uin
   if (int rc = ensure_smem_limit((const void*)vision4_nodes_warp_kernel, kWarpSmem)) return rc;
   // one group per CTA, and so one warp per scheduler, while the leaves are fewer than the SMs
   const uint32_t fused = std::min(L > 7 ? L - 7 : 0, kWarpFuse);
-  vision4_leaves_warp_kernel<<<1u << (L - fused), kGroupLanes << fused, kWarpSmem, s>>>(
-      img, elems, log_batch, nodes, L, fused);
+  launch_pdl(vision4_leaves_warp_kernel, 1u << (L - fused), kGroupLanes << fused, kWarpSmem, s, img,
+             elems, log_batch, nodes, L, fused);
   BGPU_LAUNCH_CHECK("vision4_leaves_warp_kernel");
   count_launch();
   for (uint32_t level = fused; level < L;) {
     const uint32_t f = std::min(L - level, kWarpFuse);
-    vision4_nodes_warp_kernel<<<1u << (L - level - f), kGroupLanes << (f - 1), kWarpSmem, s>>>(
-        img, nodes, L, level, f);
+    launch_pdl(vision4_nodes_warp_kernel, 1u << (L - level - f), kGroupLanes << (f - 1), kWarpSmem,
+               s, img, nodes, L, level, f);
     BGPU_LAUNCH_CHECK("vision4_nodes_warp_kernel");
     count_launch();
     level += f;
