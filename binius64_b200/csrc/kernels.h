@@ -21,9 +21,10 @@ int fold_1b_rows(const uint4* d_mat, const uint4* d_vec, uint64_t n, uint32_t* d
 // d_out[i] = sum_k bit_k(d_in[i]) * d_vec128[k]  (d_out may equal d_in).
 int fold_b128_elems(const uint4* d_in, uint4* d_out, uint64_t n, const uint4* d_vec128,
                     cudaStream_t s);
-// d_out8 = (y_1, y_inf) of the bivariate product round on (a, b) of length 2*half.
+// d_out8 = (y_1, y_inf) of the bivariate product round on (a, b) of length 2*half; clear = false:
+// d_out8 is zero already.
 int bivariate_eval(const uint4* d_a, const uint4* d_b, uint64_t half, uint32_t* d_out8,
-                   cudaStream_t s);
+                   cudaStream_t s, bool clear = true);
 // Fold (a, b) of length size by r, then (y_1, y_inf) of the next round.
 int bivariate_fold_eval(uint4* d_a, uint4* d_b, uint64_t size, const uint8_t r[16],
                         uint32_t* d_out8, cudaStream_t s);

@@ -370,7 +370,7 @@ int pcs_prove_impl(const binius_pcs* P, const binius_pcs_committed* C, const voi
         const uint64_t size = N >> round;
         uint32_t* ys = reinterpret_cast<uint32_t*>(slots + 2 * round);
         if (round == 0)
-          rc = bivariate_eval(a, b, size / 2, ys, s);
+          rc = bivariate_eval(a, b, size / 2, ys, s, false);
         else
           rc = bivariate_fold_eval_dev(a, b, size * 2, chal + round - 1, ys, s);
         if (rc) break;

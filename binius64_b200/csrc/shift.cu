@@ -219,7 +219,7 @@ __global__ void shift_g_combine_kernel(const uint4* __restrict__ g_raw, ClassPow
 }
 
 // build_h_parts (monster.rs:34-104) from l_tilde, interleaved layout.
-__global__ void shift_h_kernel(Lag64 L, uint4* __restrict__ h) {
+__global__ void shift_h_kernel(Lag64 L, uint4* __restrict__ h, uint4* __restrict__ h2) {
   pdl_wait();
   pdl_trigger();
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,6 +263,7 @@ __global__ void shift_h_kernel(Lag64 L, uint4* __restrict__ h) {
     }
   }
   h[idx] = val;
+  if (h2) h2[idx] = val;
 }
 
 // out[v] += <h_v, eq(r_j ++ r_s)> for the 8 variants (evaluate_h_op); out zeroed by the caller.
@@ -648,21 +649,30 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
   const ShiftTerms& terms = cs->shift_terms;
 
   ShiftBuffers B(s);
-  uint4 *eq_and, *eq_mul, *g, *h, *h_keep, *eq_rjs, *h_ops, *T, *W, *M, *eq_pub;
-  uint32_t *g_raw, *acc;
+  uint4 *eq_and, *eq_mul, *g, *h, *h_keep, *eq_rjs, *T, *W, *M, *eq_pub;
+  uint4 *zeroed;
   SHIFT_TRY(B.alloc(&eq_and, 16ull << log_and));
   SHIFT_TRY(B.alloc(&eq_mul, 16ull << log_mul));
-  SHIFT_TRY(B.alloc(&g_raw, 16ull * kShiftKeys * 64));
+  // what starts at zero, cleared together: the sums of shift_g_kernel, of phase 1's rounds (12 x 2)
+  // and phase 2's (log_words x 4), the claim, h at the eight operations for two points, and the
+  // in/out check's first (lo, hi)
+  const uint64_t n_g = (uint64_t)kShiftKeys * 64, n_slots = 2 * 12 + 4 * (uint64_t)log_words;
+  const uint64_t n_zeroed = n_g + n_slots + 2 + 16 + 2;
+  SHIFT_TRY(B.alloc(&zeroed, 16 * n_zeroed));
+  uint32_t* g_raw = reinterpret_cast<uint32_t*>(zeroed);
+  uint4* slots = zeroed + n_g;
+  uint4* slots2 = slots + 24;
+  uint4* claim = slots + n_slots;
+  uint4* h_ops = claim + 2;
+  uint4* init_lohi = h_ops + 16;
   SHIFT_TRY(B.alloc(&g, 16ull * kFlat));
   SHIFT_TRY(B.alloc(&h, 16ull * kFlat));
   SHIFT_TRY(B.alloc(&h_keep, 16ull * kFlat * 2));
   SHIFT_TRY(B.alloc(&eq_rjs, 16ull * kLen));
-  SHIFT_TRY(B.alloc(&h_ops, 16ull * 16));
   SHIFT_TRY(B.alloc(&T, 16ull * kShiftKeys));
   SHIFT_TRY(B.alloc(&W, 16ull * n_words));
   SHIFT_TRY(B.alloc(&M, 16ull * n_words));
   SHIFT_TRY(B.alloc(&eq_pub, 16ull << (log_public > 0 ? log_public - 1 : 0)));
-  SHIFT_TRY(B.alloc(&acc, 64));
 
   // lambdas and their powers per operand class
   const hu128 lam_and = sample(t), lam_mul = sample(t);
@@ -678,7 +688,7 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
   SHIFT_TRY(eq_tensor(to_u4(bmul.r_x).data(), log_mul, eq_mul, s));
 
   // ---- phase 1: g and h parts
-  BGPU_CUDA(cudaMemsetAsync(g_raw, 0, 16ull * kShiftKeys * 64, s));
+  BGPU_CUDA(cudaMemsetAsync(zeroed, 0, 16 * n_zeroed, s));
   if (terms.n) {
     launch_pdl(shift_g_kernel, grid_for(terms.n, kTile, 148 * 8), kTile, 0, s, terms.vi, terms.c,
                terms.key, terms.n, d_witness, eq_and, eq_mul, g_raw);
@@ -693,27 +703,22 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
     lagrange_phi(6, kind == 0 ? band.r_zhat : bmul.r_zhat, lt);
     Lag64 L;
     for (int i = 0; i < 64; i++) L.l[i] = u4(lt[i]);
-    launch_pdl(shift_h_kernel, kFlat / 256, 256, 0, s, L, h_keep + kind * kFlat);
+    launch_pdl(shift_h_kernel, kFlat / 256, 256, 0, s, L, h_keep + kind * kFlat,
+               kind == 0 ? h : nullptr);
     SHIFT_TRY(launched("shift_h_kernel"));
   }
-  BGPU_CUDA(cudaMemcpyAsync(h, h_keep, 16ull * kFlat, cudaMemcpyDeviceToDevice, s));
 
-  // device round state: phase-1 sum slots (12 x 2), phase-2 slots (log_words x 4); dstate = the
-  // phase-1 claim, the phase-2 running values (shift claim, in/out claim, eq prefix) and the
-  // in/out check's first (lo, hi); challenges (12 + log_words)
-  uint4 *slots, *dstate, *chal;
+  // device round state: dstate = the phase-1 claim and the phase-2 running values (shift claim,
+  // in/out claim, eq prefix); challenges (12 + log_words)
+  uint4 *dstate, *chal;
   ShiftRoundConst* rconst;
-  const uint64_t n_slots = 2 * 12 + 4 * (uint64_t)log_words;
-  SHIFT_TRY(B.alloc(&slots, 16 * n_slots));
-  SHIFT_TRY(B.alloc(&dstate, 16 * 6));
+  SHIFT_TRY(B.alloc(&dstate, 16 * 4));
   SHIFT_TRY(B.alloc(&chal, 16 * (12 + (uint64_t)log_words)));
   SHIFT_TRY(B.alloc(&rconst, sizeof(ShiftRoundConst) * log_words));
-  BGPU_CUDA(cudaMemsetAsync(slots, 0, 16 * n_slots, s));
-  uint4* slots2 = slots + 24;
 
   // the provers' claims: sum_v <g_v, h_v> (phase_1.rs:96-101)
-  BGPU_CUDA(cudaMemsetAsync(acc + 8, 0, 32, s));
-  launch_pdl(dot2_kernel, grid_for(kFlat, 256, 148), 256, 0, s, g, 0, 0, h, kFlat, acc + 8);
+  launch_pdl(dot2_kernel, grid_for(kFlat, 256, 148), 256, 0, s, g, 0, 0, h, kFlat,
+             reinterpret_cast<uint32_t*>(claim));
   SHIFT_TRY(launched("dot2_kernel"));
   DeviceTranscript dt;
   SHIFT_TRY(dt.begin(t, s));
@@ -724,12 +729,12 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
     const uint64_t size = (uint64_t)kFlat >> round;  // before this round's fold
     uint32_t* ys = reinterpret_cast<uint32_t*>(slots + 2 * round);
     if (round == 0) {
-      SHIFT_TRY(bivariate_eval(g, h, size / 2, ys, s));
+      SHIFT_TRY(bivariate_eval(g, h, size / 2, ys, s, false));
     } else {
       SHIFT_TRY(bivariate_fold_eval_dev(g, h, size * 2, chal + round - 1, ys, s));
     }
     SHIFT_TRY(bivariate_round_finish(dt, slots + 2 * round,
-                                     round == 0 ? reinterpret_cast<const uint4*>(acc + 8) : nullptr,
+                                     round == 0 ? claim : nullptr,
                                      dstate, nullptr, chal + round, s));
   }
   SHIFT_TRY(bivariate_tail(dt, g, h, (uint64_t)kFlat >> (tail0 - 1), 12 - tail0, chal + tail0 - 1,
@@ -763,7 +768,6 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
   eq_host(r_s.data(), 6, eq_rs);
   SHIFT_TRY(fold_words64(d_witness, n_words, eq_rj, W, s));
   SHIFT_TRY(eq_tensor(to_u4(rev).data(), 12, eq_rjs, s));
-  BGPU_CUDA(cudaMemsetAsync(h_ops, 0, 16 * 16, s));
   for (int kind = 0; kind < (same_z ? 1 : 2); kind++) {
     launch_pdl(shift_h_ops_kernel, kHopsBlocks, 256, 0, s, h_keep + kind * kFlat, eq_rjs,
                reinterpret_cast<uint32_t*>(h_ops + 8 * kind));
@@ -788,25 +792,17 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
   std::vector<hu128> z(p);
   for (auto& v : z) v = sample(t);
   const hu128 beta = sample(t);
-  // in the round loop dot2 follows a kernel and is launched programmatically (PDL relaxes only
-  // kernel-to-kernel order); the first one follows a memset and is launched plainly
-  auto dot2 = [&](uint64_t off0, uint64_t off1, uint64_t len, uint4* out, bool pdl = true) -> int {
+  auto dot2 = [&](uint64_t off0, uint64_t off1, uint64_t len, uint4* out) -> int {
     const unsigned grid = grid_for(len, 256, 148 * 2);
-    if (pdl)
-      BGPU_CUDA(launch_pdl(dot2_kernel, grid, 256, 0, s, (const uint4*)W, off0, off1,
-                           (const uint4*)eq_pub, len, reinterpret_cast<uint32_t*>(out)));
-    else
-      launch_pdl(dot2_kernel, grid, 256, 0, s, W, off0, off1, eq_pub, len,
-                 reinterpret_cast<uint32_t*>(out));
+    BGPU_CUDA(launch_pdl(dot2_kernel, grid, 256, 0, s, (const uint4*)W, off0, off1,
+                         (const uint4*)eq_pub, len, reinterpret_cast<uint32_t*>(out)));
     SHIFT_TRY(launched("dot2_kernel"));
     return BINIUS_OK;
   };
   uint32_t gn = p;  // Gruen32::n_vars_remaining
   SHIFT_TRY(eq_tensor(to_u4(z).data(), gn - 1, eq_pub, s));
   uint4* run = dstate + 1;
-  uint4* init_lohi = dstate + 4;
-  BGPU_CUDA(cudaMemsetAsync(init_lohi, 0, 32, s));
-  SHIFT_TRY(dot2(0, 1ull << (gn - 1), 1ull << (gn - 1), init_lohi, false));
+  SHIFT_TRY(dot2(0, 1ull << (gn - 1), 1ull << (gn - 1), init_lohi));
   const uint4 z0 = u4(z[gn - 1]);
   std::vector<ShiftRoundConst> consts(log_words);
   {
@@ -842,7 +838,7 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
     const uint64_t half = 1ull << (n_rem - 1);
     uint4* ys = slots2 + 4 * k;
     if (n_rem == log_words) {
-      SHIFT_TRY(bivariate_eval(W, M, half, reinterpret_cast<uint32_t*>(ys), s));
+      SHIFT_TRY(bivariate_eval(W, M, half, reinterpret_cast<uint32_t*>(ys), s, false));
     } else {
       SHIFT_TRY(bivariate_fold_eval_dev(W, M, half * 4, chal + 12 + k - 1,
                                         reinterpret_cast<uint32_t*>(ys), s));

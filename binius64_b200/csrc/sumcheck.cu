@@ -48,9 +48,21 @@ unsigned grid_for(uint64_t n, unsigned threads, unsigned max_blocks = 148 * 8) {
 // tensors are small and on the protocol's critical path, so latency matters: the tables depend
 // only on the point (a kernel argument), so under programmatic dependent launch they are built
 // while the previous kernel still runs, and only the writes wait for it.
+//
+// With blocks0 < gridDim.x the launch builds two tensors one behind the other, the first blocks0
+// blocks that of p's coordinates off .. off + n - 1, the others that of the n1 after them.
 __global__ void __launch_bounds__(256)
-    eq_small_kernel(uint4* __restrict__ out, Point32 p, uint32_t off, uint32_t n) {
+    eq_small_kernel(uint4* __restrict__ out, Point32 p, uint32_t off, uint32_t n, uint32_t blocks0,
+                    uint32_t n1) {
   __shared__ uint4 s_lo[256], s_hi[256];
+  uint32_t block = blockIdx.x, blocks = blocks0;
+  if (block >= blocks0) {
+    out += 1ull << n;
+    off += n;
+    n = n1;
+    block -= blocks0;
+    blocks = gridDim.x - blocks0;
+  }
   const uint32_t k = n < 8 ? n : 8, m = n - k;
   const uint32_t n_lo = 1u << k;
   // threads 0..127 build the low table, 128..255 the high one, by doubling: after step i a
@@ -71,8 +83,8 @@ __global__ void __launch_bounds__(256)
   pdl_trigger();
   __syncthreads();
   const uint64_t total = 1ull << n;
-  for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < total;
-       j += (uint64_t)gridDim.x * blockDim.x)
+  for (uint64_t j = block * (uint64_t)blockDim.x + threadIdx.x; j < total;
+       j += (uint64_t)blocks * blockDim.x)
     out[j] = gf_mul(s_lo[j & (n_lo - 1)], s_hi[j >> k]);
 }
 
@@ -377,8 +389,8 @@ int eq_tensor(const uint4* h_point, uint32_t n, uint4* d_out, cudaStream_t s) {
   memset(&p, 0, sizeof(p));
   if (n) memcpy(p.r, h_point, 16 * (size_t)n);
   if (n <= 16) {
-    BGPU_CUDA(launch_pdl(eq_small_kernel, grid_for(1ull << n, kThreads), kThreads, 0, s, d_out, p,
-                         0u, n));
+    const unsigned grid = grid_for(1ull << n, kThreads);
+    BGPU_CUDA(launch_pdl(eq_small_kernel, grid, kThreads, 0, s, d_out, p, 0u, n, grid, 0u));
     count_launch();
     return BINIUS_OK;
   }
@@ -386,17 +398,15 @@ int eq_tensor(const uint4* h_point, uint32_t n, uint4* d_out, cudaStream_t s) {
   uint4* tmp = nullptr;
   const uint64_t nlo = 1ull << k, nhi = 1ull << (n - k);
   BGPU_CUDA(dev_alloc(&tmp, 16 * (nlo + nhi), s));
-  cudaError_t e =
-      launch_pdl(eq_small_kernel, grid_for(nlo, kThreads), kThreads, 0, s, tmp, p, 0u, k);
-  if (e == cudaSuccess)
-    e = launch_pdl(eq_small_kernel, grid_for(nhi, kThreads), kThreads, 0, s, tmp + nlo, p, k,
-                   n - k);
+  const unsigned blocks0 = grid_for(nlo, kThreads);
+  cudaError_t e = launch_pdl(eq_small_kernel, blocks0 + grid_for(nhi, kThreads), kThreads, 0, s,
+                             tmp, p, 0u, k, blocks0, n - k);
   if (e == cudaSuccess)
     e = launch_pdl(eq_expand_kernel, grid_for(1ull << n, kThreads, 148 * 16), kThreads, 0, s,
                    d_out, (const uint4*)tmp, (const uint4*)(tmp + nlo), k, 1ull << n);
   dev_free(tmp, s);
   if (e != cudaSuccess) return cuda_error(e, "eq tensor kernels");
-  count_launch(3);
+  count_launch(2);
   return BINIUS_OK;
 }
 
@@ -432,8 +442,8 @@ int fold_b128_elems(const uint4* d_in, uint4* d_out, uint64_t n, const uint4* d_
 }
 
 int bivariate_eval(const uint4* d_a, const uint4* d_b, uint64_t half, uint32_t* d_out8,
-                   cudaStream_t s) {
-  BGPU_CUDA(cudaMemsetAsync(d_out8, 0, 32, s));
+                   cudaStream_t s, bool clear) {
+  if (clear) BGPU_CUDA(cudaMemsetAsync(d_out8, 0, 32, s));
   launch_pdl(bivariate_eval_kernel, grid_for(half, kThreads), kThreads, 0, s, d_a, d_b, half,
              d_out8);
   BGPU_LAUNCH_CHECK("bivariate_eval_kernel");
