@@ -766,19 +766,18 @@ int and_reduction_finish(const binius_cs* cs, AndPrep& p, Transcript& t, AndResu
     // finish kernel, no host round trip.  dev holds the claim, the round constants (rounds in
     // order log_n .. 1) and the challenges.
     std::vector<AndRoundConst> consts(log_n + 1);
-    for (uint32_t n_rem = log_n; n_rem > 0; n_rem--) {
-      const u128h alpha = point[n_rem - 1];
-      consts[log_n - n_rem] = {to_uint4(alpha), to_uint4(host_gf_inv(1 ^ alpha))};
-    }
+    std::vector<u128h> inv(log_n);
+    for (uint32_t i = 0; i < log_n; i++) inv[i] = 1 ^ point[i];
+    host_gf_batch_inv(inv);
+    for (uint32_t n_rem = log_n; n_rem > 0; n_rem--)
+      consts[log_n - n_rem] = {to_uint4(point[n_rem - 1]), to_uint4(inv[n_rem - 1])};
     consts[log_n].alpha = to_uint4(sum);  // the initial claim rides in the spare slot
     AndRoundConst* d_consts = reinterpret_cast<AndRoundConst*>(dev);
     uint4* d_claim = dev + 2 * log_n;
     uint4* d_chal = dev + 2 * (log_n + 1);
-    e = cudaMemcpyAsync(d_consts, consts.data(), sizeof(AndRoundConst) * (log_n + 1),
-                        cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) { rc = cuda_error(e, "round constants"); break; }
     DeviceTranscript dt;
-    if ((rc = dt.begin(t, s))) break;
+    if ((rc = dt.begin(t, s, {{d_consts, consts.data(), sizeof(AndRoundConst) * (log_n + 1)}})))
+      break;
     // rounds whose fold starts from at most tail_max_len() elements run in the single-CTA tail
     uint32_t tail_n = 0;  // n_rem of the first tail round (0: no tail)
     for (uint32_t n_rem = log_n - 1; n_rem > 0; n_rem--)

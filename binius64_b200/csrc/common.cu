@@ -87,6 +87,22 @@ hu128 host_gf_inv(hu128 a) {
   return host_gf_mul(r, r);
 }
 
+void host_gf_batch_inv(std::vector<hu128>& v) {
+  std::vector<hu128> pre(v.size());
+  hu128 acc = 1;
+  for (size_t i = 0; i < v.size(); i++) {
+    pre[i] = acc;
+    if (v[i]) acc = host_gf_mul(acc, v[i]);
+  }
+  hu128 inv = host_gf_inv(acc);
+  for (size_t i = v.size(); i-- > 0;) {
+    if (!v[i]) continue;
+    const hu128 x = v[i];
+    v[i] = host_gf_mul(inv, pre[i]);
+    inv = host_gf_mul(inv, x);
+  }
+}
+
 // Raises the dynamic shared memory limit of `func` on the current device to `bytes`, once per
 // (device, kernel).  Setting a per-launch value instead races between threads that launch the
 // same kernel with different sizes.

@@ -12,6 +12,7 @@
 #pragma once
 #include <stdint.h>
 
+#include <initializer_list>
 #include <vector>
 
 #include "gf128.cuh"
@@ -489,7 +490,13 @@ class DeviceTranscript {
   static constexpr uint32_t kTapeCap = 1u << 16;
 
   ~DeviceTranscript();
-  int begin(const Transcript& t, cudaStream_t s);
+  // With the state, `uploads` from host memory to 16-byte aligned device memory.
+  struct Upload {
+    void* dst;
+    const void* src;
+    size_t bytes;
+  };
+  int begin(const Transcript& t, cudaStream_t s, std::initializer_list<Upload> uploads = {});
   TranscriptState* state() const { return reinterpret_cast<TranscriptState*>(mem_); }
   uint8_t* tape() const { return mem_ + kStateBytes; }
   // message() of n_bytes (a multiple of 4, 4-byte aligned) that are in device memory.

@@ -154,6 +154,8 @@ static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStre
 typedef unsigned __int128 hu128;
 hu128 host_gf_mul(hu128 a, hu128 b);
 hu128 host_gf_inv(hu128 a);
+// Every element by its inverse (zero stays), with one inversion.
+void host_gf_batch_inv(std::vector<hu128>& v);
 
 }  // namespace bgpu
 

@@ -866,24 +866,6 @@ void normalize_leaves(const std::vector<hu128>& biv, IntMulResult& res) {
   }
 }
 
-// In place: v[i] <- 1 / v[i] for nonzero entries (zero stays zero, as invert_or_zero), with one
-// inversion for the whole vector (Montgomery's trick).
-void batch_inv(std::vector<hu128>& v) {
-  std::vector<hu128> pre(v.size());
-  hu128 acc = 1;
-  for (size_t i = 0; i < v.size(); i++) {
-    pre[i] = acc;
-    if (v[i]) acc = host_gf_mul(acc, v[i]);
-  }
-  hu128 inv = host_gf_inv(acc);
-  for (size_t i = v.size(); i-- > 0;) {
-    if (!v[i]) continue;
-    const hu128 x = v[i];
-    v[i] = host_gf_mul(inv, pre[i]);
-    inv = host_gf_mul(inv, x);
-  }
-}
-
 hu128 sample(Transcript& t) {
   uint8_t b[16];
   t.sample_elem(b);
@@ -1003,7 +985,7 @@ class IntMulDevice {
         if (points[g]->size() != b.n) return set_error(BINIUS_E_ARG, "intmul batch: point lengths");
         inv[t * b.n_groups + g] = 1 ^ (*points[g])[b.n - 1 - t];
       }
-    batch_inv(inv);
+    host_gf_batch_inv(inv);
     for (uint32_t t = 0; t < b.n; t++)
       for (uint32_t g = 0; g < b.n_groups; g++) {
         ha[2 * (t * b.n_groups + g)] = u4((*points[g])[b.n - 1 - t]);
@@ -1105,7 +1087,7 @@ int IntMulDevice::layer(uint4* set, uint32_t pairs, std::vector<hu128>& point,
   a.n = n;
   std::vector<hu128> inv(n);
   for (uint32_t t = 0; t < n; t++) inv[t] = 1 ^ point[n - 1 - t];
-  batch_inv(inv);
+  host_gf_batch_inv(inv);
   for (uint32_t t = 0; t < n; t++) a.alphas[t] = ImAlpha{u4(point[n - 1 - t]), u4(inv[t])};
   hu128 bp = 1, G = 0;
   for (uint32_t p = 0; p < pairs; p++, bp = host_gf_mul(bp, beta)) {

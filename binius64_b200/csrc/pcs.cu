@@ -316,8 +316,10 @@ int pcs_prove_impl(const binius_pcs* P, const binius_pcs_committed* C, const voi
       if ((rc = eq_tensor(reinterpret_cast<const uint4*>(h_point + 16 * 7), n, b, s))) break;
       // s_hat_v = fold_1b_rows_for_b128(witness, suffix_tensor)
       if ((rc = fold_1b_rows(static_cast<const uint4*>(d_witness), b, N, d_small, s))) break;
-      // the BaseFold message copy needs no challenge: queued before the host round trip
+      // the BaseFold message copy and the cleared sums need no challenge: queued before the host
+      // round trip
       cudaError_t e = cudaMemcpyAsync(a, d_witness, 16 * N, cudaMemcpyDeviceToDevice, s);
+      if (e == cudaSuccess) e = cudaMemsetAsync(slots, 0, 32ull * n, s);
       if (e != cudaSuccess) { rc = cuda_error(e, "copy witness"); break; }
       uint8_t s_hat_v[128 * 16];
       if ((rc = read_sync(s_hat_v, d_small, sizeof(s_hat_v), s))) break;
@@ -338,21 +340,15 @@ int pcs_prove_impl(const binius_pcs* P, const binius_pcs_committed* C, const voi
           h_eq[k] ^= hi;
         }
       }
-      e = cudaMemcpyAsync(eq_r, h_eq, sizeof(h_eq), cudaMemcpyHostToDevice, s);
-      if (e != cudaSuccess) { rc = cuda_error(e, "eq(r'') upload"); break; }
       u128h sum = 0;
       for (int j = 0; j < 128; j++) sum ^= host_gf_mul(u[j], h_eq[j]);
-      e = cudaMemcpyAsync(claim + 1, &sum, 16, cudaMemcpyHostToDevice, s);
-      if (e != cudaSuccess) { rc = cuda_error(e, "claim upload"); break; }
-      e = cudaMemsetAsync(slots, 0, 32ull * n, s);
-      if (e != cudaSuccess) { rc = cuda_error(e, "round sums"); break; }
+      DeviceTranscript dt;
+      if ((rc = dt.begin(t, s, {{eq_r, h_eq, sizeof(h_eq)}, {claim + 1, &sum, 16}}))) break;
       // rs_eq_ind = fold_b128_elems_inplace(suffix_tensor, eq(r'')) in place in b
       if ((rc = fold_b128_elems(b, b, N, eq_r, s))) break;
 
       // BaseFold rounds on the device transcript: the round's sums, the FRI fold and commit on a
       // commit round, then the finish kernel (message, root, challenge, next table)
-      DeviceTranscript dt;
-      if ((rc = dt.begin(t, s))) break;
       uint32_t tape_bytes = 0;
       // the rounds after the last FRI commit inside the loop whose fold starts from at most
       // tail_max_len() elements run in the single-CTA tail

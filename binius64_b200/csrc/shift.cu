@@ -818,14 +818,11 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
       if (n_rem <= p) g2--;
     }
   }
-  BGPU_CUDA(cudaMemcpyAsync(rconst, consts.data(), sizeof(ShiftRoundConst) * log_words,
-                            cudaMemcpyHostToDevice, s));
-  {
-    // the in/out claim is set by the first round from init_lohi
-    const uint4 init3[3] = {u4(gamma), u4(0), u4(1)};
-    BGPU_CUDA(cudaMemcpyAsync(run, init3, sizeof(init3), cudaMemcpyHostToDevice, s));
-  }
-  SHIFT_TRY(dt.begin(t, s));
+  // the in/out claim is set by the first round from init_lohi
+  const uint4 init3[3] = {u4(gamma), u4(0), u4(1)};
+  SHIFT_TRY(dt.begin(t, s,
+                     {{rconst, consts.data(), sizeof(ShiftRoundConst) * log_words},
+                      {run, init3, sizeof(init3)}}));
   // rounds whose fold starts from at most tail_max_len() elements run in the single-CTA tail
   uint32_t tail_n = 0;  // n_rem of the first tail round (0: no tail)
   for (uint32_t n_rem = log_words - 1; n_rem > 0; n_rem--)
