@@ -28,9 +28,16 @@ int bivariate_eval(const uint4* d_a, const uint4* d_b, uint64_t half, uint32_t* 
 // Fold (a, b) of length size by r, then (y_1, y_inf) of the next round.
 int bivariate_fold_eval(uint4* d_a, uint4* d_b, uint64_t size, const uint8_t r[16],
                         uint32_t* d_out8, cudaStream_t s);
+// Dot products of a round that go with its fold: eq (n elements, a power of two) with the folded
+// a's upper half from its start, and with the n elements after those when len = 2 n (else len = n).
+struct FoldDot {
+  const uint4* eq;
+  uint64_t n, len;
+};
 // As bivariate_fold_eval with the challenge in device memory (d_r) and no clearing of d_out8.
+// With dot, its two products are added to the two elements after the sums.
 int bivariate_fold_eval_dev(uint4* d_a, uint4* d_b, uint64_t size, const uint4* d_r,
-                            uint32_t* d_out8, cudaStream_t s);
+                            uint32_t* d_out8, cudaStream_t s, const FoldDot* dot = nullptr);
 class DeviceTranscript;
 // The device Fiat-Shamir step of a plain bivariate product round: reads (y_1, y_inf) at d_ys
 // and the claim (d_claim_init if set, else d_claim), writes the message (c_0, c_1) and then the

@@ -834,17 +834,18 @@ int shift_reduction_prove(const binius_cs* cs, const uint64_t* d_witness, Transc
     const uint32_t k = log_words - n_rem;
     const uint64_t half = 1ull << (n_rem - 1);
     uint4* ys = slots2 + 4 * k;
+    // the in/out check's dot products with the folded words, by the fold's launch after the first
+    FoldDot dot = {eq_pub, half, half};
+    if (p < n_rem)
+      dot = {eq_pub, 1ull << (gn - 1), 2ull << (gn - 1)};
+    else
+      SHIFT_TRY(eq_tensor(to_u4(z).data(), n_rem - 1, eq_pub, s));
     if (n_rem == log_words) {
       SHIFT_TRY(bivariate_eval(W, M, half, reinterpret_cast<uint32_t*>(ys), s, false));
+      SHIFT_TRY(dot2(half, half + dot.len - dot.n, dot.n, ys + 2));
     } else {
       SHIFT_TRY(bivariate_fold_eval_dev(W, M, half * 4, chal + 12 + k - 1,
-                                        reinterpret_cast<uint32_t*>(ys), s));
-    }
-    if (p < n_rem) {
-      SHIFT_TRY(dot2(half, half + (1ull << (gn - 1)), 1ull << (gn - 1), ys + 2));
-    } else {
-      SHIFT_TRY(eq_tensor(to_u4(z).data(), n_rem - 1, eq_pub, s));
-      SHIFT_TRY(dot2(half, half, half, ys + 2));
+                                        reinterpret_cast<uint32_t*>(ys), s, &dot));
     }
     if (n_rem <= p) gn--;
     BGPU_CUDA(launch_pdl(shift_round_finish_kernel, 1, kFsThreads, 0, s, dt.state(), dt.tape(),

@@ -191,10 +191,15 @@ __global__ void __launch_bounds__(kThreads)
 // j + size/4, and each forms one of the two products (the even lane y_1's fa1 fb1, the odd lane
 // y_inf's after a shuffle brings fa1, fb1 over).  The products by r go through r's nibble tables,
 // which each block builds in shared memory from r (read from r_ptr, else r_arg).
+//
+// DOT: the even lanes also multiply their folded a (the upper half's) by dot.eq.  The shift
+// reduction's in/out check takes these products of the folded words; a launch of its own after the
+// fold cost 5 us a round (with it here a proof of 2^20 words 2506 -> 2477 us, of 2^16 1211 -> 1193).
+template <bool DOT>
 __global__ void __launch_bounds__(kThreads)
     bivariate_fold_eval_kernel(uint4* __restrict__ a, uint4* __restrict__ b, uint64_t size,
                                uint4 r_arg, const uint4* __restrict__ r_ptr,
-                               uint32_t* __restrict__ out) {
+                               uint32_t* __restrict__ out, FoldDot dot) {
   __shared__ NibbleTable tab;
   __shared__ uint4 basis[128];
   pdl_wait();
@@ -203,6 +208,7 @@ __global__ void __launch_bounds__(kThreads)
   const uint64_t h = size >> 1, q = size >> 2;
   const uint32_t odd = threadIdx.x & 1;
   u256 acc = {0, 0, 0, 0};
+  uint4 d[2] = {gf_zero(), gf_zero()};
   const uint64_t all = (uint64_t)gridDim.x * blockDim.x;
   // warp-uniform sweeps: every lane of a warp runs the same iterations (shuffles below)
   for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < 2 * q;
@@ -217,6 +223,8 @@ __global__ void __launch_bounds__(kThreads)
       fb = gf_add(b_lo, gf_mul_nibble(tab, gf_add(b_hi, b_lo)));
       a[pos] = fa;
       b[pos] = fb;
+      if (DOT && !odd && j < dot.len)
+        gf_add_into(j < dot.n ? d[0] : d[1], gf_mul_nl(fa, __ldg(dot.eq + (j & (dot.n - 1)))));
     }
     // the odd lane takes its even partner's (fa1, fb1)
     const uint4 pa = shfl_gf(fa, 0, 2), pb = shfl_gf(fb, 0, 2);
@@ -224,25 +232,30 @@ __global__ void __launch_bounds__(kThreads)
     xor_into(acc, clmul128(odd ? gf_add(fa, pa) : fa, odd ? gf_add(fb, pb) : fb));
   }
   const uint4 s = reduce256(acc);
-  uint4 v[2] = {odd ? gf_zero() : s, odd ? s : gf_zero()};
-  block_xor_reduce<2>(v, out);
+  uint4 v[DOT ? 4 : 2] = {odd ? gf_zero() : s, odd ? s : gf_zero()};
+  if (DOT) {
+    v[DOT ? 2 : 0] = d[0];
+    v[DOT ? 3 : 0] = d[1];
+  }
+  block_xor_reduce<DOT ? 4 : 2>(v, out);
 }
 
 // The small rounds of bivariate_fold_eval_kernel (no nibble tables) on four lanes per position j:
 // lane k folds one of a[j], a[q + j], b[j], b[q + j] by r, the four folded values are shared by
 // shuffles, and lanes 0 and 1 form the two products.  One multiply then one product per lane,
 // where one thread per position ran six dependent out-of-line multiplies: these rounds are
-// latency chains on few CTAs.
+// latency chains on few CTAs.  DOT: lane 3 forms the position's dot product.
+template <bool DOT>
 __global__ void __launch_bounds__(kThreads)
     bivariate_fold_eval_lanes_kernel(uint4* __restrict__ a, uint4* __restrict__ b, uint64_t size,
                                      uint4 r_arg, const uint4* __restrict__ r_ptr,
-                                     uint32_t* __restrict__ out) {
+                                     uint32_t* __restrict__ out, FoldDot dot) {
   pdl_wait();
   pdl_trigger();
   const uint64_t h = size >> 1, q = size >> 2;
   const uint4 r = r_ptr ? *r_ptr : r_arg;
   const uint32_t k = threadIdx.x & 3;
-  uint4 v[2] = {gf_zero(), gf_zero()};
+  uint4 v[DOT ? 4 : 2] = {};
   const uint64_t all = (uint64_t)gridDim.x * blockDim.x;
   // warp-uniform sweeps: every lane of a warp runs the same iterations (shuffles below)
   for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < 4 * q;
@@ -259,10 +272,25 @@ __global__ void __launch_bounds__(kThreads)
     }
     const uint4 fa0 = shfl_gf(f, 0, 4), fa1 = shfl_gf(f, 1, 4), fb0 = shfl_gf(f, 2, 4),
                 fb1 = shfl_gf(f, 3, 4);
-    if (live && k == 0) gf_add_into(v[0], gf_mul_nl(fa1, fb1));
-    if (live && k == 1) gf_add_into(v[1], gf_mul_nl(gf_add(fa0, fa1), gf_add(fb0, fb1)));
+    if (!DOT) {
+      if (live && k == 0) gf_add_into(v[0], gf_mul_nl(fa1, fb1));
+      if (live && k == 1) gf_add_into(v[1], gf_mul_nl(gf_add(fa0, fa1), gf_add(fb0, fb1)));
+      continue;
+    }
+    // one product a lane, formed together
+    const bool dots = k == 3 && j < dot.len;
+    if (live && (k < 2 || dots)) {
+      const uint4 x = k == 1 ? gf_add(fa0, fa1) : fa1;
+      const uint4 y = k == 0   ? fb1
+                      : k == 1 ? gf_add(fb0, fb1)
+                               : __ldg(dot.eq + (j & (dot.n - 1)));
+      const uint4 m = gf_mul_nl(x, y);
+      if (k == 0) gf_add_into(v[0], m);
+      if (k == 1) gf_add_into(v[1], m);
+      if (k == 3) gf_add_into(j < dot.n ? v[DOT ? 2 : 0] : v[DOT ? 3 : 0], m);
+    }
   }
-  block_xor_reduce<2>(v, out);
+  block_xor_reduce<DOT ? 4 : 2>(v, out);
 }
 
 // The Fiat-Shamir step of a plain bivariate product round (BivariateProductSumcheckProver,
@@ -459,31 +487,30 @@ int bivariate_fold_eval(uint4* d_a, uint4* d_b, uint64_t size, const uint8_t r[1
   BGPU_CUDA(cudaMemsetAsync(d_out8, 0, 32, s));
   const unsigned grid = grid_for(size / 2, kThreads);  // two lanes per folded position
   if (size >= kMulTableMinSize) {
-    launch_pdl(bivariate_fold_eval_kernel, grid, kThreads, 0, s, d_a, d_b, size, rv, nullptr,
-               d_out8);
+    launch_pdl(bivariate_fold_eval_kernel<false>, grid, kThreads, 0, s, d_a, d_b, size, rv, nullptr,
+               d_out8, FoldDot{});
     BGPU_LAUNCH_CHECK("bivariate_fold_eval_kernel");
     count_launch();
     return BINIUS_OK;
   }
-  launch_pdl(bivariate_fold_eval_lanes_kernel, grid_for(size, kThreads), kThreads, 0, s, d_a, d_b,
-             size, rv, nullptr, d_out8);
+  launch_pdl(bivariate_fold_eval_lanes_kernel<false>, grid_for(size, kThreads), kThreads, 0, s, d_a,
+             d_b, size, rv, nullptr, d_out8, FoldDot{});
   BGPU_LAUNCH_CHECK("bivariate_fold_eval_lanes_kernel");
   count_launch();
   return BINIUS_OK;
 }
 
 int bivariate_fold_eval_dev(uint4* d_a, uint4* d_b, uint64_t size, const uint4* d_r,
-                            uint32_t* d_out8, cudaStream_t s) {
+                            uint32_t* d_out8, cudaStream_t s, const FoldDot* dot) {
   if (size < 4) return set_error(BINIUS_E_ARG, "bivariate_fold_eval needs size >= 4");
-  const unsigned grid = grid_for(size / 2, kThreads);  // two lanes per folded position
-  cudaError_t e;
-  if (size >= kMulTableMinSize) {
-    e = launch_pdl(bivariate_fold_eval_kernel, grid, kThreads, 0, s, d_a, d_b, size,
-                   gf_zero_host(), d_r, d_out8);
-  } else {
-    e = launch_pdl(bivariate_fold_eval_lanes_kernel, grid_for(size, kThreads), kThreads, 0, s,
-                   d_a, d_b, size, gf_zero_host(), d_r, d_out8);
-  }
+  const bool big = size >= kMulTableMinSize;
+  // two lanes per folded position, or four
+  const unsigned grid = grid_for(big ? size / 2 : size, kThreads);
+  auto kern = big ? (dot ? bivariate_fold_eval_kernel<true> : bivariate_fold_eval_kernel<false>)
+                  : (dot ? bivariate_fold_eval_lanes_kernel<true>
+                         : bivariate_fold_eval_lanes_kernel<false>);
+  cudaError_t e = launch_pdl(kern, grid, kThreads, 0, s, d_a, d_b, size, gf_zero_host(), d_r,
+                             d_out8, dot ? *dot : FoldDot{});
   if (e != cudaSuccess) return cuda_error(e, "bivariate_fold_eval_kernel");
   count_launch();
   return BINIUS_OK;
