@@ -70,7 +70,16 @@ def to_device(arr: np.ndarray, device: str | int = "cuda"):
 
 def to_host(t) -> np.ndarray:
     """device int64 (n, 2) -> numpy uint64 (n, 2)."""
-    return t.detach().cpu().contiguous().numpy().view(np.uint64).reshape(-1, 2)
+    out = t.detach().cpu().contiguous().numpy().view(np.uint64).reshape(-1, 2)
+    device_status()  # the copy has waited for what computed t
+    return out
+
+
+def device_status() -> None:
+    """Raises when a bounded wait on the device has run out (binius_device_status): for programs that
+    wait for the device and read results by themselves; to_host and the calls that return bytes ask
+    it too."""
+    check(lib().binius_device_status())
 
 
 def empty_elems(n: int, device="cuda"):
@@ -169,7 +178,9 @@ class MerkleCommitted:
     nodes: object  # torch uint8 tensor
 
     def root(self) -> bytes:
-        return bytes(self.nodes[-1].cpu().numpy().tobytes())
+        root = bytes(self.nodes[-1].cpu().numpy().tobytes())
+        device_status()
+        return root
 
     def layer(self, layer_depth: int, stream=None) -> list[bytes]:
         """MerkleTreeProver::layer (prover/prover/src/merkle_tree/mod.rs:50-55): the digests at

@@ -133,6 +133,8 @@ _SIGS = {
     "binius_queue_wait": (_int, [_vp, _u64, _vp, _c.c_size_t, _vp, _vp]),
     "binius_queue_stats": (_int, [_vp, _vp]),
     "binius_debug_fail_allocs": (None, [_c.c_int64]),
+    "binius_device_status": (_int, []),
+    "binius_debug_tensor_wait": (_int, [_vp]),
     "binius_fri_n_test_queries": (_u32, [_u32, _u32]),
     "binius_fri_estimate_optimal_arity": (_u32, [_u32, _u32, _u32]),
     "binius_gf_mul_batch": (_int, [_vp, _vp, _vp, _u64, _vp]),

@@ -32,7 +32,48 @@ int clear_error() {
   return BINIUS_OK;
 }
 
+namespace {
+std::atomic<uint32_t*> g_tensor_word{nullptr};
+const char* const kTensorStall =
+    "a bounded wait for the tensor cores ran out; results since then are undefined";
+}  // namespace
+
+bool tensor_stalled() {
+  const uint32_t* w = g_tensor_word.load(std::memory_order_acquire);
+  return w && *static_cast<const volatile uint32_t*>(w) != 0;
+}
+
+int tensor_word(uint32_t** word) {
+  static std::mutex mu;
+  if (tensor_stalled()) return set_error(BINIUS_E_TIMEOUT, kTensorStall);
+  uint32_t* w = g_tensor_word.load(std::memory_order_acquire);
+  if (!w) {
+    std::lock_guard<std::mutex> lock(mu);
+    w = g_tensor_word.load(std::memory_order_acquire);
+    if (!w) {
+      // the first launch to need it may be one that is being captured
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      BGPU_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&w), 64,
+                                          cudaHostAllocPortable | cudaHostAllocMapped);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) return cuda_error(e, "tensor status word");
+      *w = 0;
+      g_tensor_word.store(w, std::memory_order_release);
+    }
+  }
+  *word = w;
+  return BINIUS_OK;
+}
+
+// A finished wait, or the report that it came with.
+static cudaError_t waited(cudaError_t e) {
+  return e == cudaSuccess && tensor_stalled() ? cudaErrorLaunchTimeout : e;
+}
+
 int cuda_error(cudaError_t e, const char* what) {
+  if (e == cudaErrorLaunchTimeout && tensor_stalled())
+    return set_error(BINIUS_E_TIMEOUT, kTensorStall);
   char buf[512];
   snprintf(buf, sizeof(buf), "%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
   return set_error(e == cudaErrorMemoryAllocation ? BINIUS_E_OOM : BINIUS_E_CUDA, buf);
@@ -406,7 +447,7 @@ void set_blocking_waits(bool on, double poll_micros) {
 }
 
 cudaError_t stream_wait(cudaStream_t s) {
-  if (!t_blocking_wait) return cudaStreamSynchronize(s);
+  if (!t_blocking_wait) return waited(cudaStreamSynchronize(s));
   if (!t_wait_event) {
     cudaError_t e = cudaEventCreateWithFlags(&t_wait_event,
                                              cudaEventBlockingSync | cudaEventDisableTiming);
@@ -417,10 +458,10 @@ cudaError_t stream_wait(cudaStream_t s) {
   const auto t0 = std::chrono::steady_clock::now();
   for (;;) {
     e = cudaEventQuery(t_wait_event);
-    if (e != cudaErrorNotReady) return e;
+    if (e != cudaErrorNotReady) return waited(e);
     if (std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count() >=
         t_poll_micros)
-      return cudaEventSynchronize(t_wait_event);
+      return waited(cudaEventSynchronize(t_wait_event));
     std::this_thread::yield();
   }
 }
@@ -443,11 +484,11 @@ cudaError_t mark_wait() {
   const auto t0 = std::chrono::steady_clock::now();
   for (;;) {
     const cudaError_t e = cudaEventQuery(t_mark_event);
-    if (e != cudaErrorNotReady) return e;
+    if (e != cudaErrorNotReady) return waited(e);
     if (t_blocking_wait) {
       if (std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0)
               .count() >= t_poll_micros)
-        return cudaEventSynchronize(t_mark_event);
+        return waited(cudaEventSynchronize(t_mark_event));
       std::this_thread::yield();
     }
   }
@@ -480,6 +521,11 @@ const char* binius_last_error(void) { return bgpu::g_last_error.c_str(); }
 const char* binius_version(void) { return "binius64_b200 0.1.0 (sm_100a)"; }
 
 uint64_t binius_launch_count(void) { return bgpu::g_launches.load(std::memory_order_relaxed); }
+
+int binius_device_status(void) {
+  if (bgpu::tensor_stalled()) return bgpu::set_error(BINIUS_E_TIMEOUT, bgpu::kTensorStall);
+  return bgpu::clear_error();
+}
 
 void binius_debug_fail_allocs(int64_t n_before_failure) {
   bgpu::g_allocs_before_failure.store(n_before_failure < 0 ? -1 : n_before_failure);

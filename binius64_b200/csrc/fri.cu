@@ -102,16 +102,14 @@ struct FoldTcShared {
   uint4 weights[1u << kMaxChallenges];
   tc::MatrixRows rows[kFoldPass];
   uint8_t ones[tc::kOnesBytes];
-  uint64_t done[kFoldGroups][2];
+  uint64_t done[kFoldGroups][2], drain;
   uint32_t tmem;
 };
-// Set when a wait for the tensor cores ran out (nothing more of that launch is then written).
-__device__ uint32_t g_fold_tc_stalled;
 
 __global__ void __launch_bounds__(kFoldThreads, 1)
     fold_interleaved_tc_kernel(const uint4* __restrict__ cw, uint32_t log_len, uint32_t log_batch,
                                Challenges ch, const uint4* __restrict__ dch,
-                               uint4* __restrict__ out) {
+                               uint4* __restrict__ out, uint32_t* stall_word) {
   pdl_wait();
   extern __shared__ __align__(128) uint8_t fold_smem[];
   FoldTcShared& sh = *reinterpret_cast<FoldTcShared*>(fold_smem);
@@ -123,6 +121,7 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
   if (threadIdx.x == 0) {
     for (uint32_t g = 0; g < kFoldGroups; g++)
       for (uint32_t b = 0; b < 2; b++) tc::mbar_init(&sh.done[g][b], 1);
+    tc::mbar_init(&sh.drain, kFoldThreads / 32);
     tc::mbar_init_fence();
   }
   // eq_ind(r)[j] = prod_i (bit_i(j) ? r_i : 1 + r_i)
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
       for (uint32_t k = 0; k < pairs; k++) {
         const uint32_t b = k & 1;
         if (k >= 2) {  // this pair of slots' products before last
-          ok = tc::mbar_wait(&sh.done[group][b], phase[b]) && ok;
+          tc::mbar_wait(&sh.done[group][b], phase[b], ok);
           phase[b] ^= 1;
           tc::fence_after();
         }
@@ -202,7 +201,7 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
         tc::commit(&sh.done[group][b]);
       }
       for (uint32_t k = pairs > 2 ? pairs - 2 : 0; k < pairs; k++) {
-        ok = tc::mbar_wait(&sh.done[group][k & 1], phase[k & 1]) && ok;
+        tc::mbar_wait(&sh.done[group][k & 1], phase[k & 1], ok);
         phase[k & 1] ^= 1;
       }
       tc::fence_after();
@@ -210,13 +209,26 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
       const uint2 p1 = tc::collect_part(sums + tc::kSumCols + lanes);
       uint4 y = tc::join_parts(p0, p1);
       if (pass) gf_add_into(y, out[i]);
-      if (ok) out[i] = y;
+      out[i] = y;
     }
     tc::fence_before();
     __syncthreads();
   }
-  if (!ok) atomicOr(&g_fold_tc_stalled, 1u);
-  if (threadIdx.x < 32) tc::tmem_free(tmem, 512);
+  tc::finish_launch(ok, &sh.drain, tmem, 512, stall_word);
+}
+
+// A wait for the tensor cores that nothing completes, of a few polls: what the transforms and folds
+// do when one of theirs runs out.
+__global__ void __launch_bounds__(32) tensor_wait_kernel(uint32_t* stall_word) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(&bar, 1);
+    tc::mbar_init_fence();
+  }
+  __syncwarp();
+  bool ok = true;
+  tc::mbar_wait(&bar, 0, ok, 16);
+  if (!ok && threadIdx.x == 0) tc::report_stall(stall_word);
 }
 
 // SCALED: rounds of one product (sf), else challenges from ch or dch and two products a round.
@@ -394,10 +406,12 @@ int launch_fold_interleaved(const void* d_codeword, uint32_t log_len, uint32_t l
   if (log_batch > 0 && log_len >= 7 && log_len < 38) {
     const void* kern = reinterpret_cast<const void*>(fold_interleaved_tc_kernel);
     if (int rc = ensure_smem_limit(kern, sizeof(FoldTcShared))) return rc;
+    uint32_t* stall_word = nullptr;
+    if (int rc = tensor_word(&stall_word)) return rc;
     const uint64_t ctas = ((1ull << (log_len - 7)) + kFoldGroups - 1) / kFoldGroups;
     launch_pdl(fold_interleaved_tc_kernel, (unsigned)std::min<uint64_t>(ctas, 148), kFoldThreads,
                sizeof(FoldTcShared), s, static_cast<const uint4*>(d_codeword), log_len, log_batch,
-               ch, dch, static_cast<uint4*>(d_out));
+               ch, dch, static_cast<uint4*>(d_out), stall_word);
     BGPU_LAUNCH_CHECK("fold_interleaved_tc_kernel");
   } else {
     launch_pdl(fold_interleaved_kernel, grid_for(1ull << log_len, 256), 256, 0, s,
@@ -537,6 +551,15 @@ int fri_commit_interleaved(const binius_ntt* ntt, const void* d_msg, uint32_t lo
 }  // namespace bgpu
 
 extern "C" {
+
+int binius_debug_tensor_wait(void* stream) {
+  uint32_t* stall_word = nullptr;
+  if (int rc = tensor_word(&stall_word)) return rc;
+  tensor_wait_kernel<<<1, 32, 0, as_stream(stream)>>>(stall_word);
+  BGPU_LAUNCH_CHECK("tensor_wait_kernel");
+  count_launch();
+  return clear_error();
+}
 
 int binius_fri_fold_interleaved(const void* d_codeword, uint32_t log_len, uint32_t log_batch,
                                 const void* h_challenges, void* d_out, void* stream) {

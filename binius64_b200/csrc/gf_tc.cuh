@@ -88,22 +88,34 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
 __device__ __forceinline__ void mbar_init_fence() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done;
+}
 // Waits for the phase of this parity: a bounded number of polls, each of which may sleep for some
-// 20 us, far beyond any tile's time.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+// 20 us, far beyond any tile's time.  `ok` becomes false when they run out; the thread then polls
+// once or twice a wait, goes through the rest of its launch (what it stores means nothing) and
+// reports at the end (finish_launch).
+constexpr uint32_t kWaitPolls = 1u << 16;
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, bool& ok,
+                                          uint32_t polls = kWaitPolls) {
   const uint32_t a = smem_addr(bar);
-  for (uint32_t i = 0; i < (1u << 16); i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
+  if (mbar_try(a, parity)) return;
+  for (uint32_t left = ok ? polls : 1; left; left--)
+    if (mbar_try(a, parity)) return;
+  ok = false;
+}
+// Reports a wait that ran out (tensor_word in internal.h).
+__device__ __forceinline__ void report_stall(uint32_t* word) {
+  *static_cast<volatile uint32_t*>(word) = 1;
+  __threadfence_system();
 }
 
 // ---- the multiplier's matrix
@@ -310,6 +322,23 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
       "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(
           smem_addr(bar))
       : "memory");
+}
+
+// The end of a launch, by the whole block: frees the tensor memory that its first warp allocated.
+// When a wait of the block ran out, products may still be under way: every warp first waits (a
+// bounded time) for what it issued, on a barrier of as many arrivals as the block has warps, and
+// the launch is reported.
+__device__ __forceinline__ void finish_launch(bool ok, uint64_t* drain, uint32_t tmem,
+                                              uint32_t cols, uint32_t* stall_word) {
+  fence_before();
+  if (!__syncthreads_and(ok)) {
+    commit(drain);
+    bool drained = true;
+    mbar_wait(drain, 0, drained);
+    if (threadIdx.x == 0) report_stall(stall_word);
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) tmem_free(tmem, cols);
 }
 
 __device__ __forceinline__ void load_sums32(uint32_t tmem, uint32_t (&r)[32]) {

@@ -40,6 +40,14 @@ cudaError_t stream_wait(cudaStream_t s);
 // thread), while the work queued on s after it runs on; mark_wait waits as stream_wait does.
 cudaError_t stream_mark(cudaStream_t s);
 cudaError_t mark_wait();
+
+// The word of pinned memory in which a kernel reports that a bounded wait for the tensor cores ran
+// out (gf_tc.cuh).  What such a launch leaves in its output is undefined and nothing tells whose it
+// was, so the report stands for the rest of the process, as a CUDA error that corrupts a context
+// does: tensor_word then refuses the launches that would be given the word, and stream_wait and
+// mark_wait return cudaErrorLaunchTimeout, which cuda_error turns into BINIUS_E_TIMEOUT.
+int tensor_word(uint32_t** word);
+bool tensor_stalled();
 void set_blocking_waits(bool on, double poll_micros = 100.0);
 
 // Device-to-host reads through a per-thread pinned staging buffer: add() notes them, wait() queues

@@ -170,12 +170,9 @@ struct NttTcShared {
   tc::MatrixRows rows[2][kTcLowTwiddles];  // of this layer's and the next one's twiddles
   uint4 twiddles[kTcTwiddles];
   uint8_t ones[tc::kOnesBytes];
-  uint64_t done[kTcGroups];
+  uint64_t done[kTcGroups], drain;
   uint32_t tmem;
 };
-
-// Set when a wait for the tensor cores ran out (a tile of that launch is then left unwritten).
-__device__ uint32_t g_ntt_tc_stalled;
 
 __device__ __forceinline__ void cp_async16(uint4* smem_dst, const uint4* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_addr(smem_dst)),
@@ -187,11 +184,12 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 
 // One layer of a tile in shared memory on the tensor cores (SLOTS: h < 7); emit(e, x) takes the
-// results.  Returns false when a wait ran out.
+// results.  `ok` becomes false when a wait runs out.
 template <bool INVERSE, bool SLOTS, class Emit>
-__device__ __forceinline__ bool ntt_tc_layer(NttTcShared& sh, const tc::MatrixRows* rows,
+__device__ __forceinline__ void ntt_tc_layer(NttTcShared& sh, const tc::MatrixRows* rows,
                                              uint32_t h, uint32_t n_mtiles, uint32_t group,
-                                             uint32_t tmem, uint32_t& phase, const Emit& emit) {
+                                             uint32_t tmem, uint32_t& phase, bool& ok,
+                                             const Emit& emit) {
   const uint32_t gt = threadIdx.x % tc::kGroupThreads;
   const uint32_t gw = tc::uniform(gt / 32);
   const uint32_t lanes = (gw * 32) << 16;
@@ -205,7 +203,6 @@ __device__ __forceinline__ bool ntt_tc_layer(NttTcShared& sh, const tc::MatrixRo
   const uint32_t ones = tc::uniform(tc::smem_addr(sh.ones));
   const uint32_t matrices = tc::uniform(tc::smem_addr(sh.matrices));
   uint32_t buf = SLOTS ? group : 2 * group;
-  bool ok = true;
 
   if (SLOTS) {  // the matrices of the layer's twiddles of blocks 1, 2, 4, ..
     if (group < row_bits) {
@@ -266,7 +263,7 @@ __device__ __forceinline__ bool ntt_tc_layer(NttTcShared& sh, const tc::MatrixRo
     tc::commit(&sh.done[group]);
   };
   auto finish = [&]() {
-    ok = tc::mbar_wait(&sh.done[group], phase) && ok;
+    tc::mbar_wait(&sh.done[group], phase, ok);
     phase ^= 1;
     tc::fence_after();
   };
@@ -320,13 +317,13 @@ __device__ __forceinline__ bool ntt_tc_layer(NttTcShared& sh, const tc::MatrixRo
     u = nu;
     v = nv;
   }
-  return ok;
 }
 
 template <bool INVERSE, bool RS>
 __global__ void __launch_bounds__(kTcThreads, 1)
     ntt_tc_pass_kernel(uint4* __restrict__ data, const uint4* __restrict__ src,
-                       const uint4* __restrict__ tw, NttPass p, uint32_t n_tiles) {
+                       const uint4* __restrict__ tw, NttPass p, uint32_t n_tiles,
+                       uint32_t* stall_word) {
   pdl_wait();
   extern __shared__ __align__(128) uint8_t tc_smem[];
   NttTcShared& sh = *reinterpret_cast<NttTcShared*>(tc_smem);
@@ -391,6 +388,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (threadIdx.x < 32) tc::tmem_alloc(&sh.tmem, kTcTmemCols);
   if (threadIdx.x == 0) {
     for (uint32_t g = 0; g < kTcGroups; g++) tc::mbar_init(&sh.done[g], 1);
+    tc::mbar_init(&sh.drain, kTcThreads / 32);
     tc::mbar_init_fence();
   }
   load_tile(blockIdx.x);
@@ -421,22 +419,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const uint32_t m = INVERSE ? (k - 1 - mm) : mm;
       const uint32_t h = c + k - 1 - m;
       const bool last = mm + 1 == k;
-      // The last layer's results go to memory at once (unless a wait ran out: then nothing more
-      // is written), and the next tile's elements come into the places that are now free.
+      // The last layer's results go to memory at once, and the next tile's elements come into the
+      // places that are now free.
       auto emit = [&](uint32_t e, uint4 x) {
         if (!last) {
           sh.tile[e] = x;
           return;
         }
         const uint64_t offset = tile_offset(e);
-        if (ok) out[offset] = x;
+        out[offset] = x;
         if (!RS && nt < n_tiles) cp_async16(sh.tile + e, next + offset);
       };
       const tc::MatrixRows* rows = sh.rows[m & 1];
       if (h >= kTcOneBit) {
-        ok = ntt_tc_layer<INVERSE, false>(sh, rows, h, n_mtiles, group, tmem, phase, emit) && ok;
+        ntt_tc_layer<INVERSE, false>(sh, rows, h, n_mtiles, group, tmem, phase, ok, emit);
       } else if (h >= kTcLowestBit) {
-        ok = ntt_tc_layer<INVERSE, true>(sh, rows, h, n_mtiles, group, tmem, phase, emit) && ok;
+        ntt_tc_layer<INVERSE, true>(sh, rows, h, n_mtiles, group, tmem, phase, ok, emit);
       } else {
         const uint4* lt = tw + ((1ull << (p.l0 + m)) - 1) + (outer_hi << m);
         for (uint32_t q = threadIdx.x; q < half; q += kTcThreads) {
@@ -460,7 +458,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         __syncthreads();
       }
     }
-    if (!ok) atomicOr(&g_ntt_tc_stalled, 1u);
     if (nt < n_tiles) {
       __syncthreads();
       if (RS) load_tile(nt);
@@ -471,9 +468,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       __syncthreads();
     }
   }
-  tc::fence_before();
-  __syncthreads();
-  if (threadIdx.x < 32) tc::tmem_free(tmem, kTcTmemCols);
+  tc::finish_launch(ok, &sh.drain, tmem, kTcTmemCols, stall_word);
 }
 
 std::vector<NttPass> plan_passes(uint32_t log_d, uint32_t skip_early, uint32_t skip_late,
@@ -548,8 +543,10 @@ int launch_tc_pass(const NttPass& p, uint4* data, const uint4* src, const uint4*
   if (int rc = ensure_smem_limit(reinterpret_cast<const void*>(kern), sizeof(NttTcShared))) return rc;
   const uint64_t n_tiles = 1ull << (p.log_d - p.k - p.c);
   if (n_tiles > 0x7fffffffull) return set_error(BINIUS_E_ARG, "ntt: buffer too large");
+  uint32_t* stall_word = nullptr;
+  if (int rc = tensor_word(&stall_word)) return rc;
   launch_pdl(kern, (unsigned)std::min<uint64_t>(n_tiles, 148), kTcThreads, sizeof(NttTcShared),
-             stream, data, src, tw, p, (uint32_t)n_tiles);
+             stream, data, src, tw, p, (uint32_t)n_tiles, stall_word);
   BGPU_LAUNCH_CHECK("ntt_tc_pass_kernel");
   count_launch();
   return BINIUS_OK;
@@ -711,6 +708,8 @@ int binius_ntt_create(int device, const void* h_basis, uint32_t log_domain, bini
   *out = nullptr;
   BGPU_ARG(log_domain >= 1 && log_domain <= 32, "log_domain must be in [1, 32]");
   if (int rc = configure_device_pool(device)) return rc;
+  uint32_t* stall_word = nullptr;  // made here rather than by the first transform
+  if (int rc = tensor_word(&stall_word)) return rc;
   const uint32_t l = log_domain;
   std::vector<std::vector<hu128>> evals;
   if (int rc = subspace_evals(h_basis, l, evals)) return rc;

@@ -40,6 +40,16 @@ uint64_t binius_launch_count(void);
  * one (BINIUS_E_OOM from the call that made it); a negative value turns injection off.  No
  * kernel is involved: the refusal happens on the host before anything is launched with it. */
 void binius_debug_fail_allocs(int64_t n_before_failure);
+/* The transforms, encodes and interleaved folds wait for the tensor cores a bounded time.  When such
+ * a wait runs out, what the launch leaves in its output is undefined, and from then on every call of
+ * the process that waits for the device or would launch such work returns BINIUS_E_TIMEOUT (as after
+ * a CUDA error that corrupts a context, nothing but a new process helps).  A program that waits for
+ * the device by itself asks here afterwards: BINIUS_OK or BINIUS_E_TIMEOUT.  No reference
+ * counterpart. */
+int binius_device_status(void);
+/* For tests: launches on `stream` a wait of a few polls that nothing completes, which is reported
+ * as above. */
+int binius_debug_tensor_wait(void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * AdditiveNTT over a GenericPreExpanded domain context.
