@@ -356,23 +356,27 @@ int load_challenges(const void* h, uint32_t n, Challenges& ch) {
 // lane-parallel kernel.
 constexpr uint64_t kCompactFoldChunks = 148ull * 256;
 
-// Challenges the host knows take the scaled form: 16 products for a coset of 16 values against 30.
-// Measured on B200, four challenges, not scaled -> scaled: 2^22 values 390 -> 143 us, 2^20 141 -> 44,
-// 2^16 13 -> 10.  (For challenges in device memory the inversion would cost what it saves.)
+// The scaled form of rounds by challenges the host knows: 16 products for a coset of 16 values
+// against 30.
 ScaledFold scaled_fold(const Challenges& ch, uint32_t n) {
   ScaledFold sf;
   memset(&sf, 0, sizeof(sf));
+  std::vector<hu128> inv(n);
+  for (uint32_t k = 0; k < n; k++) {
+    memcpy(&inv[k], &ch.r[k], 16);
+    inv[k] ^= 1;
+  }
   hu128 scale = 1;
   for (uint32_t k = 0; k < n; k++) {
-    hu128 r;
-    memcpy(&r, &ch.r[k], 16);
-    if (r == 1) {
+    if (inv[k])
+      scale = host_gf_mul(scale, inv[k]);
+    else
       sf.ones |= 1u << k;
-      continue;
-    }
-    const hu128 rho = host_gf_mul(r, host_gf_inv(r ^ 1));
+  }
+  host_gf_batch_inv(inv);
+  for (uint32_t k = 0; k < n; k++) {
+    const hu128 rho = inv[k] ? 1 ^ inv[k] : 0;  // r / (1 + r) = 1 + 1 / (1 + r)
     memcpy(&sf.rho[k], &rho, 16);
-    scale = host_gf_mul(scale, r ^ 1);
   }
   memcpy(&sf.scale, &scale, 16);
   return sf;
@@ -391,13 +395,24 @@ void launch_fold_codeword_as(const uint4* cw, uint32_t log_len, const uint4* tw,
                sf, ch, dch, out);
 }
 
+// The scaled form saves products on the GPU and costs the host an inversion of 2 us, which a call
+// on few values does not win back, and a fold by one challenge never does: it would trade a product
+// for the scaling.  Measured on B200, us a call among others, plain -> scaled: four challenges 2^16
+// values 12.6 -> 14.7, 2^17 18.8 -> 15.0, 2^18 34.5 -> 22.9; three 2^16 12.2 -> 14.2, 2^17 14.6 ->
+// 14.3, 2^18 26.4 -> 18.7; two 2^17 12.0 -> 14.1, 2^18 14.0 -> 14.2 (alone 31.2 -> 29.5), 2^19 25.8
+// -> 18.6; one 2^16 11.4 -> 13.4, 2^22 111.1 -> 111.2.  (Challenges in device memory would need the
+// inversion there.)
 template <int N>
 void launch_fold_codeword(const uint4* cw, uint32_t log_len, const uint4* tw, const Challenges& ch,
                           const uint4* dch, uint4* out, cudaStream_t s) {
-  if (dch)
-    launch_fold_codeword_as<N, false>(cw, log_len, tw, ScaledFold{}, ch, dch, out, s);
-  else
-    launch_fold_codeword_as<N, true>(cw, log_len, tw, scaled_fold(ch, N), ch, dch, out, s);
+  constexpr uint32_t kScaledLog = N == 2 ? 18 : 17;
+  if constexpr (N > 1) {
+    if (!dch && log_len >= kScaledLog) {
+      launch_fold_codeword_as<N, true>(cw, log_len, tw, scaled_fold(ch, N), ch, dch, out, s);
+      return;
+    }
+  }
+  launch_fold_codeword_as<N, false>(cw, log_len, tw, ScaledFold{}, ch, dch, out, s);
 }
 
 int launch_fold_interleaved(const void* d_codeword, uint32_t log_len, uint32_t log_batch,

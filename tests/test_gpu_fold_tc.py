@@ -52,3 +52,20 @@ def test_fold_codeword(log_len, challenges):
     ref = orc.fri_fold_codeword(tw, log_len, cw, log_len,
                                 np.array([orc.from_int(c) for c in ch], dtype=np.uint64))
     assert np.array_equal(bg.to_host(out), ref)
+
+
+@pytest.mark.parametrize("log_len", [15, 16, 17, 18])
+@pytest.mark.parametrize("challenges", [[3], [4, 1], [5, 6], [7, 0, 1], [8, 9, 3], [1, 4, 5, 6],
+                                        [7, 8, 9, 3, 4], [1, 5, 6, 7, 8, 9]])
+def test_fold_codeword_where_the_form_changes(log_len, challenges):
+    """Rounds of one product and of two, on either side of the sizes from which the first begin, for
+    one to four challenges a launch."""
+    r = np.random.default_rng(3000 + log_len)
+    cw = orc.random_elems(r, 1 << log_len)
+    ch = [c if c < 2 else orc.to_int(orc.random_elems(r, 1)[0]) for c in challenges]
+    ntt = bg.AdditiveNTT(log_len)
+    tw = orc.domain_twiddles(log_len)
+    out = bg.fold_codeword(ntt, bg.to_device(cw), ch, log_len)
+    ref = orc.fri_fold_codeword(tw, log_len, cw, log_len,
+                                np.array([orc.from_int(c) for c in ch], dtype=np.uint64))
+    assert np.array_equal(bg.to_host(out), ref)
