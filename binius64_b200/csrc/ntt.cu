@@ -8,8 +8,9 @@
 // B200 mapping: a pass fuses up to 13 consecutive layers.  One CTA owns a tile of 2^(k+c) elements
 // (k butterfly bits plus c contiguous low index bits for coalescing) resident in shared memory
 // together with the twiddles the tile needs, so each pass reads and writes HBM once with 128-bit
-// accesses.  Transforms of 2^11 elements and more multiply on the tensor cores
-// (ntt_tc_pass_kernel), smaller ones on the integer pipes (ntt_pass_kernel, up to 8 layers).  Reed-Solomon encode (reed_solomon.rs:128-201) fuses the message bit reversal
+// accesses.  Transforms of 2^11 elements and more (but for narrow ranges of layers, tc_tile_bits)
+// multiply on the tensor cores (ntt_tc_pass_kernel), others on the integer pipes (ntt_pass_kernel,
+// up to 8 layers).  Reed-Solomon encode (reed_solomon.rs:128-201) fuses the message bit reversal
 // and the 2^R-fold replication into the first pass's load: for the first pass the butterfly bits
 // are exactly the message's low index bits after reversal, so the gather stays coalesced.
 #include <algorithm>
@@ -528,10 +529,18 @@ std::vector<NttPass> plan_tc_passes(uint32_t log_d, uint32_t skip_early, uint32_
 // Measured on B200, Reed-Solomon encode / inverse transform in us, integer passes -> these:
 // 2^26 x 64 columns 17320 -> 7690, 2^24 x 16 4399 -> 2190, 2^20 x 16 265 -> 134 (tiles of 2^12:
 // 157), 2^18 x 16 99 -> 53 (2^12: 72, 2^10: 74), 2^16 x 16 70 -> 37, 2^12 x 16 36 -> 25; inverse
-// 2^22 .. 2^12 at 0.5-0.6 of the time.  At 2^11 the two meet (39 -> 34) and below it the integer
-// passes win (2^10: 24 against 28).
+// 2^22 .. 2^12 at 0.5-0.6 of the time.
+//
+// Where the butterflies stay within ten index bits (log_d - skip_early = 10, one pass of one layer a
+// bit) and up to 32 tiles of them, the integer passes are at least as fast: they spread such a tile
+// over more CTAs.  Integer against tensor-core passes, in us: 2^11 elements without the first layer
+// 19.0 and 25.7 (encodes at rate 1/2 19.2 and 25.8, 2^12 at rate 1/4 19.4 and 25.9), and without
+// the last two 20.6 and 21.0; 2^15 without the first five 24.2 and 25.9; 2^16 without the first six
+// 33.8 and 26.0.  With eleven bits they lose: 2^11 35.4 and 30.0, 2^12 without the first layer 35.1
+// and 29.8, 2^15 without the first four 40.4 and 30.1.
 uint32_t tc_tile_bits(uint32_t log_d, uint32_t skip_early, uint32_t skip_late) {
-  if (log_d < 11 || log_d == skip_early + skip_late) return 0;
+  if (log_d == skip_early + skip_late) return 0;
+  if (log_d < 16 && log_d - skip_early <= kTcMinTileBits) return 0;
   const uint32_t bits = std::min(std::max(log_d - 7, kTcMinTileBits), kTcTileBits);
   return log_d - skip_early >= bits ? bits : 0;
 }

@@ -53,3 +53,30 @@ def test_encode(log_dim, log_inv_rate, log_batch):
         bg.AdditiveNTT(n, basis=basis), bg.to_device(msg), log_batch)
     assert np.array_equal(bg.to_host(out),
                           orc.rs_encode_batch(tw, n, msg, log_dim, log_inv_rate, log_batch))
+
+
+@pytest.mark.parametrize("log_d,skip_early,skip_late", [
+    (10, 0, 1), (11, 1, 1), (11, 0, 1), (12, 2, 0), (12, 1, 0), (14, 4, 3), (15, 5, 0), (15, 4, 0),
+    (16, 6, 0), (16, 7, 0), (17, 7, 1),
+])
+def test_transforms_where_the_passes_change(log_d, skip_early, skip_late):
+    """Butterflies within ten index bits and eleven, on either side of the size from which ten take
+    the tensor-core passes, with the encode of the same layers where there is one."""
+    r = np.random.default_rng(5000 + log_d * 100 + skip_early * 10 + skip_late)
+    data = orc.random_elems(r, 1 << log_d)
+    ntt = bg.AdditiveNTT(log_d)
+    tw = orc.domain_twiddles(log_d)
+    d = bg.to_device(data)
+    ntt.forward_transform(d, skip_early, skip_late)
+    assert np.array_equal(bg.to_host(d), orc.ntt_forward(tw, log_d, data, skip_early, skip_late))
+    ntt.inverse_transform(d, skip_early, skip_late)
+    assert np.array_equal(bg.to_host(d), data)
+    if 1 <= skip_early <= 4:
+        n, dim = log_d - skip_late, log_d - skip_late - skip_early
+        basis = bg.standard_domain_rs_basis(log_d, skip_late)
+        tw = orc.domain_twiddles(n, basis=basis)
+        msg = data[:1 << (log_d - skip_early)]
+        out = bg.ReedSolomonCode(dim, skip_early).encode_batch(
+            bg.AdditiveNTT(n, basis=basis), bg.to_device(msg), skip_late)
+        assert np.array_equal(bg.to_host(out),
+                              orc.rs_encode_batch(tw, n, msg, dim, skip_early, skip_late))
