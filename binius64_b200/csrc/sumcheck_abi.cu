@@ -518,8 +518,9 @@ int binius_sumcheck_inout_create(void* d_witness, uint32_t log_len, const void* 
 
 int binius_sumcheck_destroy(binius_sumcheck* p) {
   if (!p) return BINIUS_OK;
-  // the slot and the caller's multilinears are free once the queued work is done
-  if (p->s || p->queued) cudaStreamSynchronize(p->s);
+  // the slot and the caller's multilinears, which folds write, are free once the queued work is done
+  // (a NULL stream is the default stream, which has work like any other)
+  cudaStreamSynchronize(p->s);
   return_slot(p->result);
   if (p->eq) cudaFreeAsync(p->eq, p->s);
   if (p->acc) cudaFreeAsync(p->acc, p->s);

@@ -507,7 +507,10 @@ uint32_t binius_fri_estimate_optimal_arity(uint32_t log_block_length, uint32_t d
  * first, to h_coeffs (3 elements for the degree-2 provers, 2 for InOut) and their count to
  * *n_coeffs; finish writes the multilinears' values at the challenge point (2 for the bivariate,
  * 3 for the quadratic MLE-check, 1 for InOut).  Out-of-order calls return BINIUS_E_ARG with
- * "ExpectedFold" / "ExpectedExecute" (sumcheck/error.rs).  All calls synchronize `stream`.
+ * "ExpectedFold" / "ExpectedExecute" (sumcheck/error.rs).  execute and finish return when their
+ * results are there; fold returns with its work (the bivariate's next round sums among it) queued
+ * on `stream`; destroy waits for what is queued, so that the multilinears can be freed or used on
+ * any stream after it.
  * ------------------------------------------------------------------------------------------ */
 typedef struct binius_sumcheck binius_sumcheck;
 

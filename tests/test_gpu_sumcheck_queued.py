@@ -63,3 +63,27 @@ def test_more_provers_than_slots():
         p.fold(r)
     assert p.finish() == fin
     del held
+
+
+@pytest.mark.parametrize("kind,n", [("bivariate", 1), ("bivariate", 9), ("quadratic", 6),
+                                    ("inout", 5)])
+def test_destroy_waits_on_the_default_stream(kind, n):
+    """A prover on the legacy default stream that is dropped with a fold still queued: its multilinears
+    are the caller's again when the drop returns."""
+    r = np.random.default_rng(40 + n)
+    elems = [bg.to_device(orc.random_elems(r, 1 << n)) for _ in range(3)]
+    point = ints(orc.random_elems(r, n))
+    if kind == "bivariate":
+        p = bg.BivariateProductSumcheckProver(*elems[:2], 3)
+    elif kind == "quadratic":
+        p = bg.QuadraticMleCheckProver(*elems, point, 3)
+    else:
+        p = bg.InOutCheckProver(elems[0], point[:3])
+    s = torch.cuda.default_stream()
+    assert torch.cuda.current_stream() == s and s.cuda_stream == 0
+    p.execute()
+    torch.cuda._sleep(100_000_000)  # some 50 ms of the stream ahead of the fold
+    p.fold(7)
+    assert not s.query()
+    del p
+    assert s.query()
