@@ -292,10 +292,10 @@ int make(int kind, uint32_t n_vars, void* stream, binius_sumcheck** out) {
   return BINIUS_OK;
 }
 
-// Queues the sums of a bivariate round on the 2^n_vars values left, folding to them by r first
-// when set.
-int queue_round(binius_sumcheck* p, const uint4* r) {
-  const uint64_t L = 1ull << p->n_vars;
+// Queues the sums of a bivariate round on 2^n_vars values, folding to them by r first when set;
+// *folded then tells, on failure too, whether the fold was queued.
+int queue_round(binius_sumcheck* p, uint32_t n_vars, const uint4* r, bool* folded = nullptr) {
+  const uint64_t L = 1ull << n_vars;
   p->seq++;
   if (L <= kRoundMax) {
     const unsigned grid = (unsigned)std::min<uint64_t>((2 * L + kThreads - 1) / kThreads, kRoundBlocks);
@@ -303,11 +303,13 @@ int queue_round(binius_sumcheck* p, const uint4* r) {
                                                              r ? *r : make_uint4(0, 0, 0, 0),
                                                              p->parts, p->result, p->seq);
     BGPU_LAUNCH_CHECK("bivariate_host_round_kernel");
+    if (r) *folded = true;
   } else {
     if (r) {
       if (int rc = bivariate_fold_eval(p->cols[0], p->cols[1], 2 * L,
                                        reinterpret_cast<const uint8_t*>(r), p->acc, p->s))
         return rc;
+      *folded = true;
     } else {
       if (int rc = bivariate_eval(p->cols[0], p->cols[1], L / 2, p->acc, p->s)) return rc;
     }
@@ -356,7 +358,7 @@ int do_execute(binius_sumcheck* p, int kind, void* h_coeffs, uint32_t* n_coeffs)
     hu128 y1, yinf;
     if (p->result) {
       if (!p->queued)
-        if (int rc = queue_round(p, nullptr)) return rc;
+        if (int rc = queue_round(p, p->n_vars, nullptr)) return rc;
       if (int rc = take_round(p, y1, yinf)) return rc;
     } else {
       if (int rc = bivariate_eval(p->cols[0], p->cols[1], half, p->acc, p->s)) return rc;
@@ -402,8 +404,12 @@ int do_fold(binius_sumcheck* p, int kind, const void* h_challenge) {
   uint4 rv;
   memcpy(&rv, &r, 16);
   if (kind == kBivariate && p->result && p->n_vars >= 2) {
+    // a fold that was not queued leaves the prover as it was; one that was, without its sums, has
+    // them evaluated by the next execute
+    bool folded = false;
+    if (int rc = queue_round(p, p->n_vars - 1, &rv, &folded))
+      if (!folded) return rc;
     p->n_vars--;
-    if (int rc = queue_round(p, &rv)) return rc;
     p->last = eval_poly(p->coeffs, r);
     p->have_coeffs = false;
     return clear_error();

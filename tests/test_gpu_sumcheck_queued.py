@@ -1,6 +1,8 @@
 """Bivariate rounds whose next sums are queued by fold(): against the oracle at the sizes where the
 round kernels change, for provers that run in turn, one dropped with a round in flight, and more
 provers alive than there are pinned result slots."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -87,3 +89,33 @@ def test_destroy_waits_on_the_default_stream(kind, n):
     assert not s.query()
     del p
     assert s.query()
+
+
+@pytest.mark.parametrize("n", [3, 9, 16])
+def test_fold_that_fails_leaves_the_prover_as_it_was(n):
+    """A fold whose launches are refused (its stream records a capture that has been invalidated by a
+    synchronisation, which CUDA answers with an error) can be called again afterwards."""
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        p, ch, co, fin = case(n, 700 + n)
+        assert p.execute() == co[0]
+        p.fold(ch[0])
+        assert p.execute() == co[1]
+        s.synchronize()
+        rt = ctypes.CDLL("libcudart.so.12")  # the one torch has loaded
+        stream, graph = ctypes.c_void_p(s.cuda_stream), ctypes.c_void_p()
+        assert rt.cudaStreamBeginCapture(stream, 2) == 0
+        try:
+            assert rt.cudaStreamSynchronize(stream) != 0
+            for _ in range(2):
+                with pytest.raises(bg.BiniusError):
+                    p.fold(ch[1])
+                assert p.n_vars() == n - 1
+        finally:
+            assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) != 0
+        rt.cudaGetLastError()
+        for k in range(1, n):
+            p.fold(ch[k])
+            if k + 1 < n:
+                assert p.execute() == co[k + 1]
+        assert p.finish() == fin
