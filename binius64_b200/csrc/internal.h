@@ -128,11 +128,15 @@ void prover_note_footprint(const binius_prover* P, uint64_t bytes);
 // per statement shape); standalone entry points use the defaults.
 struct Tuning {
   uint32_t tail_log = 11;          // sumcheck rounds on <= 2^tail_log elements: single-CTA tail
-  uint32_t ntt_pass_layers = 8;    // NTT layers fused per shared-memory pass (<= 8)
+  uint32_t ntt_pass_layers = 8;    // NTT layers fused per shared-memory integer pass (<= 8)
   uint32_t merkle_leaf_fuse = 8;   // Merkle leaf CTA of a tree above 2^13 leaves: 2^fuse of them
   uint32_t merkle_node_fuse = 9;   // Merkle node CTA above it: 2^fuse inputs (<= 9)
-  uint32_t ntt_tile_bits = 12;     // NTT shared-memory tile: 2^bits elements (9..12)
+  uint32_t ntt_tile_bits = 12;     // tile of those passes: 2^bits elements (9..12)
 };
+// Whether the NTT choices (the tensor-core passes have none) and the Merkle choices reach a
+// Reed-Solomon encode and a SHA-256 tree.
+bool rs_encode_is_tuned(uint32_t log_dim, uint32_t log_inv_rate, uint32_t log_batch);
+bool merkle_is_tuned(uint32_t log_leaves);
 // The calling thread's current choices (a prove sets its prover's for its duration).
 const Tuning& tuning();
 class TuningScope {

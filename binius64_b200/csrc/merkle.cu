@@ -333,6 +333,8 @@ NodeIV node_iv() {
   return iv;
 }
 
+bool merkle_is_tuned(uint32_t log_leaves) { return log_leaves > kChainMaxLog; }
+
 int merkle_commit(const void* d_elems, uint32_t log_leaves, uint32_t log_batch, void* d_nodes,
                   cudaStream_t stream) {
   BGPU_ARG(d_elems != nullptr && d_nodes != nullptr, "elems / nodes is NULL");

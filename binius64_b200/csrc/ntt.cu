@@ -625,6 +625,10 @@ int ntt_transform(const binius_ntt* ntt, void* d_data, uint32_t log_len, uint32_
 
 namespace bgpu {
 
+bool rs_encode_is_tuned(uint32_t log_dim, uint32_t log_inv_rate, uint32_t log_batch) {
+  return tc_tile_bits(log_dim + log_batch + log_inv_rate, log_inv_rate, log_batch) == 0;
+}
+
 int rs_encode_batch(const binius_ntt* ntt, const void* d_msg, uint32_t log_dim,
                     uint32_t log_inv_rate, uint32_t log_batch, void* d_codeword,
                     cudaStream_t stream) {

@@ -353,8 +353,9 @@ int binius_prover_prove(const binius_prover* P, const void* d_witness,
   return rc ? rc : clear_error();
 }
 
-// Coordinate search over the launch-shape choices: each knob in turn takes every value in its range
-// with the others at their best so far; a candidate's score is the median CUDA-event time of
+// Coordinate search over the launch-shape choices that reach this prover's launches: each such knob in
+// turn takes every value in its range with the others at their best so far (a knob that reaches none
+// stays as it is: it would be picked by the noise of the proofs' times); a candidate's score is the median CUDA-event time of
 // `reps` proofs (after one warm-up proof), the whole proof on the stream as the bench times it.
 // Every candidate's proof must equal the proof under the starting choices byte for byte (the
 // choices change no arithmetic); a difference is reported as an error and the starting choices
@@ -401,13 +402,19 @@ int binius_prover_autotune(binius_prover* P, const void* d_witness, uint32_t rep
   struct Knob {
     uint32_t Tuning::*field;
     uint32_t lo, hi;
+    bool reaches;
   };
-  const Knob knobs[5] = {{&Tuning::tail_log, 8, 12},
-                         {&Tuning::ntt_tile_bits, 10, 12},
-                         {&Tuning::ntt_pass_layers, 6, 8},
-                         {&Tuning::merkle_leaf_fuse, 6, 8},
-                         {&Tuning::merkle_node_fuse, 7, 9}};
+  // the commitment's encode and tree are the largest of a proof
+  const uint32_t log_dim = P->log_witness_elems - P->log_batch;
+  const bool ntt = rs_encode_is_tuned(log_dim, P->log_inv_rate, P->log_batch);
+  const bool trees = P->merkle_hash != kMerkleVision4 && merkle_is_tuned(log_dim + P->log_inv_rate);
+  const Knob knobs[5] = {{&Tuning::tail_log, 8, 12, true},
+                         {&Tuning::ntt_tile_bits, 10, 12, ntt},
+                         {&Tuning::ntt_pass_layers, 6, 8, ntt},
+                         {&Tuning::merkle_leaf_fuse, 6, 8, trees},
+                         {&Tuning::merkle_node_fuse, 7, 9, trees}};
   for (const Knob& k : knobs) {
+    if (!k.reaches) continue;
     for (uint32_t v = k.lo; v <= k.hi && !rc; v++) {
       if (best.*(k.field) == v) continue;
       Tuning cand = best;

@@ -316,15 +316,17 @@ int binius_prove(const binius_prover* prover, const uint64_t* h_words, size_t n_
                  void* stream);
 /* Launch-shape choices of a prover's proofs, none of which changes a result (the arithmetic is
  * exact): h5 = {tail_log: sumcheck rounds on at most 2^tail_log elements run in one single-CTA
- * kernel (8..12, default 11); ntt_pass_layers: NTT layers fused per shared-memory pass (4..8,
+ * kernel (8..12, default 11); ntt_pass_layers: NTT layers fused per integer pass (4..8,
  * default 8); merkle_leaf_fuse: a Merkle leaf CTA hashes 2^k leaves and compresses up to k layers
  * above them (5..8, default 8); merkle_node_fuse: a node CTA has 2^k inputs (5..9, default 9; both
  * for trees of more than 2^13 leaves);
- * ntt_tile_bits: an NTT pass works on tiles of 2^k elements (9..12, default 12)}.
+ * ntt_tile_bits: an integer NTT pass works on tiles of 2^k elements (9..12, default 12)}.  The two
+ * NTT choices reach the encode of a statement of up to 2^11 words; larger ones run on the tensor
+ * cores, whose passes have no choice to make.  The Merkle choices reach SHA-256 trees only.
  * No reference counterpart (the reference's rayon code has no launch shapes).  Not while a prove
  * on the prover is in flight.
- * binius_prover_autotune measures them for the prover's statement shape: coordinate search over
- * the ranges above (tail_log 8..12, tile 10..12, ntt 6..8, leaf 6..8, node 7..9), each candidate
+ * binius_prover_autotune measures those that reach the prover's launches, for its statement shape,
+ * and leaves the others as they are: coordinate search over the ranges above (tail_log 8..12, tile 10..12, ntt 6..8, leaf 6..8, node 7..9), each candidate
  * scored by the median CUDA-event time of `reps` whole proofs of d_witness on `stream` after a
  * warm-up proof, every candidate's proof checked byte for byte against the first one
  * (BINIUS_E_CUDA if one differs; the prover keeps its choices).  The winner is kept by the

@@ -124,3 +124,36 @@ def test_launch_shapes_change_no_bytes_and_autotune():
     p2 = bg.Prover(bg.DeviceConstraintSystem(sc.cs.serialize()), 1)
     assert p2.tuning() == best
     assert p2.prove(w).finalize() == ref
+
+
+@pytest.mark.parametrize("log_words,n_and,n_mul,reached", [
+    (10, 700, 2, {"ntt_pass_layers", "ntt_tile_bits"}),       # integer passes, one small tree
+    (13, 6000, 2, set()),                                      # tensor-core passes, small trees
+    (18, 120_000, 5, {"merkle_leaf_fuse", "merkle_node_fuse"}),  # a tree of 2^14 leaves
+])
+def test_launch_shapes_where_they_reach(log_words, n_and, n_mul, reached):
+    """The NTT and Merkle choices at statements whose launches they shape give the oracle's proof, and
+    the autotuner leaves those that shape none as they were set."""
+    sc = csm.synthetic_circuit(log_words, n_and, n_mul, seed=77 + log_words, log_public=2)
+    prep = sc.cs.prepared()
+    orc.set_threads(8)
+    try:
+        ref = orc.prove(sc.witness, 2, prep.and_csr, prep.mul_csr, 1)
+    finally:
+        orc.set_threads(1)
+    p = bg.Prover(bg.DeviceConstraintSystem(sc.cs.serialize()), 1)
+    w = torch.from_numpy(sc.witness.view(np.int64)).cuda()
+    default = p.tuning()
+    values = {"ntt_pass_layers": (4, 5, 7), "ntt_tile_bits": (9, 10, 11),
+              "merkle_leaf_fuse": (5, 6, 7), "merkle_node_fuse": (5, 6, 8)}
+    for knob in sorted(reached):
+        for v in values[knob]:
+            p.set_tuning(**{knob: v})
+            assert p.prove(w).finalize() == ref, (knob, v)
+            p.set_tuning(**default)
+    start = {"ntt_pass_layers": 5, "ntt_tile_bits": 9, "merkle_leaf_fuse": 5, "merkle_node_fuse": 6}
+    p.set_tuning(**start)
+    best = p.autotune(w, reps=1)
+    assert {k: best[k] for k in start if k not in reached} == \
+        {k: v for k, v in start.items() if k not in reached}
+    assert p.prove(w).finalize() == ref
