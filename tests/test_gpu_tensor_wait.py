@@ -38,11 +38,11 @@ prover = bg.Prover(cs, 1)
 words = torch.from_numpy(circ.witness.view(np.int64)).cuda()
 ntt = bg.AdditiveNTT(11)
 data = torch.zeros((1 << 11, 2), dtype=torch.int64, device="cuda")
-small = bg.AdditiveNTT(5)
+small, wide = bg.AdditiveNTT(5), bg.AdditiveNTT(12)
 calls = {
     "transform": lambda: ntt.forward_transform(data),
     "inverse": lambda: ntt.inverse_transform(data),
-    "encode": lambda: bg.ReedSolomonCode(10, 1).encode_batch(ntt, data[:1 << 10], 0),
+    "encode": lambda: bg.ReedSolomonCode(11, 1).encode_batch(wide, data, 0),
     "fold": lambda: bg.fold_interleaved(data, [3, 5], 9, 2),
     "prove": lambda: prover.prove(words),
     "prove_host": lambda: prover.prove_host(circ.witness),
