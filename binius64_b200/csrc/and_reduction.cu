@@ -484,17 +484,16 @@ __global__ void __launch_bounds__(kFsThreads)
   pdl_trigger();
   __shared__ FsShared fs;
   FsStep st;
-  if (threadIdx.x < 32) st.begin(fs, ts);
-  __syncthreads();
   if (threadIdx.x >= 32) {
-    fs_help(fs, fs.slow);
+    fs_help(fs);
     return;
   }
+  st.begin(fs, ts);
   const uint4 y1 = ys[0], yinf = ys[1];
   const uint4 y0 = gf_mul_warp(gf_add(*claim, gf_mul_warp(y1, rc->alpha)), rc->inv_one_plus_alpha);
   const uint4 c0 = y0, c2 = yinf, c1 = gf_add(gf_add(y1, c0), c2);
   const uint4 msg[2] = {c1, c2};
-  const uint4 r = st.step(fs, ts, tape, msg, 2, fs.slow);
+  const uint4 r = st.step(fs, tape, msg, 2);
   *r_out = r;
   *claim = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
   st.end(fs, ts);
@@ -523,7 +522,6 @@ __global__ void __launch_bounds__(kAndTailThreads)
     r_sh = *r_first;
   }
   __syncthreads();
-  const bool slow = fs.slow;
   // warp 0, beside the folds: the claim after the last challenge, and what of the round's
   // interpolation y_0 = (claim + alpha y_1) / (1 + alpha) does not wait for the sums
   uint4 c0 = gf_zero(), c1 = gf_zero(), c2 = gf_zero(), rr = gf_zero();
@@ -568,11 +566,11 @@ __global__ void __launch_bounds__(kAndTailThreads)
       c2 = yinf;
       c1 = gf_add(gf_add(y1, c0), c2);
       const uint4 msg[2] = {c1, c2};
-      rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
+      rr = st.step(fs, tape, msg, 2);
       chal[k] = rr;
       r_sh = rr;
     } else {
-      fs_help(fs, slow && k == 0);
+      fs_help(fs);
     }
     __syncthreads();
   }

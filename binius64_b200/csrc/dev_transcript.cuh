@@ -26,9 +26,7 @@ namespace bgpu {
 // latency and every logic instruction takes the warp's 16-lane pipe for two cycles.  Measured on a
 // B200, one warp: the multiply below 0.13 us (a 32x32 carry-less product per lane and eight warp
 // reductions: 0.37 us; one thread: 0.67 us); a SHA-256 compression fully unrolled on registers 1.5
-// us.  The steps of a stretch run as FsStep below (2.4 us for message and challenge) where the
-// transcript is in its usual state, else as DevTr (4.9 us).
-__device__ __forceinline__ uint4 gf_mul_1t(uint4 a, uint4 b) { return gf_mul_nl(a, b); }
+// us.  The steps of a stretch run as FsStep below (2.4 us for message and challenge).
 
 // A product on the critical path of a Fiat-Shamir step, computed by a whole warp.  One out-of-line
 // copy keeps the code of the launches that call it small.
@@ -48,11 +46,11 @@ static __device__ __noinline__ void sha256_compress_1t(uint32_t* st, const uint3
   for (int i = 0; i < 8; i++) st[i] = s[i];
 }
 
-// The challenger held by the warp that advances it.  The partial SHA-256 block is kept as 16
-// big-endian words, the sample buffer as 8 little-endian words; absorbing a word is one store at
-// a run-time index (the arrays live in local memory, which the out-of-line compression copies to
-// registers), so the code around the compression stays small.  The stream is
-// absorbed in 4-byte pieces (every message of the protocol is a whole number of words); a piece
+// The challenger held by a thread that adds a message without a challenge after it.  The partial
+// SHA-256 block is kept as 16 big-endian words, the sample buffer as 8 little-endian words;
+// absorbing a word is one store at a run-time index (the arrays live in local memory, which the
+// out-of-line compression copies to registers), so the code around the compression stays small.  The
+// stream is absorbed in 4-byte pieces (every message of the protocol is a whole number of words); a piece
 // may start at any byte offset.  Words at or past `len` hold no meaning except that a partially
 // filled word is zero past its bytes.
 struct DevTr {
@@ -116,24 +114,6 @@ struct DevTr {
     }
   }
 
-  // Digest of the stream (FIPS 180-4 padding) as 8 big-endian words; the stream is unchanged.
-  __device__ __noinline__ void digest(uint32_t d[8]) const {
-    uint32_t st[8], m[16];
-    for (int i = 0; i < 8; i++) st[i] = h[i];
-    const uint32_t full = len >> 2, part = len & 3u;
-    for (uint32_t i = 0; i < 16; i++) m[i] = (i < full || (i == full && part)) ? w[i] : 0u;
-    m[full] |= 0x80u << (24 - 8 * part);
-    const uint64_t bits = total * 8;
-    if (len + 9 > 64) {
-      compress(st, m);
-      for (int i = 0; i < 16; i++) m[i] = 0;
-    }
-    m[14] = (uint32_t)(bits >> 32);
-    m[15] = (uint32_t)bits;
-    compress(st, m);
-    for (int i = 0; i < 8; i++) d[i] = st[i];
-  }
-
   __device__ __forceinline__ void to_observer() {
     if (sampling) {
       const uint32_t idx = index;
@@ -149,8 +129,7 @@ struct DevTr {
       error = 1;
       return;
     }
-    if (threadIdx.x & 31) {  // a warp advancing the transcript together writes from lane 0
-    } else if ((tape_len & 3u) == 0) {
+    if ((tape_len & 3u) == 0) {
       uint32_t* t32 = reinterpret_cast<uint32_t*>(tape + tape_len);
       for (uint32_t i = 0; i < n; i++) t32[i] = v[i];
     } else {
@@ -180,90 +159,24 @@ struct DevTr {
       }
     }
   }
-  __device__ __forceinline__ void message_elems(uint8_t* tape, const uint4* e, uint32_t n) {
-    message_words(tape, reinterpret_cast<const uint32_t*>(e), 4 * n);
-  }
-  __device__ __forceinline__ void observe_words(const uint32_t* v, uint32_t n) {
-    to_observer();
-    for (uint32_t i = 0; i < n; i++) absorb_word(v[i]);
-  }
-
-  // Refills the sample buffer from the digest of the stream, which restarts as that digest.
-  __device__ __noinline__ void refill() {
-    uint32_t d[8];
-    digest(d);
-    const uint32_t iv[8] = {0x6a09e667u, 0xbb67ae85u, 0x3c6ef372u, 0xa54ff53au,
-                            0x510e527fu, 0x9b05688cu, 0x1f83d9abu, 0x5be0cd19u};
-    for (int i = 0; i < 8; i++) {
-      h[i] = iv[i];
-      w[i] = d[i];
-      buf[i] = bswap32(d[i]);
-    }
-    len = 32;
-    total = 32;
-    index = 0;
-  }
-
-  __device__ __forceinline__ void begin_sampling() {
-    if (!sampling) {
-      sampling = 1;
-      index = 32;
-    }
-  }
-
-  // n bytes as little-endian words out[(n + 3) / 4].
-  __device__ __forceinline__ void sample_words(uint32_t* out, uint32_t n) {
-    begin_sampling();
-    for (uint32_t i = 0; i < (n + 3) / 4; i++) out[i] = 0;
-    for (uint32_t i = 0; i < n; i++) {
-      if (index == 32) refill();
-      out[i >> 2] |= ((buf[index >> 2] >> (8 * (index & 3u))) & 255u) << (8 * (i & 3u));
-      index++;
-    }
-  }
-
-  // A field element: 16 bytes read as a little-endian u128 (transcript.rs:398-407).
-  __device__ __forceinline__ uint4 sample_elem() {
-    begin_sampling();
-    if (index == 32) refill();
-    if ((index & 3u) == 0 && index + 16 <= 32) {
-      const uint32_t k = index >> 2;
-      index += 16;
-      return make_uint4(buf[k], buf[k + 1], buf[k + 2], buf[k + 3]);
-    }
-    uint32_t o[4];
-    sample_words(o, 16);
-    return make_uint4(o[0], o[1], o[2], o[3]);
-  }
-
-  // sample_bits_reader (fiat_shamir/sampling.rs:34-50): a little-endian u32, masked.
-  __device__ __forceinline__ uint32_t sample_bits(uint32_t bits) {
-    uint32_t v;
-    sample_words(&v, 4);
-    return bits >= 32 ? v : v & ((1u << bits) - 1);
-  }
 };
-
 
 // A round's Fiat-Shamir step, message() of n elements then sample(), by three warps of a block.
 //
-// Between the rounds of a stretch the transcript is nearly always in one state: it has just been
-// sampled, so the SHA-256 stream holds the 32 bytes of the last digest and nothing else.  From
-// there a step absorbs those, 8 bytes for the return to observing and the message, and digests
+// Between the rounds of a stretch the transcript is in one state: it has just been sampled, so the
+// SHA-256 stream holds the 32 bytes of the last digest and nothing else.  From there a step absorbs those, 8 bytes for the return to observing and the message, and digests
 // the padded stream: two blocks, whose words are all known before the first compression.  Warp 0
 // lays the words out (one per lane) and runs the 64 + 64 rounds; warps 1 and 2, on other
 // schedulers, expand the two message schedules meanwhile and hand them over through shared memory
 // with the round constants added.  A compression on one warp is bound by that warp's logic pipe
 // (1376 instructions of two cycles); without the schedules 900 are left.  Measured, one step:
-// 2.4 us against 4.9 us with DevTr; a 2^12-word proof 2.55 -> 2.20 ms, one of 2^18 words and 256
+// 2.4 us against 4.9 us on one warp; a 2^12-word proof 2.55 -> 2.20 ms, one of 2^18 words and 256
 // multiplications 5.30 -> 4.46 ms, one of 2^20 words 3.04 -> 2.78 ms (with the multiply above).
-// From any other state (a stretch that begins before the host has sampled; none of the protocol's
-// does) the first step runs as DevTr.
+// A stretch begins in that state: DeviceTranscript::check has the host sample first.
 constexpr uint32_t kFsThreads = 96;  // warps 0, 1 and 2 take part
 struct __align__(16) FsShared {
   uint32_t words[32];   // the stream's two padded blocks; between steps the digest in 0..7
   uint32_t kw[2][64];   // their schedules plus round constants
-  uint32_t slow;        // not in the usual state (set by FsStep::begin)
 };
 
 // Named barriers of a step; 0 is __syncthreads.
@@ -353,7 +266,6 @@ struct FsStep {
   uint32_t k16;  // round constant lane mod 16
   uint32_t index, tape_len, tape_cap, error;
 
-  // Before a barrier of the block, after which every warp reads sh.slow.
   __device__ __forceinline__ void begin(FsShared& sh, const TranscriptState* g) {
     const uint32_t lane = threadIdx.x & 31;
     k16 = kSha256K[lane & 15];
@@ -362,30 +274,10 @@ struct FsStep {
     tape_cap = g->tape_cap;
     error = g->error;
     if (lane < 8) sh.words[lane] = g->w[lane];
-    if (lane == 0)
-      sh.slow = !(g->block_len == 32 && g->total == 32 && g->sampling && (tape_len & 3u) == 0);
   }
 
-  // The step from a state that is not the usual one: the transcript as begin() found it.
-  __device__ __noinline__ uint4 step_slow(FsShared& sh, const TranscriptState* g, uint8_t* tape,
-                                          const uint4* msg, uint32_t n) {
-    DevTr st;
-    st.load(g);
-    st.message_elems(tape, msg, n);
-    const uint4 r = st.sample_elem();
-    if ((threadIdx.x & 31) == 0)
-      for (int i = 0; i < 8; i++) sh.words[i] = st.w[i];
-    index = st.index;
-    tape_len = st.tape_len;
-    error = st.error;
-    __syncwarp();
-    return r;
-  }
-
-  // n <= 4 elements.  `slow` (the block's first step, when sh.slow was set): fs_help does nothing.
-  __device__ __forceinline__ uint4 step(FsShared& sh, const TranscriptState* g, uint8_t* tape,
-                                        const uint4* msg, uint32_t n, bool slow) {
-    if (slow) return step_slow(sh, g, tape, msg, n);
+  // n <= 4 elements.
+  __device__ __forceinline__ uint4 step(FsShared& sh, uint8_t* tape, const uint4* msg, uint32_t n) {
     const uint32_t lane = threadIdx.x & 31;
     if (lane == 0) {
 #pragma unroll
@@ -458,9 +350,9 @@ struct FsStep {
 };
 
 // The other warps of the block during a step.
-__device__ __forceinline__ void fs_help(FsShared& sh, bool slow) {
+__device__ __forceinline__ void fs_help(FsShared& sh) {
   const uint32_t warp = threadIdx.x / 32;
-  if (!slow && (warp == 1 || warp == 2)) fs_schedule(sh, warp - 1);
+  if (warp == 1 || warp == 2) fs_schedule(sh, warp - 1);
 }
 
 // The products of a small sumcheck round in one block: job(j, mul, own) for j < n, on threads
@@ -497,6 +389,8 @@ class DeviceTranscript {
     size_t bytes;
   };
   int begin(const Transcript& t, cudaStream_t s, std::initializer_list<Upload> uploads = {});
+  // A state that FsStep can go on from: just sampled (the stream is the last digest, 32 bytes).
+  static int check(const TranscriptState& st);
   TranscriptState* state() const { return reinterpret_cast<TranscriptState*>(mem_); }
   uint8_t* tape() const { return mem_ + kStateBytes; }
   // message() of n_bytes (a multiple of 4, 4-byte aligned) that are in device memory.

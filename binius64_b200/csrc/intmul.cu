@@ -434,14 +434,14 @@ __global__ void __launch_bounds__(kImFinishThreads)
   }
   block_xor_sum<4>(acc);
   if (threadIdx.x < 32) {
-    const uint4 r = st.step(fs, ts, tape, acc, msg_coeffs, fs.slow);
+    const uint4 r = st.step(fs, tape, acc, msg_coeffs);
     if (threadIdx.x == 0) {
       *r_out = r;
       s_r = r;
     }
     st.end(fs, ts);
   } else {
-    fs_help(fs, fs.slow);
+    fs_help(fs);
   }
   __syncthreads();
   const uint4 r = s_r;
@@ -540,12 +540,11 @@ __global__ void __launch_bounds__(kFsThreads)
   pdl_trigger();
   __shared__ FsShared fs;
   FsStep st;
-  if (threadIdx.x < 32) st.begin(fs, &ls->a.ts);
-  __syncthreads();
   if (threadIdx.x >= 32) {
-    fs_help(fs, fs.slow);
+    fs_help(fs);
     return;
   }
+  st.begin(fs, &ls->a.ts);
   const ImAlpha al = ls->a.alphas[t];
   const uint4 y1 = ls->y[t][0], yinf = ls->y[t][1], pf = ls->prefix;
   uint4 oma = al.alpha;
@@ -556,7 +555,7 @@ __global__ void __launch_bounds__(kFsThreads)
   const uint4 T1 = gf_add(gf_add(y1, T0), yinf), T2 = yinf;
   const uint4 m[3] = {gf_mul_warp(po, T0), gf_add(gf_mul_warp(po, T1), gf_mul_warp(pf, T0)),
                       gf_add(gf_mul_warp(po, T2), gf_mul_warp(pf, T1))};
-  const uint4 r = st.step(fs, &ls->a.ts, tape, m, 3, fs.slow);
+  const uint4 r = st.step(fs, tape, m, 3);
   ls->chal[t] = r;
   ls->a.G = gf_add(T0, gf_mul_warp(r, gf_add(T1, gf_mul_warp(r, T2))));
   uint4 f = gf_add(r, al.alpha);
@@ -619,7 +618,6 @@ __global__ void __launch_bounds__(kImTailThreads)
       __syncthreads();
     }
   }
-  const bool slow = fs.slow;
   uint4 T0 = gf_zero(), T1 = gf_zero(), T2 = gf_zero(), rr = gf_zero();
   for (uint32_t t = t0; t < n; t++) {
     const bool fold = t > 0;
@@ -678,11 +676,11 @@ __global__ void __launch_bounds__(kImTailThreads)
       const uint4 m[3] = {gf_mul_warp(po, T0),
                           gf_add(gf_mul_warp(po, T1), gf_mul_warp(pf, T0)),
                           gf_add(gf_mul_warp(po, T2), gf_mul_warp(pf, T1))};
-      rr = st.step(fs, &ts_sh, tape, m, 3, slow && t == t0);
+      rr = st.step(fs, tape, m, 3);
       if (threadIdx.x == 0) res->chal[t] = rr;
       r_sh = rr;
     } else {
-      fs_help(fs, slow && t == t0);
+      fs_help(fs);
     }
     __syncthreads();
   }
@@ -736,7 +734,6 @@ __global__ void __launch_bounds__(kImTailThreads)
     }
     __syncthreads();
   }
-  const bool slow = fs.slow;
   uint4 T[2][3] = {}, rr = gf_zero();
   for (uint32_t t = t0; t < n; t++) {
     const bool fold = t > 0;
@@ -815,11 +812,11 @@ __global__ void __launch_bounds__(kImTailThreads)
         gf_add_into(m3[1], gf_add(gf_mul_warp(po[g], T[g][1]), gf_mul_warp(pf[g], T[g][0])));
         gf_add_into(m3[2], gf_add(gf_mul_warp(po[g], T[g][2]), gf_mul_warp(pf[g], T[g][1])));
       }
-      rr = st.step(fs, ts, tape, m3, 3, slow && t == t0);
+      rr = st.step(fs, tape, m3, 3);
       chal[t] = rr;
       r_sh = rr;
     } else {
-      fs_help(fs, slow && t == t0);
+      fs_help(fs);
     }
     __syncthreads();
   }
@@ -1082,6 +1079,7 @@ int IntMulDevice::layer(uint4* set, uint32_t pairs, std::vector<hu128>& point,
   LayerArgs a;
   memset(&a, 0, sizeof(a));
   t_.save(a.ts);
+  if (int rc = DeviceTranscript::check(a.ts)) return rc;
   a.ts.tape_cap = 48 * n;
   a.pairs = pairs;
   a.n = n;

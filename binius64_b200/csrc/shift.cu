@@ -392,12 +392,11 @@ __global__ void __launch_bounds__(kFsThreads)
   pdl_trigger();
   __shared__ FsShared fs;
   FsStep st;
-  if (threadIdx.x < 32) st.begin(fs, ts);
-  __syncthreads();
   if (threadIdx.x >= 32) {
-    fs_help(fs, fs.slow);
+    fs_help(fs);
     return;
   }
+  st.begin(fs, ts);
   {
     const ShiftRoundConst c = *rc;
     uint4 inout = st3[1];
@@ -420,7 +419,7 @@ __global__ void __launch_bounds__(kFsThreads)
     const uint4 d0 = gf_mul_warp(gf_mul_warp(q0, one_a), eqp);
     const uint4 d1 = gf_mul_warp(gf_add(gf_mul_warp(q1, one_a), q0), eqp);
     const uint4 msg[2] = {gf_add(s0, gf_mul_warp(beta, d0)), gf_add(s1, gf_mul_warp(beta, d1))};
-    const uint4 r = st.step(fs, ts, tape, msg, 2, fs.slow);
+    const uint4 r = st.step(fs, tape, msg, 2);
     *r_out = r;
     st3[0] = gf_add(s0, gf_mul_warp(r, gf_add(s1, gf_mul_warp(s2, r))));
     st3[1] = gf_add(q0, gf_mul_warp(q1, r));
@@ -459,7 +458,6 @@ __global__ void __launch_bounds__(kShiftTailThreads)
     r_sh = *r_first;
   }
   __syncthreads();
-  const bool slow = fs.slow;
   uint4 s0 = gf_zero(), s1 = gf_zero(), s2 = gf_zero(), q0 = gf_zero(), q1 = gf_zero();
   uint4 rr = gf_zero(), alpha = gf_zero();
   auto next_state = [&]() {  // warp 0: the running sums after the last challenge
@@ -542,11 +540,11 @@ __global__ void __launch_bounds__(kShiftTailThreads)
       const uint4 msg[2] = {
           gf_add(s0, gf_mul_warp(k1, q0)),
           gf_add(s1, gf_add(gf_mul_warp(k1, q1), gf_mul_warp(k0, q0)))};
-      rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
+      rr = st.step(fs, tape, msg, 2);
       chal[k] = rr;
       r_sh = rr;
     } else {
-      fs_help(fs, slow && k == 0);
+      fs_help(fs);
     }
     __syncthreads();
   }

@@ -308,12 +308,11 @@ __global__ void __launch_bounds__(kFsThreads)
   pdl_trigger();
   __shared__ FsShared fs;
   FsStep st;
-  if (threadIdx.x < 32) st.begin(fs, ts);
-  __syncthreads();
   if (threadIdx.x >= 32) {
-    fs_help(fs, fs.slow);
+    fs_help(fs);
     return;
   }
+  st.begin(fs, ts);
   const uint4 y1 = ys[0], yinf = ys[1];
   const uint4 c0 = gf_add(claim_init ? *claim_init : *claim, y1), c2 = yinf;
   const uint4 c1 = gf_add(gf_add(y1, c0), c2);
@@ -324,7 +323,7 @@ __global__ void __launch_bounds__(kFsThreads)
     msg[2] = make_uint4(root[0], root[1], root[2], root[3]);
     msg[3] = make_uint4(root[4], root[5], root[6], root[7]);
   }
-  const uint4 r = st.step(fs, ts, tape, msg, commitment ? 4 : 2, fs.slow);
+  const uint4 r = st.step(fs, tape, msg, commitment ? 4 : 2);
   *r_out = r;
   *claim = gf_add(c0, gf_mul_warp(r, gf_add(c1, gf_mul_warp(c2, r))));
   st.end(fs, ts);
@@ -353,7 +352,6 @@ __global__ void __launch_bounds__(kTailThreads)
     if (r_first) r_sh = *r_first;
   }
   __syncthreads();
-  const bool slow = fs.slow;
   uint4 c0 = gf_zero(), c1 = gf_zero(), c2 = gf_zero(), rr = gf_zero();
   auto next_claim = [&]() {  // warp 0: the claim after round k - 1's challenge
     cl = gf_add(c0, gf_mul_warp(rr, gf_add(c1, gf_mul_warp(c2, rr))));
@@ -391,11 +389,11 @@ __global__ void __launch_bounds__(kTailThreads)
       c2 = yinf;
       c1 = gf_add(gf_add(y1, c0), c2);
       const uint4 msg[2] = {c0, c1};
-      rr = st.step(fs, ts, tape, msg, 2, slow && k == 0);
+      rr = st.step(fs, tape, msg, 2);
       chal[k] = rr;
       r_sh = rr;
     } else {
-      fs_help(fs, slow && k == 0);
+      fs_help(fs);
     }
     __syncthreads();
   }

@@ -57,12 +57,18 @@ DeviceTranscript::~DeviceTranscript() {
   if (mem_) dev_free(mem_, s_);
 }
 
+int DeviceTranscript::check(const TranscriptState& st) {
+  if (st.sampling && st.block_len == 32 && st.total == 32 && st.tape_len == 0) return BINIUS_OK;
+  return set_error(BINIUS_E_ARG, "a device stretch begins when the transcript has been sampled");
+}
+
 int DeviceTranscript::begin(const Transcript& t, cudaStream_t s,
                             std::initializer_list<Upload> uploads) {
   s_ = s;
   if (!mem_) BGPU_CUDA(dev_alloc(reinterpret_cast<void**>(&mem_), kStateBytes + kTapeCap, s));
   LoadArgs a;
   t.save(a.st);
+  if (int rc = check(a.st)) return rc;
   a.st.tape_cap = kTapeCap;
   a.dst = state();
   uint32_t n = 0, used = 0;
