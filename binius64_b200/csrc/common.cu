@@ -211,6 +211,16 @@ __global__ void __launch_bounds__(kGatherThreads) gather_reads_kernel(GatherSegm
 
 StagedReads::StagedReads(cudaStream_t s) : s_(s) {}
 
+StagedReads::~StagedReads() {
+  if (written_) cudaStreamSynchronize(s_);
+}
+
+int StagedReads::pinned(size_t bytes, uint8_t** at) {
+  if (int rc = reserve(bytes, at)) return rc;
+  written_ = written_ || *at;
+  return BINIUS_OK;
+}
+
 int StagedReads::reserve(size_t bytes, uint8_t** at) {
   *at = nullptr;
   const size_t need = used_ + ((bytes + 15) & ~size_t(15));
@@ -252,6 +262,7 @@ int StagedReads::copy(const Pending& p, size_t dpitch) {
 
 // Queues the reads: small pieces in launches of kGatherSegments, a large or a lone one as a copy.
 int StagedReads::queue() {
+  written_ = written_ || !pending_.empty();
   GatherSegments g;
   uint32_t n = 0;
   const Pending* lone = nullptr;
@@ -281,6 +292,7 @@ int StagedReads::queue() {
 int StagedReads::wait() {
   if (int rc = queue()) return rc;
   BGPU_CUDA(stream_wait(s_));
+  written_ = false;
   for (const auto& p : pending_)
     for (size_t r = 0; r < p.height; r++)
       memcpy(static_cast<uint8_t*>(p.dst) + r * p.dpitch, p.stage + r * p.width, p.width);

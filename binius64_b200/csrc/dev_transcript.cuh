@@ -325,7 +325,7 @@ struct FsStep {
     return make_uint4(bswap32(s[0]), bswap32(s[1]), bswap32(s[2]), bswap32(s[3]));
   }
 
-  // After at least one step.
+  // After at least one step.  Writes every field but tape_cap.
   __device__ __forceinline__ void end(const FsShared& sh, TranscriptState* g) const {
     const uint32_t lane = threadIdx.x & 31;
     if (lane < 8) {
@@ -335,9 +335,9 @@ struct FsStep {
 #pragma unroll
       for (int i = 1; i < 8; i++) v = lane == (uint32_t)i ? iv[i] : v;
       g->h[lane] = v;
-      g->w[lane] = sh.words[lane];
       g->buf[lane] = bswap32(sh.words[lane]);
     }
+    if (lane < 16) g->w[lane] = lane < 8 ? sh.words[lane] : 0u;
     if (lane == 0) {
       g->block_len = 32;
       g->total = 32;

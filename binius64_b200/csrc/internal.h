@@ -52,16 +52,21 @@ void set_blocking_waits(bool on, double poll_micros = 100.0);
 
 // Device-to-host reads through a per-thread pinned staging buffer: add() notes them, wait() queues
 // them on the stream (small ones together as one launch, which writes the stage), synchronises once
-// and scatters them to their destinations.  The sources stay as they are from add() to wait().
+// and scatters them to their destinations.  The sources stay as they are from add() to wait().  A
+// thread has one at a time: each starts at the stage's front, so one that ends before its wait() has
+// returned (a call that failed on the way) first waits for what may still write the stage.
 class StagedReads {
  public:
   explicit StagedReads(cudaStream_t s);
+  ~StagedReads();
+  StagedReads(const StagedReads&) = delete;
+  StagedReads& operator=(const StagedReads&) = delete;
   int add(void* dst, const void* src, size_t bytes);
   int add2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width,
             size_t height);
   // Pinned memory that kernels on the stream write themselves (its device address is the same),
   // valid from wait() until the thread's next reads; nullptr when the stage has no room.
-  int pinned(size_t bytes, uint8_t** at) { return reserve(bytes, at); }
+  int pinned(size_t bytes, uint8_t** at);
   int wait();
 
  private:
@@ -76,6 +81,7 @@ class StagedReads {
   int queue();
   cudaStream_t s_;
   size_t used_ = 0;
+  bool written_ = false;  // work that writes the stage is queued, or may be
   std::vector<Pending> pending_;
 };
 

@@ -1126,10 +1126,8 @@ int IntMulDevice::layer(uint4* set, uint32_t pairs, std::vector<hu128>& point,
   const LayerResult* res = reinterpret_cast<const LayerResult*>(result);
   if (res->ts.error || res->ts.tape_len != 48 * n)
     return set_error(BINIUS_E_CUDA, "device transcript wrote an unexpected number of bytes");
-  // the tail leaves the fields it does not own as they were handed over
-  TranscriptState ts = res->ts;
-  ts.tape_cap = a.ts.tape_cap;
-  t_.load(ts, result + kLayerTape);
+  // (the tail writes every field of the state but tape_cap, which only the device reads)
+  t_.load(res->ts, result + kLayerTape);
   std::vector<hu128> evals(2 * pairs);
   memcpy(evals.data(), result + kLayerTape + 48 * n, 32 * pairs);
   point.resize(n);

@@ -157,3 +157,28 @@ def test_launch_shapes_where_they_reach(log_words, n_and, n_mul, reached):
     assert {k: best[k] for k in start if k not in reached} == \
         {k: v for k, v in start.items() if k not in reached}
     assert p.prove(w).finalize() == ref
+
+
+@pytest.mark.parametrize("n_mul", [1, 40])
+def test_proof_after_one_that_failed(n_mul):
+    """A proof that ends early, here at each of its allocations in turn, leaves nothing behind that the
+    thread's next proof meets."""
+    from binius64_b200._ffi import lib as ffi_lib
+    sc = csm.synthetic_circuit(11, 1500, n_mul, seed=5, log_public=2)
+    prep = sc.cs.prepared()
+    ref = orc.prove(sc.witness, 2, prep.and_csr, prep.mul_csr, 1)
+    p = bg.Prover(bg.DeviceConstraintSystem(sc.cs.serialize()), 1)
+    w = torch.from_numpy(sc.witness.view(np.int64)).cuda()
+    failed = 0
+    for allowed in range(0, 400):
+        ffi_lib().binius_debug_fail_allocs(allowed)
+        try:
+            p.prove(w)
+        except bg.OutOfMemoryError:
+            failed += 1
+        else:
+            break
+        finally:
+            ffi_lib().binius_debug_fail_allocs(-1)
+        assert p.prove(w).finalize() == ref, allowed
+    assert failed > 10 and p.prove(w).finalize() == ref
