@@ -162,37 +162,22 @@ void put_elem(uint32_t* w, hu128 v) {
   for (int i = 0; i < 4; i++) w[i] = (uint32_t)(v >> (32 * i));
 }
 
-// The shared-memory image, uploaded once per device.
-int device_image(const uint4** out) {
-  static std::mutex mu;
-  static const uint4* images[64] = {};
-  int dev = 0;
-  BGPU_CUDA(cudaGetDevice(&dev));
-  BGPU_ARG(dev >= 0 && dev < 64, "device ordinal out of range");
-  std::lock_guard<std::mutex> g(mu);
-  if (!images[dev]) {
-    const HostParams& p = host_params();
-    std::vector<uint32_t> img(kImageBytes / 4, 0);
-    for (uint32_t m = 0; m < kMaps; m++)
-      for (uint32_t pos = 0; pos < 32; pos++)
-        for (uint32_t nib = 0; nib < 16; nib++) {
-          hu128 v = 0;
-          for (int b = 0; b < 4; b++)
-            if ((nib >> b) & 1) v ^= p.cols[m][4 * pos + b];
-          for (int plane = 0; plane < 4; plane++)
-            img[m * kMapWords + plane * 512 + pos * 16 + nib] = (uint32_t)(v >> (32 * plane));
-        }
-    for (int r = 0; r < 17; r++)
-      for (int i = 0; i < 4; i++) put_elem(&img[4 * (kRcOff + 4 * r + i)], p.rc[r][i]);
-    put_elem(&img[4 * kC0Off], kBFwd[0]);
-    put_elem(&img[4 * kBinv0Off], p.binv0);
-    void* d = nullptr;
-    BGPU_CUDA(cudaMalloc(&d, kImageBytes));
-    BGPU_CUDA(cudaMemcpy(d, img.data(), kImageBytes, cudaMemcpyHostToDevice));
-    images[dev] = static_cast<const uint4*>(d);
-  }
-  *out = images[dev];
-  return BINIUS_OK;
+// The shared-memory image of the one-thread kernels.
+void build_image(uint32_t* img) {
+  const HostParams& p = host_params();
+  for (uint32_t m = 0; m < kMaps; m++)
+    for (uint32_t pos = 0; pos < 32; pos++)
+      for (uint32_t nib = 0; nib < 16; nib++) {
+        hu128 v = 0;
+        for (int b = 0; b < 4; b++)
+          if ((nib >> b) & 1) v ^= p.cols[m][4 * pos + b];
+        for (int plane = 0; plane < 4; plane++)
+          img[m * kMapWords + plane * 512 + pos * 16 + nib] = (uint32_t)(v >> (32 * plane));
+      }
+  for (int r = 0; r < 17; r++)
+    for (int i = 0; i < 4; i++) put_elem(&img[4 * (kRcOff + 4 * r + i)], p.rc[r][i]);
+  put_elem(&img[4 * kC0Off], kBFwd[0]);
+  put_elem(&img[4 * kBinv0Off], p.binv0);
 }
 
 // The image of the warp kernels: the maps of their inversion chain and the two affine maps after
@@ -205,42 +190,59 @@ constexpr uint32_t kWarpRcOff = kWarpMaps * kWarpMapRows;
 constexpr uint32_t kWarpC0Off = kWarpRcOff + 17 * 4, kWarpBinv0Off = kWarpC0Off + 1;
 constexpr size_t kWarpImageBytes = 16 * (kWarpBinv0Off + 1);
 
-int device_warp_image(const uint4** out) {
+void build_warp_image(uint32_t* img) {
+  const HostParams& p = host_params();
+  const uint32_t sq_k[6] = {1, 3, 6, 12, 24, 48};
+  for (uint32_t m = 0; m < kWarpMaps; m++) {
+    hu128 cols[128];
+    for (int i = 0; i < 128; i++) {
+      hu128 x = (hu128)1 << i;
+      for (uint32_t k = 0; k < (m < 6 ? sq_k[m] : 1); k++) x = host_gf_mul(x, x);
+      if (m >= 6) x = apply_cols(p.cols[m == kWarpLinv ? kMapLinv : kMapLfwd], x);
+      cols[i] = x;
+    }
+    for (uint32_t row = 0; row < kWarpMapRows; row++) {
+      hu128 v = 0;
+      for (int b = 0; b < 4; b++)
+        if ((row >> b) & 1) v ^= cols[4 * (row / 16) + b];
+      put_elem(&img[4 * (m * kWarpMapRows + row)], v);
+    }
+  }
+  for (int r = 0; r < 17; r++)
+    for (int i = 0; i < 4; i++) put_elem(&img[4 * (kWarpRcOff + 4 * r + i)], p.rc[r][i]);
+  put_elem(&img[4 * kWarpC0Off], kBFwd[0]);
+  put_elem(&img[4 * kWarpBinv0Off], p.binv0);
+}
+
+// Both images, uploaded together on a device's first call of any kind, so that whichever call a
+// program makes before it captures a stream leaves nothing to allocate in the capture.
+struct Images {
+  const uint4 *one, *warp;
+};
+int device_images(Images* out) {
   static std::mutex mu;
   static const uint4* images[64] = {};
   int dev = 0;
   BGPU_CUDA(cudaGetDevice(&dev));
   BGPU_ARG(dev >= 0 && dev < 64, "device ordinal out of range");
+  static_assert(kImageBytes % 16 == 0, "the second image is 16-byte aligned");
   std::lock_guard<std::mutex> g(mu);
   if (!images[dev]) {
-    const HostParams& p = host_params();
-    std::vector<uint32_t> img(kWarpImageBytes / 4, 0);
-    const uint32_t sq_k[6] = {1, 3, 6, 12, 24, 48};
-    for (uint32_t m = 0; m < kWarpMaps; m++) {
-      hu128 cols[128];
-      for (int i = 0; i < 128; i++) {
-        hu128 x = (hu128)1 << i;
-        for (uint32_t k = 0; k < (m < 6 ? sq_k[m] : 1); k++) x = host_gf_mul(x, x);
-        if (m >= 6) x = apply_cols(p.cols[m == kWarpLinv ? kMapLinv : kMapLfwd], x);
-        cols[i] = x;
-      }
-      for (uint32_t row = 0; row < kWarpMapRows; row++) {
-        hu128 v = 0;
-        for (int b = 0; b < 4; b++)
-          if ((row >> b) & 1) v ^= cols[4 * (row / 16) + b];
-        put_elem(&img[4 * (m * kWarpMapRows + row)], v);
-      }
-    }
-    for (int r = 0; r < 17; r++)
-      for (int i = 0; i < 4; i++) put_elem(&img[4 * (kWarpRcOff + 4 * r + i)], p.rc[r][i]);
-    put_elem(&img[4 * kWarpC0Off], kBFwd[0]);
-    put_elem(&img[4 * kWarpBinv0Off], p.binv0);
+    std::vector<uint32_t> img((kImageBytes + kWarpImageBytes) / 4, 0);
+    build_image(img.data());
+    build_warp_image(img.data() + kImageBytes / 4);
     void* d = nullptr;
-    BGPU_CUDA(cudaMalloc(&d, kWarpImageBytes));
-    BGPU_CUDA(cudaMemcpy(d, img.data(), kWarpImageBytes, cudaMemcpyHostToDevice));
+    BGPU_CUDA(cudaMalloc(&d, kImageBytes + kWarpImageBytes));
+    cudaError_t e = cudaMemcpy(d, img.data(), kImageBytes + kWarpImageBytes, cudaMemcpyHostToDevice);
+    // the copy may still be under way when it returns, and the caller's stream need not follow it
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) {
+      cudaFree(d);
+      return cuda_error(e, "vision4 images");
+    }
     images[dev] = static_cast<const uint4*>(d);
   }
-  *out = images[dev];
+  *out = {images[dev], images[dev] + kImageBytes / 16};
   return BINIUS_OK;
 }
 
@@ -621,10 +623,8 @@ __global__ void __launch_bounds__(kGroupLanes << kWarpFuse)
   v4w_layers(buf, 1u << fused, fused, nodes, L, in_level, group, e, mix);
 }
 
-int vision4_commit_warps(const uint4* elems, uint32_t L, uint32_t log_batch, uint4* nodes,
-                         cudaStream_t s) {
-  const uint4* img = nullptr;
-  if (int rc = device_warp_image(&img)) return rc;
+int vision4_commit_warps(const uint4* img, const uint4* elems, uint32_t L, uint32_t log_batch,
+                         uint4* nodes, cudaStream_t s) {
   if (int rc = ensure_smem_limit((const void*)vision4_leaves_warp_kernel, kWarpSmem)) return rc;
   if (int rc = ensure_smem_limit((const void*)vision4_nodes_warp_kernel, kWarpSmem)) return rc;
   // one group per CTA, and so one warp per scheduler, while the leaves are fewer than the SMs
@@ -652,26 +652,26 @@ int vision4_merkle_commit(const void* d_elems, uint32_t log_leaves, uint32_t log
                           void* d_nodes, cudaStream_t s) {
   BGPU_ARG(d_elems != nullptr && d_nodes != nullptr, "elems / nodes is NULL");
   BGPU_ARG(log_leaves <= 34 && log_batch <= 20, "tree too large");
-  const uint4* img = nullptr;
-  if (int rc = device_image(&img)) return rc;
+  Images img;
+  if (int rc = device_images(&img)) return rc;
   if (int rc = ensure_smem_limit((const void*)vision4_leaves_kernel, kV4Smem)) return rc;
   if (int rc = ensure_smem_limit((const void*)vision4_nodes_kernel, kV4Smem)) return rc;
   const uint32_t L = log_leaves;
   uint4* nodes = static_cast<uint4*>(d_nodes);
   if (L <= kWarpMaxLog)
-    return vision4_commit_warps(static_cast<const uint4*>(d_elems), L, log_batch, nodes, s);
+    return vision4_commit_warps(img.warp, static_cast<const uint4*>(d_elems), L, log_batch, nodes, s);
   // at least 2^8 CTAs: mid-size trees spread over every SM in smaller CTAs
   const uint32_t fused = L - 8 < kV4LeafFuse ? L - 8 : kV4LeafFuse;
   const uint64_t grid = 1ull << (L - fused);
   BGPU_ARG(grid <= 0x7fffffffull, "too many leaves");
   vision4_leaves_kernel<<<(unsigned)grid, 1u << fused, kV4Smem, s>>>(
-      img, static_cast<const uint4*>(d_elems), log_batch, nodes, L, fused);
+      img.one, static_cast<const uint4*>(d_elems), log_batch, nodes, L, fused);
   BGPU_LAUNCH_CHECK("vision4_leaves_kernel");
   count_launch();
   for (uint32_t level = fused; level < L;) {
     const uint32_t f = (L - level) < kV4NodeFuse ? (L - level) : kV4NodeFuse;
     const uint64_t g = 1ull << (L - level - f);
-    vision4_nodes_kernel<<<(unsigned)g, 1u << (f - 1), kV4Smem, s>>>(img, nodes, L, level, f);
+    vision4_nodes_kernel<<<(unsigned)g, 1u << (f - 1), kV4Smem, s>>>(img.one, nodes, L, level, f);
     BGPU_LAUNCH_CHECK("vision4_nodes_kernel");
     count_launch();
     level += f;
@@ -686,13 +686,13 @@ extern "C" {
 int binius_vision4_permute(void* d_states, uint64_t n, void* stream) {
   BGPU_ARG(d_states != nullptr || n == 0, "states is NULL");
   if (n == 0) return clear_error();
-  const uint4* img = nullptr;
-  if (int rc = device_image(&img)) return rc;
+  Images img;
+  if (int rc = device_images(&img)) return rc;
   if (int rc = ensure_smem_limit((const void*)vision4_permute_kernel, kV4Smem)) return rc;
   const uint64_t blocks = (n + kV4Threads - 1) / kV4Threads;
   const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
   vision4_permute_kernel<<<grid, kV4Threads, kV4Smem, as_stream(stream)>>>(
-      img, static_cast<uint4*>(d_states), n);
+      img.one, static_cast<uint4*>(d_states), n);
   BGPU_LAUNCH_CHECK("vision4_permute_kernel");
   count_launch();
   return clear_error();
