@@ -223,6 +223,7 @@ struct binius_sumcheck {
   RoundPartials* parts = nullptr;
   RoundResult* result = nullptr;
   uint64_t seq = 0;             // rounds evaluated or queued
+  int device = 0;               // whose memory and default stream these are
   bool queued = false;          // the next execute's sums are on their way
 };
 
@@ -274,6 +275,7 @@ int make(int kind, uint32_t n_vars, void* stream, binius_sumcheck** out) {
   if (int rc = configure_device_pool(dev)) return rc;
   binius_sumcheck* p = new binius_sumcheck();
   p->kind = kind;
+  p->device = dev;
   p->s = as_stream(stream);
   p->n_vars = n_vars;
   // the sums and, for bivariate rounds, the partial sums with their counter clear
@@ -524,12 +526,15 @@ int binius_sumcheck_inout_create(void* d_witness, uint32_t log_len, const void* 
 
 int binius_sumcheck_destroy(binius_sumcheck* p) {
   if (!p) return BINIUS_OK;
+  int prev = p->device;
+  if (cudaGetDevice(&prev) == cudaSuccess && prev != p->device) cudaSetDevice(p->device);
   // the slot and the caller's multilinears, which folds write, are free once the queued work is done
   // (a NULL stream is the default stream, which has work like any other)
   cudaStreamSynchronize(p->s);
   return_slot(p->result);
   if (p->eq) cudaFreeAsync(p->eq, p->s);
   if (p->acc) cudaFreeAsync(p->acc, p->s);
+  if (prev != p->device) cudaSetDevice(prev);
   delete p;
   return BINIUS_OK;
 }
