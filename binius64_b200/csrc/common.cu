@@ -33,36 +33,34 @@ int clear_error() {
 }
 
 namespace {
-std::atomic<uint32_t*> g_tensor_word{nullptr};
+// Registered rather than allocated: the first pinned allocation of a process takes 1.2 ms, this 0.3.
+alignas(4096) uint8_t g_tensor_page[4096];
+std::atomic<bool> g_tensor_ready{false};
 const char* const kTensorStall =
     "a bounded wait for the tensor cores ran out; results since then are undefined";
 }  // namespace
 
 bool tensor_stalled() {
-  const uint32_t* w = g_tensor_word.load(std::memory_order_acquire);
-  return w && *static_cast<const volatile uint32_t*>(w) != 0;
+  return *reinterpret_cast<const volatile uint32_t*>(g_tensor_page) != 0;
 }
 
 int tensor_word(uint32_t** word) {
   static std::mutex mu;
   if (tensor_stalled()) return set_error(BINIUS_E_TIMEOUT, kTensorStall);
-  uint32_t* w = g_tensor_word.load(std::memory_order_acquire);
-  if (!w) {
+  if (!g_tensor_ready.load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lock(mu);
-    w = g_tensor_word.load(std::memory_order_acquire);
-    if (!w) {
+    if (!g_tensor_ready.load(std::memory_order_acquire)) {
       // the first launch to need it may be one that is being captured
       cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
       BGPU_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-      const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&w), 64,
-                                          cudaHostAllocPortable | cudaHostAllocMapped);
+      const cudaError_t e = cudaHostRegister(g_tensor_page, sizeof(g_tensor_page),
+                                             cudaHostRegisterPortable | cudaHostRegisterMapped);
       cudaThreadExchangeStreamCaptureMode(&mode);
       if (e != cudaSuccess) return cuda_error(e, "tensor status word");
-      *w = 0;
-      g_tensor_word.store(w, std::memory_order_release);
+      g_tensor_ready.store(true, std::memory_order_release);
     }
   }
-  *word = w;
+  BGPU_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(word), g_tensor_page, 0));
   return BINIUS_OK;
 }
 
