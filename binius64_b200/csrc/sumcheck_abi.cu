@@ -224,6 +224,7 @@ struct binius_sumcheck {
   RoundResult* result = nullptr;
   uint64_t seq = 0;             // rounds evaluated or queued
   int device = 0;               // whose memory and default stream these are
+  bool busy = true;             // work may be queued (until finish has waited for all of it)
   bool queued = false;          // the next execute's sums are on their way
 };
 
@@ -445,6 +446,7 @@ int do_finish(binius_sumcheck* p, int kind, void* h_evals) {
   for (int i = 0; i < n; i++)
     if (int rc = rd.add(static_cast<uint8_t*>(h_evals) + 16 * i, p->cols[i], 16)) return rc;
   if (int rc = rd.wait()) return rc;
+  p->busy = false;  // no call but finish and destroy is left
   return clear_error();
 }
 
@@ -530,7 +532,7 @@ int binius_sumcheck_destroy(binius_sumcheck* p) {
   if (cudaGetDevice(&prev) == cudaSuccess && prev != p->device) cudaSetDevice(p->device);
   // the slot and the caller's multilinears, which folds write, are free once the queued work is done
   // (a NULL stream is the default stream, which has work like any other)
-  cudaStreamSynchronize(p->s);
+  if (p->busy) cudaStreamSynchronize(p->s);
   return_slot(p->result);
   if (p->eq) cudaFreeAsync(p->eq, p->s);
   if (p->acc) cudaFreeAsync(p->acc, p->s);
