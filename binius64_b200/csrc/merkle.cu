@@ -33,7 +33,8 @@ constexpr uint32_t kNodeFuse = 9;  // at most 2^9 inputs per CTA (Tuning::merkle
 // Measured on B200, all layers of a CTA -> three, in us: 2^24 leaves of one element 3147 -> 2458
 // (13.7 G compressions/s), 2^22 819 -> 653, 2^20 237 -> 194, 2^20 of 16 elements 545 -> 471, 2^18 89
 // -> 74, 2^17 64 -> 58; at 2^16 (47 -> 46) and below (2^15 33 -> 44) the added launches cost what the
-// idle lanes do, or more.  Two or four layers are within 4% of three.
+// idle lanes do, or more.  Two or four layers are within 4% of three.  (Both sides with the last
+// block's schedule as an argument; without that and with all layers 3278, 858, .., 579, 95.)
 constexpr uint32_t kFullLog = 17;
 constexpr uint32_t kFullLayers = 3;
 
