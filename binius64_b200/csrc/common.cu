@@ -35,7 +35,7 @@ int clear_error() {
 namespace {
 // Registered rather than allocated: the first pinned allocation of a process takes 1.2 ms, this 0.3.
 alignas(4096) uint8_t g_tensor_page[4096];
-std::atomic<bool> g_tensor_ready{false};
+std::atomic<uint32_t*> g_tensor_word{nullptr};  // its device address
 const char* const kTensorStall =
     "a bounded wait for the tensor cores ran out; results since then are undefined";
 }  // namespace
@@ -47,20 +47,26 @@ bool tensor_stalled() {
 int tensor_word(uint32_t** word) {
   static std::mutex mu;
   if (tensor_stalled()) return set_error(BINIUS_E_TIMEOUT, kTensorStall);
-  if (!g_tensor_ready.load(std::memory_order_acquire)) {
+  uint32_t* w = g_tensor_word.load(std::memory_order_acquire);
+  if (!w) {
     std::lock_guard<std::mutex> lock(mu);
-    if (!g_tensor_ready.load(std::memory_order_acquire)) {
+    w = g_tensor_word.load(std::memory_order_acquire);
+    if (!w) {
       // the first launch to need it may be one that is being captured
       cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
       BGPU_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-      const cudaError_t e = cudaHostRegister(g_tensor_page, sizeof(g_tensor_page),
-                                             cudaHostRegisterPortable | cudaHostRegisterMapped);
+      cudaError_t e = cudaHostRegister(g_tensor_page, sizeof(g_tensor_page),
+                                       cudaHostRegisterPortable | cudaHostRegisterMapped);
+      if (e == cudaErrorHostMemoryAlreadyRegistered) e = cudaSuccess;  // an earlier try got this far
+      // (the address is the same on every device of a unified address space)
+      if (e == cudaSuccess)
+        e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&w), g_tensor_page, 0);
       cudaThreadExchangeStreamCaptureMode(&mode);
       if (e != cudaSuccess) return cuda_error(e, "tensor status word");
-      g_tensor_ready.store(true, std::memory_order_release);
+      g_tensor_word.store(w, std::memory_order_release);
     }
   }
-  BGPU_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(word), g_tensor_page, 0));
+  *word = w;
   return BINIUS_OK;
 }
 
